@@ -155,6 +155,7 @@ int sg_set_particles(sg_context *ctx, int n_particles, const double *xy, int n_u
       SG_CUDA(cudaMemcpy(ctx->map.ptr, map.data(), n_unknowns * sizeof(int), cudaMemcpyHostToDevice));
     }
     ctx->pairs_ready = false;
+    ctx->ib.ready = false;
     ctx->tuned_df.clear();
     ctx->kind = -1;  // the table must be re-uploaded for a new geometry
     ctx->vol = false;
@@ -209,6 +210,7 @@ int sg_set_lookup(sg_context *ctx, int kind, int len_rho, double rho_min, double
     ctx->rho_min = rho_min;
     ctx->res = resolution;
     ctx->pairs_ready = false;
+    ctx->ib.ready = false;
     ctx->df_ready = false;
     ctx->tuned_df.clear();
     ctx->pgraphs.clear();  // their near-field blocks came from the old table
@@ -405,6 +407,8 @@ static int matvec_host(sg_context *ctx, const double *x, double *y, int nrhs, in
       throw sg::Error{SG_ERR_CUDA, "pair-symmetric FP32 operator: a bounded wait ran out"};
     if (precision == SG_FP32 && sg::tc_check_error(ctx, st))
       throw sg::Error{SG_ERR_CUDA, "tensor-core operator: a bounded wait ran out"};
+    if (precision == SG_FP64 && sg::ib_check_error(ctx, st))
+      throw sg::Error{SG_ERR_CUDA, "interval-batched operator: a bounded wait ran out"};
     return SG_OK;
   });
 }
@@ -479,6 +483,8 @@ static int solve_dev_impl(sg_context *ctx, const double2 *b, double2 *x, int nrh
     throw sg::Error{SG_ERR_CUDA, "pair-symmetric FP32 operator: a bounded wait ran out"};
   if ((precision & SG_FP32) && sg::tc_check_error(ctx, st))
     throw sg::Error{SG_ERR_CUDA, "tensor-core operator: a bounded wait ran out"};
+  if (sg::ib_check_error(ctx, st))
+    throw sg::Error{SG_ERR_CUDA, "interval-batched operator: a bounded wait ran out"};
   if (!std::isfinite(local.max_rel_residual)) throw sg::Error{SG_ERR_NAN, "solver produced NaN or Inf"};
   if (local.converged < nrhs) {
     sg::set_error("GMRES did not reach the tolerance for every right-hand side");

@@ -1151,6 +1151,14 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
   return v;
 }
 
+// The interval-batched operator keeps a workspace and orders its calls by an event, which a captured
+// graph could not follow: under stream capture the per-receiver kernel runs.
+static bool ib_usable(const sg_context *c, cudaStream_t st) {
+  if (!ib_supported(c)) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool master, bool fp32, cudaStream_t st) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c->profiling) {
@@ -1176,7 +1184,9 @@ void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool maste
       sym_rt = c->tuned.back().sym_rt;
     }
   }
-  if (variant == 5) {
+  if (variant == 0 && !fp32 && ib_usable(c, st)) {
+    c->launches += launch_ibatch(c, x, y, R, master, st);
+  } else if (variant == 5) {
     c->launches += launch_tcsym_matvec(c, x, y, R, master, st);
   } else if (variant == 4) {
     c->launches += launch_tc_matvec(c, x, y, R, master, st);

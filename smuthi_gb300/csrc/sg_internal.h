@@ -104,6 +104,14 @@ void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool maste
 void solve_padded(sg_context *c, const double2 *b, double2 *x, int R, double rtol, int restart, int maxiter,
                   int precision, sg_solve_info *info, cudaStream_t st);
 void residual_norms(sg_context *c, const double2 *b, const double2 *x, int R, double *rel, cudaStream_t st);
+// FP64 operator batched by lookup interval on the tensor cores (sg_ibatch.cu)
+bool ib_supported(const sg_context *c);
+int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
+bool ib_check_error(sg_context *c, cudaStream_t st);  // reads and clears the timeout flag (synchronises)
+struct IbRec {  // one ordered pair: fraction within its interval, direction, receiver i and emitter j
+  double t, c, s;
+  int i, j;
+};
 // choose the j-split for a problem (>= 1)
 int choose_split(int n_particles, int nrhs);
 
@@ -266,6 +274,29 @@ struct sg_context {
   sg::DevBuf<float2> sym_yacc;
   sg::DevBuf<int> sym_err;  // set when a bounded wait of the pair-symmetric kernel ran out
   bool sym_err_init = false;
+
+  // interval-batched FP64 operator (sg_ibatch.cu): ordered pairs sorted by lookup interval, the
+  // intervals' digit operands, the pairs' contributions V of one chunk
+  struct IbTiles {
+    int per = 0;  // pairs per tile
+    std::vector<int> h_toff;
+    sg::DevBuf<int> toff;
+  };
+  struct Ib {
+    bool ready = false;
+    int nb = 0;
+    std::vector<int> h_boff;
+    sg::DevBuf<sg::IbRec> rec;
+    sg::DevBuf<unsigned> slot;
+    sg::DevBuf<int> boff, exps, err;
+    sg::DevBuf<unsigned char> B;
+    sg::DevBuf<double2> V, acc;
+    std::vector<std::unique_ptr<IbTiles>> tiles;
+    cudaEvent_t done = nullptr;  // end of the last call: calls on other streams wait for it
+    ~Ib() {
+      if (done) cudaEventDestroy(done);
+    }
+  } ib;
 
   // T-matrices
   int n_types = 0, t_diag = 1;
