@@ -5,42 +5,45 @@
 // interval turns the operator into one small GEMM per interval, whose matrices C_{k,c} all pairs of
 // the interval share:
 //
-//   y_i += D^H [ (C_0 u + C_2 t^2 u) + t (C_1 u + C_3 t^2 u) ],   u = D x_j,
+//   y_i += D^H [ ((C_3 u t + C_2 u) t + C_1 u) t + C_0 u ],   u = D x_j,
 //
-// so the work per pair that is not on the tensor cores falls from O(B^2) to O(B): rotate x_j, form
-// t^2 u, and combine and rotate back the two half sums. The per-receiver kernel (sg_coupling.cu)
-// interpolates B^2 coefficients in FP64 for every ordered pair, on a pipe that runs two FP64
-// multiply-adds per clock and SM.
+// so the work per pair that is not on the tensor cores falls from O(B^2) to O(B): rotate x_j, combine
+// the powers of t and rotate back. The per-receiver kernel (sg_coupling.cu) interpolates B^2
+// coefficients in FP64 for every ordered pair, on a pipe that runs two FP64 multiply-adds per clock
+// and SM.
 //
 // FP64 accuracy on FP16 tensor cores (error-free slicing, the scheme of Ozaki, Ogita, Oishi and Rump,
-// Numer. Algorithms 59 (2012)): every operand is a 60-bit fixed-point number under a power-of-two
-// scale (per column of C, then per row of C; per pair and right-hand side for u) cut into six signed
-// 10-bit digits, which FP16 holds exactly. A product of two digits is at most 2^18 and at most 64 of
-// them are summed (K = 32 or 64), so every FP32 accumulator stays an exact integer of at most 2^24
-// whatever the order of the sums. The digit products of equal weight share one accumulator (six of
-// them; products below 2^-60 of the scales are dropped), and the epilogue combines the accumulators
-// in 64-bit integers. The result is bitwise independent of how the pairs are grouped.
+// Numer. Algorithms 59 (2012)): every operand is a 63-bit fixed-point number under a power-of-two
+// scale (per column of C, then per row of C; per pair and right-hand side for u) cut into seven signed
+// 9-bit digits, which FP16 holds exactly. The digit products of equal weight 2^(-9 d), d = 0..6, share
+// one FP32 accumulator; smaller products (below 2^-60 of the scales) are dropped. A digit product is at
+// most 2^16 and K = 32 of them (at most 30 nonzero for blocksize <= 30) times d + 1 <= 7 pairs of digits
+// are summed, at most 7 * 30 * 2^16 = 13,762,560 < 2^24: every accumulator stays an exact integer
+// whatever the order of the sums. (Ten-bit digits would need fewer products, but the sums of the
+// middle weights could pass 2^24.) The digits are combined in 64-bit integers, in which the powers of
+// t and the rotations follow; the result is independent of how the pairs are grouped.
 //
-// One CTA per SM (216 KB of shared memory) walks a contiguous range of tiles; a tile is up to 64
-// complex columns (pairs x right-hand sides) of one interval:
-//   * rotate: 512 threads form u and t^2 u in FP64, cut them into digits and store them as the A
-//     operand (128 rows: Re and Im of 64 columns; K = 32 per power of t^2);
+// One CTA per SM walks a contiguous range of tiles; a tile is up to 64 complex columns (pairs x
+// right-hand sides) of one interval:
+//   * the warps rotate x_j, cut u into digits and store them as the A operand (128 rows: Re and Im of 64
+//     columns, K = 32);
 //   * one thread issues the digit products against the interval's B operand (resident while the
-//     interval lasts), N = 32 columns at a time: 8 rows n1 x (Re, Im) x (even, odd powers), into
-//     two tensor-memory buffers of six accumulators;
-//   * all warps read a buffer back, combine digits, real and imaginary parts (neighbouring lanes) and
-//     the powers of t, rotate back and store the pair's contribution V while the next buffer fills.
+//     interval lasts): passes of 128 rows (n1, power of t, Re / Im), one job per weight d = 6..0 in a
+//     ring of four tensor-memory accumulators of 128 columns;
+//   * the warps read the jobs back (32 columns per warp), combine digits, real and imaginary parts
+//     (neighbouring lanes) and powers of t, rotate back and store the pair's contribution V.
 // A second kernel sums V over the emitters of every receiver in index order (deterministic) and forms
 // W x or x - T W x. V is a bounded workspace: larger problems run in chunks of tiles.
 //
-// Bound: the FP64 pipe, about 11 operations per real output and input of a pair (two at the digits'
-// conversion, the rotations, the scaling) against 20 B per output of the per-receiver kernel.
+// Integer arithmetic instead of FP64 for everything but the last conversion: a GB300 SM sub-partition
+// issues an FP64 instruction every 64 cycles, a 32-bit integer one every two.
 #include <cub/cub.cuh>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "sg_epilogue.h"
@@ -49,27 +52,60 @@
 
 namespace sg {
 
-static constexpr int kIbThreads = 512;
-static constexpr int kIbCols = 64;    // complex columns per tile
-static constexpr int kIbDig = 6;      // digits per operand
-static constexpr int kIbBP = 32;      // padded blocksize
-static constexpr int kIbMaxM = 7;     // largest |m| of the phase table
-static constexpr int kIbGroupN = 32;  // MMA N: 8 rows n1 x (Re, Im) x (even, odd powers)
-static constexpr unsigned long long kIbBias =
-    512ull * (1ull + (1ull << 10) + (1ull << 20) + (1ull << 30) + (1ull << 40) + (1ull << 50));
+static constexpr int kIbWarps = 16;
+static constexpr int kIbThreads = 32 * kIbWarps;
+static constexpr int kIbCols = 64;   // complex columns per tile
+static constexpr int kIbDig = 7;     // digits per operand
+static constexpr int kIbBits = 9;    // bits per digit
+static constexpr int kIbK = 32;      // padded blocksize
+static constexpr int kIbMaxB = 30;   // largest blocksize whose accumulators are exact
+static constexpr int kIbMaxM = 3;    // largest |m| of the phase table
+static constexpr int kIbN = 128;     // B operand rows per pass: n1 x powers of t x (Re, Im)
+static constexpr int kIbKC = kIbK / 8;                 // core columns of 16 bytes
+static constexpr int kIbSlice = 128 * kIbK * 2;        // bytes of one digit of an operand
+static constexpr int kIbOperand = kIbDig * kIbSlice;   // bytes of an A operand or one pass of B
+static constexpr unsigned long long ib_bias() {
+  unsigned long long b = 0;
+  for (int i = 0; i < kIbDig; ++i) b |= 1ull << (kIbBits * i + kIbBits - 1);
+  return b;
+}
+static constexpr unsigned long long kIbBias = ib_bias();
+static_assert(kIbDig * kIbMaxB * (1 << (2 * kIbBits - 2)) <= (1 << 24), "exact FP32 accumulators");
+// largest t in units of 2^-62 whose high word fits (t < 1 up to its last places)
+static constexpr long long kIbBelowOne = (1ll << 62) - (1ll << 30) - 1;
 
 template <int NC>
 struct IbShape {
-  static constexpr int K = kIbBP * (NC / 2), KC = K / 8;  // K elements, core columns of 16 bytes
-  static constexpr int ASLICE = kIbCols * 2 * K * 2;      // bytes of one digit of the A operand
-  static constexpr int BSLICE = kIbGroupN * K * 2;        // bytes of one digit of one B group
-  static constexpr int BBYTES = 4 * kIbDig * BSLICE;      // one interval's B operand
-  static constexpr int PHS = kIbMaxM + 2;                 // phase-table row stride (double2)
-  static constexpr size_t META = 2 * kIbCols * (PHS * sizeof(double2) + sizeof(double) + sizeof(long long)) +
-                                 kIbCols * sizeof(int) + 2 * 64 * sizeof(int) + kIbBP * sizeof(int) + 128;
-  static constexpr size_t SMEM = (size_t)kIbDig * ASLICE + BBYTES + META;
-  static_assert(SMEM <= kTcSmemBudget, "shared memory");
+  static constexpr int RN = 2 * NC;            // B rows per n1
+  static constexpr int PN = kIbN / RN;         // n1 per pass
+  static constexpr int PASSES = 32 / PN;       // at most
+  static constexpr int BBYTES = PASSES * kIbOperand;
 };
+
+// per-tile data, four tiles deep: written two tiles ahead, read until the tile is stored
+struct IbTile {
+  int4 ph[kIbCols][kIbMaxM + 1];  // cos, sin of m phi in words of 2^-61
+  int2 t[kIbCols];                // t in words of 2^-62
+  long long xoff[kIbCols];        // x_j of the column
+  int eb[kIbK], ea[kIbK];         // column and row exponents of the interval
+  int cexp[kIbCols];              // scale of x_j (written with the A operand)
+  int ncol, bucket;
+  long long pair0;                // first pair, from the start of V
+};
+
+struct IbSmem {
+  IbTile tile[4];
+  uint64_t dfull[4], dempty[4], afull, meta[4], bfull, done;
+  int mofn[kIbK];
+  uint32_t tmem;
+  int lb[2];  // bucket of the two look-ahead warps
+};
+static constexpr size_t kIbSmemTail = (sizeof(IbSmem) + 127) / 128 * 128;
+template <int NC>
+constexpr size_t ib_smem() {
+  return (size_t)kIbOperand + IbShape<NC>::BBYTES + kIbSmemTail;
+}
+static_assert(ib_smem<4>() <= kTcSmemBudget, "shared memory");
 
 struct IbArgs {
   const IbRec *rec;       // ordered pairs sorted by interval
@@ -77,331 +113,408 @@ struct IbArgs {
   const int *toff;        // [nb + 1] first tile
   const unsigned char *B; // [nb] B operands
   const int *exps;        // [nb][64]: column exponents eb[32], row exponents ea[32]
-  const double2 *x;       // [N][bs][R]
+  const double *x;        // [N][bs][R] complex
   const int *mofn;
-  double2 *V;             // [pair - s0][rt][bs]
+  double *V;              // [pair - s0][rt][bs] complex
   long long s0;           // first pair of this chunk
   int nb, bs, mmax, R, r0, rt, per, t0, t1;  // rt right-hand sides from r0; per = pairs per tile; tiles [t0, t1)
   int *err;
 };
 
-// 60-bit digits of |v| 2^(59 - scale) as sum of six 10-bit fields, each offset by 512; `below` = how far the
-// exponent of v lies below the scale's
-__device__ __forceinline__ unsigned long long ib_fixed(double v, int below) {
+__device__ __forceinline__ int ib_field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
+
+// v 2^(53 + UP - scale) truncated, for an exponent of v that lies `below` under the scale's
+template <int UP>
+__device__ __forceinline__ long long ib_fixed(double v, int below) {
   const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
   const unsigned mh = (hi & 0xFFFFFu) | 0x100000u;
-  unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 6) << 32) | (lo << 6);
+  unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, UP) << 32) | (lo << UP);
   m = (hi & 0x7FF00000u) == 0u || below > 63 ? 0ull : m >> (below & 63);
-  return (int)hi < 0 ? kIbBias - m : kIbBias + m;
+  return (int)hi < 0 ? -(long long)m : (long long)m;
 }
 
-// the digits of two fixed-point numbers as packed FP16 integers in [-512, 512]
-__device__ __forceinline__ void ib_digits(unsigned long long f0, unsigned long long f1, uint32_t (&d)[kIbDig]) {
+// the digits of two 63-bit fixed-point numbers as packed FP16 integers in [-256, 256]
+__device__ __forceinline__ void ib_digits(long long v0, long long v1, uint32_t (&d)[kIbDig]) {
+  const unsigned long long f0 = (unsigned long long)v0 + kIbBias, f1 = (unsigned long long)v1 + kIbBias;
 #pragma unroll
   for (int s = 0; s < kIbDig; ++s) {
-    const int sh = 10 * (kIbDig - 1 - s);
-    uint32_t a = (uint32_t)(f0 >> sh), b = (uint32_t)(f1 >> sh);
-    if (s > 0) {
-      a &= 1023u;
-      b &= 1023u;
-    }
-    // FP16 1024 + digit is 0x6400 + digit; the top digit may be 1024, where the sum is still exact (2048)
-    const uint32_t p = (a | (b << 16)) + 0x64006400u;
-    const __half2 h = __hadd2(*reinterpret_cast<const __half2 *>(&p), __floats2half2_rn(-1536.f, -1536.f));
+    const int sh = kIbBits * (kIbDig - 1 - s);
+    const uint32_t mask = s > 0 ? 511u : 1023u;  // the top digit may be 512
+    const uint32_t a = (uint32_t)(f0 >> sh);
+    const uint32_t b = sh >= 16 ? (uint32_t)(f1 >> (sh - 16)) : (uint32_t)f1 << (16 - sh);
+    const uint32_t p = (a & mask) | (b & (mask << 16)) | 0x64006400u;  // FP16 1024 + digit + 256
+    const __half2 h = __hadd2(*reinterpret_cast<const __half2 *>(&p), __floats2half2_rn(-1280.f, -1280.f));
     d[s] = *reinterpret_cast<const uint32_t *>(&h);
   }
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-               : "r"(taddr));
+// Products of 62-bit fixed-point numbers from 31-bit words: three 32 x 32 -> 64 bit multiply-adds, low
+// word by low word (below the last place kept) is dropped. The factors that stay the same for a pair
+// (t, the phases) carry a signed low word in [-2^30, 2^30), so that what is dropped has no bias that
+// would add up over the pairs.
+struct IbWords {
+  int h, l;
+};
+__device__ __forceinline__ IbWords ib_split(long long v) {
+  return {(int)(v >> 31), (int)((unsigned)v & 0x7FFFFFFFu)};
+}
+__device__ __forceinline__ IbWords ib_split_signed(long long v) {
+  return {(int)((v + 0x40000000ll) >> 31), (int)((unsigned)v << 1) >> 1};
+}
+__device__ __forceinline__ long long ib_mad(int a, int b, long long c) { return (long long)a * b + c; }
+// a b / 2^62 + c
+__device__ __forceinline__ long long ib_mul(IbWords a, int bh, int bl, long long c) {
+  const long long mid = ib_mad(a.h, bl, ib_mad(a.l, bh, 0x40000000ll));
+  return ib_mad(a.h, bh, c + (mid >> 31));
 }
 
-// v as double, exact to rounding: high and low words placed in the mantissas of 2^84 and 2^52
-__device__ __forceinline__ double ib_ll2d(long long v) {
+// v 2^e rounded to double: the words placed in the mantissas of 2^84 and 2^52, two FP64 additions
+__device__ __forceinline__ double ib_to_double(long long v, int e) {
   const unsigned lo = (unsigned)v, hi = (unsigned)((unsigned long long)v >> 32) ^ 0x80000000u;
   const double h = __hiloint2double(0x45300000, (int)hi) - (19342813113834066795298816.0 +  // 2^84
                                                             9223372036854775808.0 +         // 2^63
                                                             4503599627370496.0);            // 2^52
-  return h + __hiloint2double(0x43300000, (int)lo);
+  const double d = h + __hiloint2double(0x43300000, (int)lo);
+  const int f = ib_field(d);
+  if (f != 0 && f + e > 0 && f + e < 0x7FF) return __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
+  return scalbn(d, e);  // zero, or outside the normal range
 }
 
-// x 2^e for a finite x
-__device__ __forceinline__ double ib_scale(double x, int e) {
-  const int hi = __double2hiint(x);
-  const int ex = (hi >> 20) & 0x7FF;
-  if (ex != 0 && ex + e > 0 && ex + e < 0x7FF) return __hiloint2double(hi + (e << 20), __double2loint(x));
-  return scalbn(x, e);
+// One product of a digit of A and a digit of B (K = 16) into dst; the descriptors differ from those of the
+// operands' first bytes by a constant in their low word.
+template <bool ACC>
+__device__ __forceinline__ void ib_mma(uint32_t dst, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %3};\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(dst),
+      "r"(a), "r"(b), "r"(hi), "r"(idesc), "n"(ACC ? 1 : 0)
+      : "memory");
+}
+
+// all digit products of weight D; unrolled, because one thread issues them and every instruction between two
+// MMAs costs it several cycles
+template <int D>
+__device__ __forceinline__ void ib_issue(uint32_t dst, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc) {
+#pragma unroll
+  for (int i = 0; i <= D; ++i)
+#pragma unroll
+    for (int ks = 0; ks < kIbK / 16; ++ks) {
+      const uint32_t ao = a + (uint32_t)((i * kIbSlice + ks * 256) >> 4), bo = b + (uint32_t)(((D - i) * kIbSlice + ks * 256) >> 4);
+      if (i == 0 && ks == 0) ib_mma<false>(dst, ao, bo, hi, idesc);
+      else ib_mma<true>(dst, ao, bo, hi, idesc);
+    }
 }
 
 template <int NC>
 __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
   using Sh = IbShape<NC>;
-  constexpr int KC = Sh::KC, PHS = Sh::PHS, DBUF = kIbDig * kIbGroupN;
-  extern __shared__ __align__(1024) unsigned char ib_smem[];
-  unsigned char *As = ib_smem, *Bs = ib_smem + (size_t)kIbDig * Sh::ASLICE;
-  double2 *ph = reinterpret_cast<double2 *>(Bs + Sh::BBYTES);                  // [2][64][PHS]
-  double *tf = reinterpret_cast<double *>(ph + 2 * kIbCols * PHS);             // [2][64]
-  long long *xoff = reinterpret_cast<long long *>(tf + 2 * kIbCols);           // [2][64]
-  uint64_t *bars = reinterpret_cast<uint64_t *>(xoff + 2 * kIbCols);           // dfull[2], bfull, fin
-  int *cexp = reinterpret_cast<int *>(bars + 4);                               // [64] column scale
-  int *ex = cexp + kIbCols;                                                    // [2][64]
-  int *mofn_s = ex + 2 * 64;                                                   // [32]
-  int *tinfo = mofn_s + kIbBP;                                                 // [2][4]: bucket, columns, first pair
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tinfo + 8);
+  constexpr int RN = Sh::RN, PN = Sh::PN, WN = PN / 4;  // WN rows n1 per warp and pass
+  extern __shared__ __align__(1024) unsigned char ib_raw[];
+  unsigned char *As = ib_raw, *Bs = ib_raw + kIbOperand;
+  IbSmem &S = *reinterpret_cast<IbSmem *>(Bs + Sh::BBYTES);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bs = a.bs;
-
   const int ntiles = a.t1 - a.t0;
   const int T0 = a.t0 + (int)((long long)ntiles * blockIdx.x / gridDim.x);
-  const int T1 = a.t0 + (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
+  const int NT = a.t0 + (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x) - T0;  // this CTA's tiles
+  const int passes = (bs + PN - 1) / PN;
 
-  if (tid < kIbBP) mofn_s[tid] = tid < bs ? a.mofn[tid] : 0;
+  if (tid < kIbK) S.mofn[tid] = tid < bs ? a.mofn[tid] : 0;
   if (tid == 0) {
-    for (int b = 0; b < 4; ++b)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[b])) : "memory");
+    auto init = [](uint64_t *b, int n) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n) : "memory");
+    };
+    for (int b = 0; b < 4; ++b) {
+      init(&S.dfull[b], 1);
+      init(&S.dempty[b], kIbWarps);
+      init(&S.meta[b], 2);
+    }
+    init(&S.afull, kIbWarps);
+    init(&S.bfull, 1);
+    init(&S.done, kIbWarps);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tmem)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-
-  // the two last warps look one tile ahead: column c = lane of their 64 threads
-  const int mc = tid - (kIbThreads - kIbCols);
-  int mb = 0;
-  if (mc >= 0 && T0 < T1) {  // bucket of the first tile
-    int lo = 0, hi = a.nb - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (a.toff[mid] <= T0) lo = mid;
-      else hi = mid - 1;
-    }
-    mb = lo;
-  }
-  auto look_ahead = [&](int T, int buf) {
-    if (mc < 0 || T >= T1) return;
-    while (T >= a.toff[mb + 1]) ++mb;
-    const int p0 = a.boff[mb] + (T - a.toff[mb]) * a.per, p1 = min(a.boff[mb + 1], p0 + a.per);
-    const int ncol = (p1 - p0) * a.rt;
-    if (mc == 0) {
-      tinfo[buf * 4] = mb;
-      tinfo[buf * 4 + 1] = ncol;
-      tinfo[buf * 4 + 2] = p0;
-    }
-    ex[buf * 64 + mc] = a.exps[(size_t)mb * 64 + mc];
-    if (mc < ncol) {
-      const int p = p0 + mc / a.rt, r = mc % a.rt;
-      const IbRec rc = a.rec[p];
-      tf[buf * kIbCols + mc] = rc.t;
-      xoff[buf * kIbCols + mc] = (long long)rc.j * bs * a.R + a.r0 + r;
-      double2 *o = ph + (size_t)(buf * kIbCols + mc) * PHS;
-      double pr = 1.0, pi = 0.0;
-      o[0] = make_double2(1.0, 0.0);
-      for (int m = 1; m <= a.mmax; ++m) {
-        const double nr = pr * rc.c - pi * rc.s;
-        pi = pr * rc.s + pi * rc.c;
-        pr = nr;
-        o[m] = make_double2(pr, pi);
-      }
-    }
-  };
-  look_ahead(T0, 0);
-
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-  const uint32_t idesc = (1u << 4) | ((uint32_t)(kIbGroupN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);  // F16 in, F32 out
-  const int nq = (bs + 7) / 8;  // groups of 8 rows n1
-  const uint32_t a_base = smem_u32(As), b_base = smem_u32(Bs);
+  const uint32_t tmem = S.tmem;
+  bool good = true;
 
-  // digit products of row group q into buffer q & 1 (one thread)
-  auto issue = [&](int q) {
-    const uint32_t d0 = tmem + (uint32_t)((q & 1) * DBUF);
-#pragma unroll 1
-    for (int d = 0; d < kIbDig; ++d) {
-#pragma unroll 1
-      for (int i = 0; i <= d; ++i) {
-        const uint32_t aa = a_base + (uint32_t)(i * Sh::ASLICE);
-        const uint32_t bb = b_base + (uint32_t)((q * kIbDig + d - i) * Sh::BSLICE);
-#pragma unroll
-        for (int ks = 0; ks < Sh::K / 16; ++ks) {
-          const uint32_t acc = (i == 0 && ks == 0) ? 0u : 1u;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\t"
-              "setp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d0 + (uint32_t)(d * kIbGroupN)),
-              "l"(tc_desc<KC>(aa + ks * 256)), "l"(tc_desc<KC>(bb + ks * 256)), "r"(idesc), "r"(acc)
-              : "memory");
-        }
+  // ------------------------------------------------------------------ look ahead (two warps, 32 columns each)
+  const int look_half = warp == 5 ? 0 : (warp == 10 ? 1 : -1);
+  if (look_half >= 0) {  // bucket of the first tile
+    int lb = 0, hi = a.nb - 1;
+    while (lb < hi) {
+      const int mid = (lb + hi + 1) >> 1;
+      if (a.toff[mid] <= T0) lb = mid;
+      else hi = mid - 1;
+    }
+    S.lb[look_half] = lb;
+    __syncwarp();
+  }
+  auto look = [&](int ti) {
+    if (look_half < 0 || ti >= NT) return;
+    IbTile &t = S.tile[ti & 3];
+    const int T = T0 + ti;
+    int lb = S.lb[look_half];
+    while (T >= a.toff[lb + 1]) ++lb;
+    __syncwarp();
+    S.lb[look_half] = lb;
+    const int p0 = a.boff[lb] + (T - a.toff[lb]) * a.per, p1 = min(a.boff[lb + 1], p0 + a.per);
+    const int ncol = (p1 - p0) * a.rt;
+    if (look_half == 0) {
+      t.eb[lane] = a.exps[(size_t)lb * 64 + lane];
+      if (lane == 0) {
+        t.ncol = ncol;
+        t.bucket = lb;
+        t.pair0 = p0 - a.s0;
+      }
+    } else {
+      t.ea[lane] = a.exps[(size_t)lb * 64 + 32 + lane];
+    }
+    const int c = look_half * 32 + lane;
+    if (c < ncol) {
+      const int p = p0 + c / a.rt, r = c % a.rt;
+      const IbRec rc = a.rec[p];
+      auto words = [](double v, int up) {  // v in units of 2^-up, |v| <= 1
+        return ib_split_signed(min(ib_fixed<10>(v, 1023 + 62 - up - ib_field(v)), kIbBelowOne));
+      };
+      const IbWords tw = words(rc.t, 62);
+      t.t[c] = make_int2(tw.h, tw.l);
+      t.xoff[c] = 2 * ((long long)rc.j * bs * a.R + a.r0 + r);
+      t.ph[c][0] = make_int4(1 << 30, 0, 0, 0);
+      double pr = rc.c, pi = rc.s;
+      for (int m = 1; m <= a.mmax; ++m) {
+        const IbWords cw = words(pr, 61), sw = words(pi, 61);
+        t.ph[c][m] = make_int4(cw.h, cw.l, sw.h, sw.l);
+        const double nr = pr * rc.c - pi * rc.s;
+        pi = pr * rc.s + pi * rc.c;
+        pr = nr;
       }
     }
-    tc_commit(smem_u32(&bars[q & 1]));
+    __syncwarp();
+    if (lane == 0) tc_arrive(smem_u32(&S.meta[ti & 3]));
   };
-
-  int cur_b = -1, bloads = 0, uses0 = 0, uses1 = 0;
-  bool good = true, issued = false;
-  for (int T = T0; T < T1 && good; ++T) {
-    const int buf = (T - T0) & 1;
-    const int b = tinfo[buf * 4], ncol = tinfo[buf * 4 + 1];
-    const long long pair0 = (long long)tinfo[buf * 4 + 2] - a.s0;
-    if (b != cur_b) {  // every MMA that read the old operand has completed (its accumulators were drained)
-      cur_b = b;
-      if (tid == 0) {
-        const uint32_t bar = smem_u32(&bars[2]);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)Sh::BBYTES)
-                     : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(b_base),
-            "l"(a.B + (size_t)b * Sh::BBYTES), "r"((uint32_t)Sh::BBYTES), "r"(bar)
-            : "memory");
+  // ------------------------------------------------------------------ issue
+  // Job number g (counted over the CTA's tiles) is issued by warp g mod 16, so that the time a thread is held while
+  // the tensor core takes its MMAs (73 cycles each) is spread over the warps. Its accumulator is free once every warp
+  // has read job g - 4.
+  const uint32_t idesc = (1u << 4) | ((uint32_t)(kIbN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);  // F16 in, F32 out
+  const uint64_t da = tc_desc<kIbKC>(smem_u32(As)), db = tc_desc<kIbKC>(smem_u32(Bs));
+  const uint32_t dal = (uint32_t)da, dbl = (uint32_t)db, dhi = (uint32_t)(da >> 32);
+  auto issue = [&](uint32_t g, int pass, auto weight) {
+    int ok = 1;
+    if (lane == 0) {
+      if (g >= 4) ok = tc_wait1(smem_u32(&S.dempty[g & 3]), ((g >> 2) - 1) & 1);
+      if (ok) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        ib_issue<decltype(weight)::value>(tmem + (g & 3) * kIbN, dal, dbl + (uint32_t)(pass * (kIbOperand >> 4)), dhi, idesc);
+        tc_commit(smem_u32(&S.dfull[g & 3]));
       }
-      ++bloads;
     }
-    // ---------------------------------------------------------------- rotate and cut into digits
-    {
+    return __shfl_sync(kTcFull, ok, 0) != 0;
+  };
+    // rotate the columns of tile ti and cut them into digits
+    auto form = [&](int ti) {
+      IbTile &t = S.tile[ti & 3];
       const int rl = lane & 7, chunk = lane >> 3, row = warp * 8 + rl, col = row >> 1, part = row & 1;
-      const int *eb = ex + buf * 64;
-      const bool have = col < ncol;
-      double v[8];
-      int e[8], emax = 0;
-      const double2 *xp = a.x + (have ? xoff[buf * kIbCols + col] : 0);
-      double2 xv[8];
+      const bool have = col < t.ncol;
+      if (warp * 4 < t.ncol) {
+        const double *xp = a.x + (have ? t.xoff[col] + part : 0);
+        double xv[8];
+        int emax = 0;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int n2 = chunk * 8 + q;
-        xv[q] = have && n2 < bs ? __ldg(xp + (size_t)n2 * a.R) : make_double2(0.0, 0.0);
-      }
+        for (int q = 0; q < 8; ++q) {
+          const int n2 = chunk * 8 + q;
+          xv[q] = have && n2 < bs ? __ldg(xp + 2 * (size_t)n2 * a.R) : 0.0;
+        }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int n2 = chunk * 8 + q;
-        const int m = mofn_s[n2];
-        double2 p = ph[(size_t)(buf * kIbCols + (have ? col : 0)) * PHS + (m < 0 ? -m : m)];
-        if (m < 0) p.y = -p.y;
-        v[q] = part ? fma(p.x, xv[q].y, p.y * xv[q].x) : fma(p.x, xv[q].x, -p.y * xv[q].y);
-        if (!have) v[q] = 0.0;
-        const int f = (__double2hiint(v[q]) >> 20) & 0x7FF;
-        e[q] = f + eb[n2];
-        if (f == 0x7FF) emax = 1 << 20;  // Inf or NaN: the column's result is NaN
-        else if (f != 0) emax = max(emax, e[q] + 4096);
-      }
-      emax = max(emax, __shfl_xor_sync(kTcFull, emax, 1));
-      emax = max(emax, __shfl_xor_sync(kTcFull, emax, 8));
-      emax = max(emax, __shfl_xor_sync(kTcFull, emax, 16));
-      if (part == 0 && chunk == 0) cexp[col] = emax;
-      const int es = emax - 4096;  // |u| < 2^(es - 1022)
-      const double t = have ? tf[buf * kIbCols + col] : 0.0;
-      const double t2 = t * t;
-      unsigned char *dst = As + (size_t)(row >> 3) * (KC * 128) + (row & 7) * 16;
-#pragma unroll
-      for (int h = 0; h < NC / 2; ++h) {
+        for (int q = 0; q < 8; ++q) {
+          const int f = ib_field(xv[q]);
+          if (f != 0) emax = max(emax, f == 0x7FF ? 1 << 20 : f + t.eb[chunk * 8 + q] + 4096);  // Inf, NaN: see below
+        }
+        emax = max(emax, __shfl_xor_sync(kTcFull, emax, 1));
+        emax = max(emax, __shfl_xor_sync(kTcFull, emax, 8));
+        emax = max(emax, __shfl_xor_sync(kTcFull, emax, 16));
+        if (part == 0 && chunk == 0) t.cexp[col] = emax;
+        const int es = emax - 4096;  // |Re x|, |Im x| < 2^(es - 1022) under the column exponents
+        const int4 *pc = t.ph[have ? col : 0];
+        unsigned char *dst = As + (size_t)(row >> 3) * (kIbKC * 128) + (row & 7) * 16 +
+                             chunk * 128;
         uint32_t o[kIbDig][4];
 #pragma unroll
         for (int q = 0; q < 8; q += 2) {
-          unsigned long long f[2];
+          long long u[2];
 #pragma unroll
           for (int w = 0; w < 2; ++w) {
-            const double val = h == 0 ? v[q + w] : t2 * v[q + w];
-            const int fe = (__double2hiint(val) >> 20) & 0x7FF;
-            f[w] = ib_fixed(val, es - (fe + (e[q + w] - ((__double2hiint(v[q + w]) >> 20) & 0x7FF))));
+            const int n2 = chunk * 8 + q + w, m = S.mofn[n2];
+            const IbWords f = ib_split(ib_fixed<9>(xv[q + w], es - t.eb[n2] - ib_field(xv[q + w])));
+            const int oh = __shfl_xor_sync(kTcFull, f.h, 1), ol = __shfl_xor_sync(kTcFull, f.l, 1);
+            // half of Re = c xr - s xi or Im = c xi + s xr
+            int4 p = pc[m < 0 ? -m : m];
+            if ((m < 0) == (part != 0)) {
+              p.z = -p.z;
+              p.w = -p.w;
+            }
+            const long long mid = ib_mad(f.h, p.y, ib_mad(f.l, p.x, ib_mad(oh, p.w, ib_mad(ol, p.z, 0x40000000ll))));
+            u[w] = ib_mad(f.h, p.x, ib_mad(oh, p.z, mid >> 31));
           }
           uint32_t dg[kIbDig];
-          ib_digits(f[0], f[1], dg);
+          ib_digits(u[0], u[1], dg);
 #pragma unroll
           for (int s = 0; s < kIbDig; ++s) o[s][q >> 1] = dg[s];
         }
 #pragma unroll
         for (int s = 0; s < kIbDig; ++s)
-          *reinterpret_cast<uint4 *>(dst + (size_t)s * Sh::ASLICE + (h * 4 + chunk) * 128) =
-              make_uint4(o[s][0], o[s][1], o[s][2], o[s][3]);
+          *reinterpret_cast<uint4 *>(dst + (size_t)s * kIbSlice) = make_uint4(o[s][0], o[s][1], o[s][2], o[s][3]);
       }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
-      good = tc_wait1(smem_u32(&bars[2]), (uint32_t)((bloads - 1) & 1));
-      if (good) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        issue(0);
-        if (nq > 1) issue(1);
-        issued = true;
-      }
-    }
-    good = __shfl_sync(kTcFull, (int)good, 0) != 0;  // one decision per warp
-    look_ahead(T + 1, buf ^ 1);
-    // ---------------------------------------------------------------- read back, combine, rotate back
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc_arrive(smem_u32(&S.afull));
+    };
     const int sp = warp & 3, grp = warp >> 2;
-    const int col = sp * 16 + (lane >> 1), part = lane & 1;
-    const bool have = col < ncol;
-    const double t = have ? tf[buf * kIbCols + col] : 0.0;
-    const int ce = have ? cexp[col] : 0;
-    const int cs = ce - 4096 - 1022;
-    const double2 *pc = ph + (size_t)(buf * kIbCols + (have ? col : 0)) * PHS;
-    double *vo = reinterpret_cast<double *>(a.V + (pair0 * a.rt + (have ? col : 0)) * bs) + part;
-    for (int q = 0; q < nq; ++q) {
-      bool ok = good;
-      if (ok) {
-        const int u = (q & 1) ? uses1 : uses0;
-        ok = tc_waitw(smem_u32(&bars[q & 1]), (uint32_t)(u & 1));
-      }
-      if (q & 1) ++uses1;
-      else ++uses0;
-      const int n1 = q * 8 + grp * 2;
-      if (ok && sp * 16 < ncol && n1 < bs) {
+    const int col = sp * 16 + (lane >> 1), part = lane & 1, sg = part ? -1 : 1;
+    const uint32_t lanes = tmem + ((uint32_t)(sp * 32) << 16) + (uint32_t)(grp * 32);
+    uint32_t g = 0;  // jobs read
+    // waits for the next job (weight D of pass p); read() gets 16 of this warp's 32 columns at a time; then the
+    // buffer is free for the job after next three, whose issuing warp sends it off
+    auto job = [&](auto weight, int p, bool work, auto &&read) {
+      constexpr int D = decltype(weight)::value, DN = D >= 4 ? D - 4 : D + 3;
+      if (!tc_waitw(smem_u32(&S.dfull[g & 3]), (g >> 2) & 1)) return false;
+      if (work) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        float f[kIbDig][8];
-        const uint32_t base = tmem + ((uint32_t)(sp * 32) << 16) + (uint32_t)((q & 1) * DBUF + grp * 8);
 #pragma unroll
-        for (int d = 0; d < kIbDig; ++d) tmem_ld8(base + d * kIbGroupN, f[d]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        long long w[8];
+        for (int h = 0; h < 32; h += 16) {
+          float f[16];
+          tmem_ld16(lanes + (g & 3) * kIbN + h, f);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const long long hi = ((long long)__float2int_rn(f[0][c]) << 20) + ((long long)__float2int_rn(f[1][c]) << 10) +
-                               __float2int_rn(f[2][c]);
-          const long long lo = ((long long)__float2int_rn(f[3][c]) << 20) + ((long long)__float2int_rn(f[4][c]) << 10) +
-                               __float2int_rn(f[5][c]);
-          w[c] = (hi << 18) + ((lo + 2048) >> 12);  // in units of 2^-56 of the scales
+          for (int c = 0; c < 16; ++c) read(h + c, f[c]);
         }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      }
+      __syncwarp();
+      if (lane == 0) tc_arrive(smem_u32(&S.dempty[g & 3]));
+      ++g;
+      const int pn = D >= 4 ? p : p + 1;
+      return ((g + 3) & (kIbWarps - 1)) != warp || pn >= passes || issue(g + 3, pn, std::integral_constant<int, DN>());
+    };
+    int cur_b = -1, bloads = 0;
+    look(0);
+    look(1);
+    for (int ti = 0; ti < NT && good; ++ti) {
+      IbTile &t = S.tile[ti & 3];
+      look(ti + 2);
+      if (!tc_waitw(smem_u32(&S.meta[ti & 3]), (uint32_t)((ti >> 2) & 1))) {
+        good = false;
+        break;
+      }
+      // every job of the last tile has been read: its operands are free
+      if (t.bucket != cur_b) {
+        cur_b = t.bucket;
+        ++bloads;
+        if (warp == 0 && lane == 0) {
+          const uint32_t bar = smem_u32(&S.bfull), bytes = (uint32_t)(passes * kIbOperand);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                  smem_u32(Bs)),
+              "l"(a.B + (size_t)cur_b * Sh::BBYTES), "r"(bytes), "r"(bar)
+              : "memory");
+        }
+      }
+      form(ti);
+      const int mine = (int)((uint32_t)warp - g) & (kIbWarps - 1);  // the tile's first four jobs
+      if (mine < 4) {
+        good = tc_waitw(smem_u32(&S.afull), (uint32_t)(ti & 1)) &&
+               tc_waitw(smem_u32(&S.bfull), (uint32_t)((bloads - 1) & 1));
+        if (good) {
+          if (mine == 0) good = issue(g, 0, std::integral_constant<int, 6>());
+          else if (mine == 1) good = issue(g + 1, 0, std::integral_constant<int, 5>());
+          else if (mine == 2) good = issue(g + 2, 0, std::integral_constant<int, 4>());
+          else good = issue(g + 3, 0, std::integral_constant<int, 3>());
+        }
+      }
+      for (int p = 0; p < passes && good; ++p) {
+        const int n0 = p * PN + grp * WN;
+        const bool work = sp * 16 < t.ncol && n0 < bs;
+        // The digits in units of 2^-55 of the scales; the Im rows of C are negated in the Im u lanes. What is
+        // below 2^22 becomes an integer by an FP32 addition, whose exponent bits are taken off again.
+        auto integer = [](float f) { return __float_as_int(f) - 0x4B400000; };  // f = n + 1.5 2^23
+        auto unit = [&](int c, int u) { return c & 1 ? sg * u : u; };
+        int lo[32];
+        long long w[32] = {};
+        std::integral_constant<int, 6> w6;
+        std::integral_constant<int, 5> w5;
+        std::integral_constant<int, 4> w4;
+        std::integral_constant<int, 3> w3;
+        std::integral_constant<int, 2> w2;
+        std::integral_constant<int, 1> w1;
+        std::integral_constant<int, 0> w0;
+        good = job(w6, p, work, [&](int c, float f) { lo[c] = __float_as_int(f); });
+        good = good && job(w5, p, work, [&](int c, float f) {
+          lo[c] = integer(fmaf(fmaf(__int_as_float(lo[c]), 0x1p-9f, f), c & 1 ? sg * 0x1p-6f : 0x1p-6f, 12582912.f));
+        });
+        good = good && job(w4, p, work, [&](int c, float f) { lo[c] += __float2int_rn(f) * unit(c, 8); });
+        good = good && job(w3, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 12), lo[c]); });
+        good = good && job(w2, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 21), w[c]); });
+        good = good && job(w1, p, work, [&](int c, float f) {
+          w[c] = ib_mad(integer(f + 12582912.f), unit(c, 1 << 30), w[c]);
+        });
+        good = good && job(w0, p, work, [&](int c, float f) {
+          const unsigned n = (unsigned)(integer(f + 12582912.f) * unit(c, 1 << 7));
+          w[c] += (long long)((unsigned long long)n << 32);
+        });
+        if (!good || !work) continue;
+        const bool have = col < t.ncol;
+        const int2 tw = have ? t.t[col] : make_int2(0, 0);
+        const int ce = have ? t.cexp[col] : 0;
+        const int cs = ce - 4096 - 1022 + 1 - 55;  // scale of x, half of its rotation, units
+        const int4 *pc = t.ph[have ? col : 0];
+        double *vo = a.V + 2 * ((t.pair0 * a.rt + (have ? col : 0)) * bs) + part;
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < WN; ++s) {
+          const int n = n0 + s;
           // lane pair (Re u, Im u): Re y = C_re u_re - C_im u_im, Im y = C_re u_im + C_im u_re
-          const long long oe = __shfl_xor_sync(kTcFull, w[s * 4 + 1], 1), oo = __shfl_xor_sync(kTcFull, w[s * 4 + 3], 1);
-          const double E = ib_ll2d(part ? w[s * 4] + oe : w[s * 4] - oe);
-          const double O = ib_ll2d(part ? w[s * 4 + 2] + oo : w[s * 4 + 2] - oo);
-          const int n = n1 + s;
-          double val = ib_scale(fma(t, O, E), cs + ex[buf * 64 + 32 + (n & 31)] - 56);
-          if (ce >= (1 << 20)) val = __longlong_as_double(0x7FF8000000000000ll);
-          const double other = __shfl_xor_sync(kTcFull, val, 1);
-          const int m = mofn_s[n & 31];
-          const double2 p = pc[m < 0 ? -m : m];
-          // times e^{-i m phi}
-          const double sg = (m < 0) != (part != 0) ? -p.y : p.y;
-          const double out = fma(p.x, val, sg * other);
-          if (have && n < bs) vo[2 * n] = out;
+          long long acc = 0;
+#pragma unroll
+          for (int c = NC - 1; c >= 0; --c) {
+            const long long e = w[s * RN + 2 * c] + __shfl_xor_sync(kTcFull, w[s * RN + 2 * c + 1], 1);
+            acc = c == NC - 1 ? e : ib_mul(ib_split(acc), tw.x, tw.y, e);
+          }
+          const IbWords v = ib_split(acc);
+          const int oh = __shfl_xor_sync(kTcFull, v.h, 1), ol = __shfl_xor_sync(kTcFull, v.l, 1);
+          const int m = S.mofn[n & 31];
+          int4 ph = pc[m < 0 ? -m : m];
+          if ((m < 0) != (part != 0)) {
+            ph.z = -ph.z;
+            ph.w = -ph.w;
+          }
+          // e^{-i m phi} times the value: c v +- s (other part)
+          const long long mid = ib_mad(v.h, ph.y, ib_mad(v.l, ph.x, ib_mad(oh, ph.w, ib_mad(ol, ph.z, 0x20000000ll))));
+          const long long out = 2 * ib_mad(v.h, ph.x, (long long)oh * ph.z) + (mid >> 30);
+          double res = ib_to_double(out, cs + t.ea[n & 31]);
+          if (ce >= (1 << 20)) res = __longlong_as_double(0x7FF8000000000000ll);  // Inf or NaN in x
+          if (have && n < bs) vo[2 * n] = res;
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      good = __syncthreads_and(ok);
-      if (!good) break;
-      if (tid == 0 && q + 2 < nq) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        issue(q + 2);
-      }
     }
+  if (!good && lane == 0) atomicExch(a.err, 1);
+  // nothing of this CTA may be in flight when its memory is given back
+  if (lane == 0) {
+    tc_commit(smem_u32(&S.done));
+    if (!tc_wait1(smem_u32(&S.done), 0u)) atomicExch(a.err, 1);
+    if (warp == 0 && bloads > 0) tc_wait1(smem_u32(&S.bfull), (uint32_t)((bloads - 1) & 1));
   }
-  if (tid == 0) {
-    if (!good) atomicExch(a.err, 1);
-    if (bloads > 0) tc_wait1(smem_u32(&bars[2]), (uint32_t)((bloads - 1) & 1));
-    if (issued) {
-      tc_commit(smem_u32(&bars[3]));
-      if (!tc_wait1(smem_u32(&bars[3]), 0u)) atomicExch(a.err, 1);
-    }
-  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -520,59 +633,61 @@ template <int NC>
 __global__ void __launch_bounds__(256) ib_operand_kernel(const double2 *coef, const int *bk, int bs, unsigned char *B,
                                                          int *exps) {
   using Sh = IbShape<NC>;
-  __shared__ int eb[kIbBP], ea[kIbBP];
+  __shared__ int eb[kIbK], ea[kIbK];
   const int tid = threadIdx.x, b = blockIdx.x, bs2 = bs * bs;
   const double2 *C = coef + (size_t)bk[b] * NC * bs2;
-  if (tid < kIbBP) eb[tid] = ea[tid] = -(1 << 20);
+  if (tid < kIbK) {
+    eb[tid] = ea[tid] = -(1 << 20);
+  }
   __syncthreads();
-  auto field = [](double v) { return (__double2hiint(v) >> 20) & 0x7FF; };
   for (int e = tid; e < NC * bs2; e += blockDim.x) {
-    const int f = max(field(C[e].x), field(C[e].y));
+    const int f = max(ib_field(C[e].x), ib_field(C[e].y));
     if (f) atomicMax(&eb[(e % bs2) / bs], f - 1022);
   }
   __syncthreads();
+  if (tid < kIbK && eb[tid] == -(1 << 20)) eb[tid] = 0;
+  __syncthreads();
   for (int e = tid; e < NC * bs2; e += blockDim.x) {
-    const int f = max(field(C[e].x), field(C[e].y)), n2 = (e % bs2) / bs;
-    if (f) atomicMax(&ea[e % bs], f - 1022 - eb[n2]);
+    const int f = max(ib_field(C[e].x), ib_field(C[e].y));
+    if (f) atomicMax(&ea[e % bs], f - 1022 - eb[(e % bs2) / bs]);
   }
   __syncthreads();
-  if (tid < kIbBP) {
-    if (eb[tid] == -(1 << 20)) eb[tid] = 0;
-    if (ea[tid] == -(1 << 20)) ea[tid] = 0;
+  if (tid < kIbK && ea[tid] == -(1 << 20)) ea[tid] = 0;
+  __syncthreads();
+  if (tid < kIbK) {
     exps[(size_t)b * 64 + tid] = eb[tid];
     exps[(size_t)b * 64 + 32 + tid] = ea[tid];
   }
-  __syncthreads();
   unsigned char *out = B + (size_t)b * Sh::BBYTES;
-  // one thread per (n1, part, parity of c, pair of k): k = (c / 2) * 32 + n2
-  for (int e = tid; e < 128 * Sh::K / 2; e += blockDim.x) {
-    const int row = e / (Sh::K / 2), k = 2 * (e - row * (Sh::K / 2));
-    const int n1 = row >> 2, im = row & 1, odd = (row >> 1) & 1;  // row of the operand: n1, then Re/Im, even/odd
-    unsigned long long f[2];
+  // one thread per row (n1, power, part) and pair of n2
+  for (int e = tid; e < Sh::PASSES * kIbN * kIbK / 2; e += blockDim.x) {
+    const int row = e / (kIbK / 2), k = 2 * (e - row * (kIbK / 2));
+    const int n1 = row / Sh::RN, c = (row % Sh::RN) >> 1, im = row & 1;
+    long long f[2];
     for (int w = 0; w < 2; ++w) {
-      const int n2 = (k + w) % kIbBP, c = 2 * ((k + w) / kIbBP) + odd;
+      const int n2 = k + w;
       double v = 0.0;
       if (n1 < bs && n2 < bs) {
         const double2 cv = C[(size_t)c * bs2 + n2 * bs + n1];
         v = im ? cv.y : cv.x;
       }
-      f[w] = ib_fixed(v, n1 < bs && n2 < bs ? ea[n1] + eb[n2] + 1022 - field(v) : 0);
+      f[w] = ib_fixed<9>(v, n1 < bs && n2 < bs ? ea[n1] + eb[n2] + 1022 - ib_field(v) : 0);
     }
     uint32_t dg[kIbDig];
     ib_digits(f[0], f[1], dg);
-    const int q = n1 >> 3, rq = row & 31;
+    const int pass = row / kIbN, r = row % kIbN;
     for (int s = 0; s < kIbDig; ++s)
-      *reinterpret_cast<uint32_t *>(out + (size_t)(q * kIbDig + s) * Sh::BSLICE +
-                                    ((size_t)(rq >> 3) * Sh::KC + (k >> 3)) * 128 + (rq & 7) * 16 + (k & 7) * 2) = dg[s];
+      *reinterpret_cast<uint32_t *>(out + (size_t)pass * kIbOperand + (size_t)s * kIbSlice +
+                                    ((size_t)(r >> 3) * kIbKC + (k >> 3)) * 128 + (r & 7) * 16 + (k & 7) * 2) = dg[s];
   }
 }
 
 static constexpr int kIbMinParticles = 32;
 static constexpr long long kIbMaxPairs = 1ll << 27;      // 4 GB of pair records
-static constexpr size_t kIbWorkspace = (size_t)1 << 30;  // bytes of V per chunk
+static constexpr size_t kIbWorkspace = (size_t)2 << 30;  // bytes of V per chunk
 
 bool ib_supported(const sg_context *c) {
-  if (c->vol || c->kind < 0 || c->bs > kIbBP) return false;
+  if (c->vol || c->kind < 0 || c->bs > kIbMaxB) return false;
   if ((long long)c->n * c->n > kIbMaxPairs || c->n < kIbMinParticles) return false;
   for (int m : c->h_mofn)
     if (m > kIbMaxM || m < -kIbMaxM) return false;
@@ -655,8 +770,8 @@ template <int NC>
 static void ib_launch(const IbArgs &a, cudaStream_t st) {
   static bool attr_done[64] = {};
   if (first_on_device(attr_done))
-    SG_CUDA(cudaFuncSetAttribute(ib_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IbShape<NC>::SMEM));
-  ib_kernel<NC><<<std::min(sm_count(), a.t1 - a.t0), kIbThreads, IbShape<NC>::SMEM, st>>>(a);
+    SG_CUDA(cudaFuncSetAttribute(ib_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ib_smem<NC>()));
+  ib_kernel<NC><<<std::min(sm_count(), a.t1 - a.t0), kIbThreads, ib_smem<NC>(), st>>>(a);
   SG_CUDA(cudaGetLastError());
 }
 
@@ -699,9 +814,9 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     a.toff = tl.toff.ptr;
     a.B = P.B.ptr;
     a.exps = P.exps.ptr;
-    a.x = x;
+    a.x = reinterpret_cast<const double *>(x);
     a.mofn = c->mofn.ptr;
-    a.V = P.V.ptr;
+    a.V = reinterpret_cast<double *>(P.V.ptr);
     a.nb = P.nb;
     a.bs = bs;
     a.mmax = mmax;
