@@ -28,7 +28,7 @@
 //   * the warps rotate x_j, cut u into digits and store them as the A operand (128 rows: Re and Im of 64
 //     columns, K = 32);
 //   * one thread issues the digit products against the interval's B operand (resident while the
-//     interval lasts): passes of 128 rows (n1, power of t, Re / Im), one job per weight d = 6..0 in a
+//     interval lasts): passes of 128 rows (n1, power of t, Re / Im), one job per weight d = 0..6 in a
 //     ring of four tensor-memory accumulators of 128 columns;
 //   * the warps read the jobs back (32 columns per warp), combine digits, real and imaginary parts
 //     (neighbouring lanes) and powers of t, rotate back and store the pair's contribution V.
@@ -71,6 +71,11 @@ static constexpr unsigned long long ib_bias() {
 }
 static constexpr unsigned long long kIbBias = ib_bias();
 static_assert(kIbDig * kIbMaxB * (1 << (2 * kIbBits - 2)) <= (1 << 24), "exact FP32 accumulators");
+// 1.5 2^23, and what its bits add to a combination of digits
+static constexpr float kIbMagic = 12582912.f;
+static constexpr unsigned long long kIbOffset =
+    ((unsigned long long)(0x4B400000u * 128u) << 32) + 0x4B400000ull * ((1ull << 30) + 1 + 1);
+
 // largest t in units of 2^-62 whose high word fits (t < 1 up to its last places)
 static constexpr long long kIbBelowOne = (1ll << 62) - (1ll << 30) - 1;
 
@@ -93,8 +98,14 @@ struct IbTile {
   long long pair0;                // first pair, from the start of V
 };
 
+static constexpr int kIbXPitch = 31;  // x_j of a column: element n2 at (n2 mod 8) 4 + n2 / 8
+
 struct IbSmem {
   IbTile tile[4];
+  IbRec rec[2][kIbCols];              // records, exponents and (columns, bucket, first pair) of the next tiles
+  int exps[2][64];
+  int next[2][3];
+  double2 x[kIbCols * kIbXPitch];     // x_j of the next tile's columns
   uint64_t dfull[4], dempty[4], afull, meta[4], bfull, done;
   int mofn[kIbK];
   uint32_t tmem;
@@ -146,6 +157,10 @@ __device__ __forceinline__ void ib_digits(long long v0, long long v1, uint32_t (
     const __half2 h = __hadd2(*reinterpret_cast<const __half2 *>(&p), __floats2half2_rn(-1280.f, -1280.f));
     d[s] = *reinterpret_cast<const uint32_t *>(&h);
   }
+}
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
 // Products of 62-bit fixed-point numbers from 31-bit words: three 32 x 32 -> 64 bit multiply-adds, low
@@ -260,45 +275,61 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
     S.lb[look_half] = lb;
     __syncwarp();
   }
-  auto look = [&](int ti) {
+  // records of tile ti on their way to shared memory
+  auto look_fetch = [&](int ti) {
     if (look_half < 0 || ti >= NT) return;
-    IbTile &t = S.tile[ti & 3];
     const int T = T0 + ti;
     int lb = S.lb[look_half];
     while (T >= a.toff[lb + 1]) ++lb;
+    const int p0 = a.boff[lb] + (T - a.toff[lb]) * a.per, p1 = min(a.boff[lb + 1], p0 + a.per);
     __syncwarp();
     S.lb[look_half] = lb;
-    const int p0 = a.boff[lb] + (T - a.toff[lb]) * a.per, p1 = min(a.boff[lb + 1], p0 + a.per);
-    const int ncol = (p1 - p0) * a.rt;
+    if (look_half == 0 && lane == 0) {
+      S.next[ti & 1][0] = (p1 - p0) * a.rt;
+      S.next[ti & 1][1] = lb;
+      S.next[ti & 1][2] = p0;
+    }
+    if (lane < 8)
+      cp_async16(&S.exps[ti & 1][32 * look_half + 4 * lane], a.exps + (size_t)lb * 64 + 32 * look_half + 4 * lane);
+    const int c = look_half * 32 + lane;
+    if (c < (p1 - p0) * a.rt) {
+      const IbRec *r = a.rec + p0 + c / a.rt;
+      cp_async16(&S.rec[ti & 1][c], r);
+      cp_async16(reinterpret_cast<char *>(&S.rec[ti & 1][c]) + 16, reinterpret_cast<const char *>(r) + 16);
+    }
+  };
+  // the words of its t and phases
+  auto look_form = [&](int ti) {
+    if (look_half < 0 || ti >= NT) return;
+    IbTile &t = S.tile[ti & 3];
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    const int c = look_half * 32 + lane;
+    const IbRec rc = S.rec[ti & 1][c];  // unused columns hold an old record
     if (look_half == 0) {
-      t.eb[lane] = a.exps[(size_t)lb * 64 + lane];
+      t.eb[lane] = S.exps[ti & 1][lane];
       if (lane == 0) {
-        t.ncol = ncol;
-        t.bucket = lb;
-        t.pair0 = p0 - a.s0;
+        t.ncol = S.next[ti & 1][0];
+        t.bucket = S.next[ti & 1][1];
+        t.pair0 = S.next[ti & 1][2] - a.s0;
       }
     } else {
-      t.ea[lane] = a.exps[(size_t)lb * 64 + 32 + lane];
+      t.ea[lane] = S.exps[ti & 1][32 + lane];
     }
-    const int c = look_half * 32 + lane;
-    if (c < ncol) {
-      const int p = p0 + c / a.rt, r = c % a.rt;
-      const IbRec rc = a.rec[p];
-      auto words = [](double v, int up) {  // v in units of 2^-up, |v| <= 1
-        return ib_split_signed(min(ib_fixed<10>(v, 1023 + 62 - up - ib_field(v)), kIbBelowOne));
-      };
-      const IbWords tw = words(rc.t, 62);
-      t.t[c] = make_int2(tw.h, tw.l);
-      t.xoff[c] = 2 * ((long long)rc.j * bs * a.R + a.r0 + r);
-      t.ph[c][0] = make_int4(1 << 30, 0, 0, 0);
-      double pr = rc.c, pi = rc.s;
-      for (int m = 1; m <= a.mmax; ++m) {
-        const IbWords cw = words(pr, 61), sw = words(pi, 61);
-        t.ph[c][m] = make_int4(cw.h, cw.l, sw.h, sw.l);
-        const double nr = pr * rc.c - pi * rc.s;
-        pi = pr * rc.s + pi * rc.c;
-        pr = nr;
-      }
+    auto words = [](double v, int up) {  // v in units of 2^-up, |v| <= 1
+      return ib_split_signed(min(ib_fixed<10>(v, 1023 + 62 - up - ib_field(v)), kIbBelowOne));
+    };
+    const IbWords tw = words(rc.t, 62);
+    t.t[c] = make_int2(tw.h, tw.l);
+    t.xoff[c] = 2 * ((long long)rc.j * bs * a.R + a.r0 + c % a.rt);
+    t.ph[c][0] = make_int4(1 << 30, 0, 0, 0);
+    double pr = rc.c, pi = rc.s;
+    for (int m = 1; m <= a.mmax; ++m) {
+      const IbWords cw = words(pr, 61), sw = words(pi, 61);
+      t.ph[c][m] = make_int4(cw.h, cw.l, sw.h, sw.l);
+      const double nr = pr * rc.c - pi * rc.s;
+      pi = pr * rc.s + pi * rc.c;
+      pr = nr;
     }
     __syncwarp();
     if (lane == 0) tc_arrive(smem_u32(&S.meta[ti & 3]));
@@ -322,20 +353,28 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
     }
     return __shfl_sync(kTcFull, ok, 0) != 0;
   };
+    // x_j of this warp's four columns of tile ti on their way to shared memory
+    auto fetch = [&](int ti) {
+      const IbTile &t = S.tile[ti & 3];
+      const int chunk = lane >> 3, q = lane & 7, n2 = chunk * 8 + q;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int col = warp * 4 + c;
+        if (col < t.ncol && n2 < bs)
+          cp_async16(&S.x[col * kIbXPitch + q * 4 + chunk], a.x + t.xoff[col] + 2 * (size_t)n2 * a.R);
+      }
+    };
     // rotate the columns of tile ti and cut them into digits
     auto form = [&](int ti) {
       IbTile &t = S.tile[ti & 3];
       const int rl = lane & 7, chunk = lane >> 3, row = warp * 8 + rl, col = row >> 1, part = row & 1;
       const bool have = col < t.ncol;
       if (warp * 4 < t.ncol) {
-        const double *xp = a.x + (have ? t.xoff[col] + part : 0);
+        const double *xp = reinterpret_cast<const double *>(S.x + col * kIbXPitch + chunk) + part;
         double xv[8];
         int emax = 0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int n2 = chunk * 8 + q;
-          xv[q] = have && n2 < bs ? __ldg(xp + 2 * (size_t)n2 * a.R) : 0.0;
-        }
+        for (int q = 0; q < 8; ++q) xv[q] = have && chunk * 8 + q < bs ? xp[8 * q] : 0.0;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int f = ib_field(xv[q]);
@@ -387,7 +426,7 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
     // waits for the next job (weight D of pass p); read() gets 16 of this warp's 32 columns at a time; then the
     // buffer is free for the job after next three, whose issuing warp sends it off
     auto job = [&](auto weight, int p, bool work, auto &&read) {
-      constexpr int D = decltype(weight)::value, DN = D >= 4 ? D - 4 : D + 3;
+      constexpr int D = decltype(weight)::value, DN = D <= 2 ? D + 4 : D - 3;
       if (!tc_waitw(smem_u32(&S.dfull[g & 3]), (g >> 2) & 1)) return false;
       if (work) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -404,19 +443,21 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
       __syncwarp();
       if (lane == 0) tc_arrive(smem_u32(&S.dempty[g & 3]));
       ++g;
-      const int pn = D >= 4 ? p : p + 1;
+      const int pn = D <= 2 ? p : p + 1;
       return ((g + 3) & (kIbWarps - 1)) != warp || pn >= passes || issue(g + 3, pn, std::integral_constant<int, DN>());
     };
     int cur_b = -1, bloads = 0;
-    look(0);
-    look(1);
+    auto wait_meta = [&](int ti) { return tc_waitw(smem_u32(&S.meta[ti & 3]), (uint32_t)((ti >> 2) & 1)); };
+    look_fetch(0);
+    look_form(0);
+    look_fetch(1);
+    look_form(1);
+    look_fetch(2);
+    good = NT == 0 || wait_meta(0);
+    if (good && NT > 0) fetch(0);
     for (int ti = 0; ti < NT && good; ++ti) {
       IbTile &t = S.tile[ti & 3];
-      look(ti + 2);
-      if (!tc_waitw(smem_u32(&S.meta[ti & 3]), (uint32_t)((ti >> 2) & 1))) {
-        good = false;
-        break;
-      }
+      look_form(ti + 2);
       // every job of the last tile has been read: its operands are free
       if (t.bucket != cur_b) {
         cur_b = t.bucket;
@@ -431,15 +472,23 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
               : "memory");
         }
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
       form(ti);
+      look_fetch(ti + 3);
+      if (ti + 1 < NT) {
+        good = wait_meta(ti + 1);
+        if (!good) break;
+        fetch(ti + 1);
+      }
       const int mine = (int)((uint32_t)warp - g) & (kIbWarps - 1);  // the tile's first four jobs
       if (mine < 4) {
         good = tc_waitw(smem_u32(&S.afull), (uint32_t)(ti & 1)) &&
                tc_waitw(smem_u32(&S.bfull), (uint32_t)((bloads - 1) & 1));
         if (good) {
-          if (mine == 0) good = issue(g, 0, std::integral_constant<int, 6>());
-          else if (mine == 1) good = issue(g + 1, 0, std::integral_constant<int, 5>());
-          else if (mine == 2) good = issue(g + 2, 0, std::integral_constant<int, 4>());
+          if (mine == 0) good = issue(g, 0, std::integral_constant<int, 0>());
+          else if (mine == 1) good = issue(g + 1, 0, std::integral_constant<int, 1>());
+          else if (mine == 2) good = issue(g + 2, 0, std::integral_constant<int, 2>());
           else good = issue(g + 3, 0, std::integral_constant<int, 3>());
         }
       }
@@ -447,37 +496,39 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
         const int n0 = p * PN + grp * WN;
         const bool work = sp * 16 < t.ncol && n0 < bs;
         // The digits in units of 2^-55 of the scales; the Im rows of C are negated in the Im u lanes. What is
-        // below 2^22 becomes an integer by an FP32 addition, whose exponent bits are taken off again.
-        auto integer = [](float f) { return __float_as_int(f) - 0x4B400000; };  // f = n + 1.5 2^23
+        // below 2^22 becomes an integer by an FP32 addition of 1.5 2^23, whose exponent bits stay in the sum
+        // and are taken off it (kIbOffset) below.
         auto unit = [&](int c, int u) { return c & 1 ? sg * u : u; };
-        int lo[32];
-        long long w[32] = {};
-        std::integral_constant<int, 6> w6;
-        std::integral_constant<int, 5> w5;
-        std::integral_constant<int, 4> w4;
-        std::integral_constant<int, 3> w3;
-        std::integral_constant<int, 2> w2;
-        std::integral_constant<int, 1> w1;
+        long long w[32];
         std::integral_constant<int, 0> w0;
-        good = job(w6, p, work, [&](int c, float f) { lo[c] = __float_as_int(f); });
-        good = good && job(w5, p, work, [&](int c, float f) {
-          lo[c] = integer(fmaf(fmaf(__int_as_float(lo[c]), 0x1p-9f, f), c & 1 ? sg * 0x1p-6f : 0x1p-6f, 12582912.f));
+        std::integral_constant<int, 1> w1;
+        std::integral_constant<int, 2> w2;
+        std::integral_constant<int, 3> w3;
+        std::integral_constant<int, 4> w4;
+        std::integral_constant<int, 5> w5;
+        std::integral_constant<int, 6> w6;
+        good = job(w0, p, work, [&](int c, float f) {
+          w[c] = (long long)((unsigned long long)(__float_as_uint(f + kIbMagic) * (unsigned)unit(c, 1 << 7)) << 32);
         });
-        good = good && job(w4, p, work, [&](int c, float f) { lo[c] += __float2int_rn(f) * unit(c, 8); });
-        good = good && job(w3, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 12), lo[c]); });
-        good = good && job(w2, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 21), w[c]); });
         good = good && job(w1, p, work, [&](int c, float f) {
-          w[c] = ib_mad(integer(f + 12582912.f), unit(c, 1 << 30), w[c]);
+          w[c] = ib_mad(__float_as_int(f + kIbMagic), unit(c, 1 << 30), w[c]);
         });
-        good = good && job(w0, p, work, [&](int c, float f) {
-          const unsigned n = (unsigned)(integer(f + 12582912.f) * unit(c, 1 << 7));
-          w[c] += (long long)((unsigned long long)n << 32);
+        good = good && job(w2, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 21), w[c]); });
+        good = good && job(w3, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 12), w[c]); });
+        good = good && job(w4, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 8), w[c]); });
+        good = good && job(w5, p, work, [&](int c, float f) {
+          w[c] = ib_mad(__float_as_int(fmaf(f, 0x1p-6f, kIbMagic)), unit(c, 1), w[c]);
+        });
+        good = good && job(w6, p, work, [&](int c, float f) {
+          w[c] = ib_mad(__float_as_int(fmaf(f, 0x1p-15f, kIbMagic)), unit(c, 1), w[c]);
         });
         if (!good || !work) continue;
         const bool have = col < t.ncol;
         const int2 tw = have ? t.t[col] : make_int2(0, 0);
         const int ce = have ? t.cexp[col] : 0;
         const int cs = ce - 4096 - 1022 + 1 - 55;  // scale of x, half of its rotation, units
+        // the Re lane receives the negated Im sum (offsets cancel), the Im lane adds two positive ones
+        const unsigned long long offset = part ? 0ull - 2ull * kIbOffset : 0ull;
         const int4 *pc = t.ph[have ? col : 0];
         double *vo = a.V + 2 * ((t.pair0 * a.rt + (have ? col : 0)) * bs) + part;
 #pragma unroll
@@ -487,7 +538,8 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
           long long acc = 0;
 #pragma unroll
           for (int c = NC - 1; c >= 0; --c) {
-            const long long e = w[s * RN + 2 * c] + __shfl_xor_sync(kTcFull, w[s * RN + 2 * c + 1], 1);
+            const long long e = (long long)((unsigned long long)w[s * RN + 2 * c] + offset +
+                                            (unsigned long long)__shfl_xor_sync(kTcFull, w[s * RN + 2 * c + 1], 1));
             acc = c == NC - 1 ? e : ib_mul(ib_split(acc), tw.x, tw.y, e);
           }
           const IbWords v = ib_split(acc);
