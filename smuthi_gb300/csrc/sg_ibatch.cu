@@ -19,7 +19,8 @@
 // one FP32 accumulator; smaller products (below 2^-60 of the scales) are dropped. A digit product is at
 // most 2^16 and K = 32 of them (at most 30 nonzero for blocksize <= 30) times d + 1 <= 7 pairs of digits
 // are summed, at most 7 * 30 * 2^16 = 13,762,560 < 2^24: every accumulator stays an exact integer
-// whatever the order of the sums. (Ten-bit digits would need fewer products, but the sums of the
+// whatever the order of the sums. Blocksizes 31 to 48 (K = 48) take 8-bit digits of 56-bit numbers and the
+// weights d = 0..7, at most 7 * 48 * 2^14 = 5,505,024 per accumulator. (Ten-bit digits would need fewer products, but the sums of the
 // middle weights could pass 2^24.) The digits are combined in 64-bit integers, in which the powers of
 // t and the rotations follow; the result is independent of how the pairs are grouped.
 //
@@ -28,8 +29,9 @@
 //   * the warps rotate x_j, cut u into digits and store them as the A operand (128 rows: Re and Im of 64
 //     columns, K = 32);
 //   * one thread issues the digit products against the interval's B operand (resident while the
-//     interval lasts): passes of 128 rows (n1, power of t, Re / Im), one job per weight d = 0..6 in a
-//     ring of four tensor-memory accumulators of 128 columns;
+//     interval lasts; with K = 48 one pass at a time, copied while the last pass is combined): passes of
+//     128 rows (n1, power of t, Re / Im), one job per weight d = 0..6 in a ring of four tensor-memory
+//     accumulators of 128 columns;
 //   * the warps read the jobs back (32 columns per warp), combine digits, real and imaginary parts
 //     (neighbouring lanes) and powers of t, rotate back and store the pair's contribution V.
 // A second kernel sums V over the emitters of every receiver in index order (deterministic) and forms
@@ -56,43 +58,56 @@ static constexpr int kIbWarps = 16;
 static constexpr int kIbThreads = 32 * kIbWarps;
 static constexpr int kIbCols = 64;   // complex columns per tile
 static constexpr int kIbDig = 7;     // digits per operand
-static constexpr int kIbBits = 9;    // bits per digit
-static constexpr int kIbK = 32;      // padded blocksize
-static constexpr int kIbMaxB = 30;   // largest blocksize whose accumulators are exact
-static constexpr int kIbMaxM = 3;    // largest |m| of the phase table
 static constexpr int kIbN = 128;     // B operand rows per pass: n1 x powers of t x (Re, Im)
-static constexpr int kIbKC = kIbK / 8;                 // core columns of 16 bytes
-static constexpr int kIbSlice = 128 * kIbK * 2;        // bytes of one digit of an operand
-static constexpr int kIbOperand = kIbDig * kIbSlice;   // bytes of an A operand or one pass of B
-static constexpr unsigned long long ib_bias() {
-  unsigned long long b = 0;
-  for (int i = 0; i < kIbDig; ++i) b |= 1ull << (kIbBits * i + kIbBits - 1);
-  return b;
-}
-static constexpr unsigned long long kIbBias = ib_bias();
-static_assert(kIbDig * kIbMaxB * (1 << (2 * kIbBits - 2)) <= (1 << 24), "exact FP32 accumulators");
-// 1.5 2^23, and what its bits add to a combination of digits
+// 1.5 2^23: added to an integer below 2^22 it leaves that in the mantissa
 static constexpr float kIbMagic = 12582912.f;
-static constexpr unsigned long long kIbOffset =
-    ((unsigned long long)(0x4B400000u * 128u) << 32) + 0x4B400000ull * ((1ull << 30) + 1 + 1);
-
+static constexpr unsigned long long kIbMagicBits = 0x4B400000ull;
 // largest t in units of 2^-62 whose high word fits (t < 1 up to its last places)
 static constexpr long long kIbBelowOne = (1ll << 62) - (1ll << 30) - 1;
 
-template <int NC>
+// KP: padded blocksize, 32 or 48
+template <int KP>
+struct IbNumbers {
+  static constexpr int BITS = KP == 32 ? 9 : 8;        // bits per digit
+  static constexpr int MAXB = KP == 32 ? 30 : 48;      // largest blocksize
+  static constexpr int MAXM = KP == 32 ? 3 : 4;        // largest |m| of the phase table
+  static constexpr int UP = KP == 32 ? 9 : 2;          // operands are 53 + UP bits below their scale
+  static constexpr int UNIT = KP == 32 ? 55 : 54;      // combinations are in units of 2^-UNIT of the scales
+  static constexpr int JOBS = KP == 32 ? 7 : 8;        // weights kept: what is dropped is below 2^-60 of the scales
+  static constexpr unsigned long long bias() {
+    unsigned long long b = 0;
+    for (int i = 0; i < kIbDig; ++i) b |= 1ull << (BITS * i + BITS - 1);
+    return b;
+  }
+  static constexpr unsigned long long BIAS = bias();
+  // what the bits of 1.5 2^23 add to a combination of digits: the weights that take them
+  static constexpr unsigned long long OFFSET =
+      kIbMagicBits * (KP == 32 ? (1ull << 39) + (1ull << 30) + 1 + 1
+                               : (1ull << 40) + (1ull << 32) + (1ull << 24) + (1ull << 16) + (1ull << 8) + 1 + 1);
+  static_assert(kIbDig * MAXB * (1 << (2 * BITS - 2)) <= (1 << 24), "exact FP32 accumulators");
+  static_assert((KP == 32 ? 2 : 5) * MAXB * (1 << (2 * BITS - 2)) < (1 << 22), "weights that become integers by addition");
+};
+
+template <int NC, int KP>
 struct IbShape {
-  static constexpr int RN = 2 * NC;            // B rows per n1
-  static constexpr int PN = kIbN / RN;         // n1 per pass
-  static constexpr int PASSES = 32 / PN;       // at most
-  static constexpr int BBYTES = PASSES * kIbOperand;
+  static constexpr int KC = KP / 8;               // core columns of 16 bytes
+  static constexpr int SLICE = 128 * KP * 2;      // bytes of one digit of an operand
+  static constexpr int OPERAND = kIbDig * SLICE;  // bytes of an A operand or one pass of B
+  static constexpr int RN = 2 * NC;               // B rows per n1
+  static constexpr int PN = kIbN / RN;            // n1 per pass
+  static constexpr int PASSES = (KP + PN - 1) / PN;  // at most
+  static constexpr int BBYTES = PASSES * OPERAND;
+  static constexpr bool STREAM = KP > 32;         // B in shared memory: one pass, or all
+  static constexpr int BSMEM = STREAM ? OPERAND : BBYTES;
 };
 
 // per-tile data, four tiles deep: written two tiles ahead, read until the tile is stored
+template <int KP>
 struct IbTile {
-  int4 ph[kIbCols][kIbMaxM + 1];  // cos, sin of m phi in words of 2^-61
+  int4 ph[kIbCols][IbNumbers<KP>::MAXM + 1];  // cos, sin of m phi in words of 2^-61
   int2 t[kIbCols];                // t in words of 2^-62
   long long xoff[kIbCols];        // x_j of the column
-  int eb[kIbK], ea[kIbK];         // column and row exponents of the interval
+  int eb[KP], ea[KP];             // column and row exponents of the interval
   int cexp[kIbCols];              // scale of x_j (written with the A operand)
   int ncol, bucket;
   long long pair0;                // first pair, from the start of V
@@ -100,30 +115,30 @@ struct IbTile {
 
 static constexpr int kIbXPitch = 31;  // x_j of a column: element n2 at (n2 mod 8) 4 + n2 / 8
 
+template <int KP>
 struct IbSmem {
-  IbTile tile[4];
+  IbTile<KP> tile[4];
   IbRec rec[2][kIbCols];              // records, exponents and (columns, bucket, first pair) of the next tiles
-  int exps[2][64];
+  int exps[2][2 * KP];
   int next[2][3];
-  double2 x[kIbCols * kIbXPitch];     // x_j of the next tile's columns
+  double2 x[KP == 32 ? kIbCols * kIbXPitch : 1];  // x_j of the next tile's columns (K = 48 leaves no room for it)
   uint64_t dfull[4], dempty[4], afull, meta[4], bfull, done;
-  int mofn[kIbK];
+  int mofn[KP];
   uint32_t tmem;
   int lb[2];  // bucket of the two look-ahead warps
 };
-static constexpr size_t kIbSmemTail = (sizeof(IbSmem) + 127) / 128 * 128;
-template <int NC>
+template <int NC, int KP>
 constexpr size_t ib_smem() {
-  return (size_t)kIbOperand + IbShape<NC>::BBYTES + kIbSmemTail;
+  return (size_t)IbShape<NC, KP>::OPERAND + IbShape<NC, KP>::BSMEM + (sizeof(IbSmem<KP>) + 127) / 128 * 128;
 }
-static_assert(ib_smem<4>() <= kTcSmemBudget, "shared memory");
+static_assert(ib_smem<4, 32>() <= kTcSmemBudget && ib_smem<4, 48>() <= kTcSmemBudget, "shared memory");
 
 struct IbArgs {
   const IbRec *rec;       // ordered pairs sorted by interval
   const int *boff;        // [nb + 1] first pair of every non-empty interval
   const int *toff;        // [nb + 1] first tile
   const unsigned char *B; // [nb] B operands
-  const int *exps;        // [nb][64]: column exponents eb[32], row exponents ea[32]
+  const int *exps;        // [nb][2 KP]: column exponents eb[KP], row exponents ea[KP]
   const double *x;        // [N][bs][R] complex
   const int *mofn;
   double *V;              // [pair - s0][rt][bs] complex
@@ -144,17 +159,20 @@ __device__ __forceinline__ long long ib_fixed(double v, int below) {
   return (int)hi < 0 ? -(long long)m : (long long)m;
 }
 
-// the digits of two 63-bit fixed-point numbers as packed FP16 integers in [-256, 256]
+// the digits of two fixed-point numbers as packed FP16 integers in [-2^(BITS - 1), 2^(BITS - 1)]
+template <int KP>
 __device__ __forceinline__ void ib_digits(long long v0, long long v1, uint32_t (&d)[kIbDig]) {
-  const unsigned long long f0 = (unsigned long long)v0 + kIbBias, f1 = (unsigned long long)v1 + kIbBias;
+  constexpr int BITS = IbNumbers<KP>::BITS;
+  const unsigned long long f0 = (unsigned long long)v0 + IbNumbers<KP>::BIAS, f1 = (unsigned long long)v1 + IbNumbers<KP>::BIAS;
 #pragma unroll
   for (int s = 0; s < kIbDig; ++s) {
-    const int sh = kIbBits * (kIbDig - 1 - s);
-    const uint32_t mask = s > 0 ? 511u : 1023u;  // the top digit may be 512
+    const int sh = BITS * (kIbDig - 1 - s);
+    const uint32_t mask = s > 0 ? (1u << BITS) - 1 : (2u << BITS) - 1;  // the top digit may be 2^BITS
     const uint32_t a = (uint32_t)(f0 >> sh);
     const uint32_t b = sh >= 16 ? (uint32_t)(f1 >> (sh - 16)) : (uint32_t)f1 << (16 - sh);
-    const uint32_t p = (a & mask) | (b & (mask << 16)) | 0x64006400u;  // FP16 1024 + digit + 256
-    const __half2 h = __hadd2(*reinterpret_cast<const __half2 *>(&p), __floats2half2_rn(-1280.f, -1280.f));
+    const uint32_t p = (a & mask) | (b & (mask << 16)) | 0x64006400u;  // FP16 1024 + digit + 2^(BITS - 1)
+    const float off = -1024.f - (1 << (BITS - 1));
+    const __half2 h = __hadd2(*reinterpret_cast<const __half2 *>(&p), __floats2half2_rn(off, off));
     d[s] = *reinterpret_cast<const uint32_t *>(&h);
   }
 }
@@ -211,25 +229,27 @@ __device__ __forceinline__ void ib_mma(uint32_t dst, uint32_t a, uint32_t b, uin
 
 // all digit products of weight D; unrolled, because one thread issues them and every instruction between two
 // MMAs costs it several cycles
-template <int D>
+template <int D, int KP>
 __device__ __forceinline__ void ib_issue(uint32_t dst, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc) {
 #pragma unroll
-  for (int i = 0; i <= D; ++i)
+  for (int i = D < kIbDig ? 0 : D - kIbDig + 1; i <= (D < kIbDig ? D : kIbDig - 1); ++i)
 #pragma unroll
-    for (int ks = 0; ks < kIbK / 16; ++ks) {
-      const uint32_t ao = a + (uint32_t)((i * kIbSlice + ks * 256) >> 4), bo = b + (uint32_t)(((D - i) * kIbSlice + ks * 256) >> 4);
-      if (i == 0 && ks == 0) ib_mma<false>(dst, ao, bo, hi, idesc);
+    for (int ks = 0; ks < KP / 16; ++ks) {
+      constexpr int SLICE = 128 * KP * 2;
+      const uint32_t ao = a + (uint32_t)((i * SLICE + ks * 256) >> 4), bo = b + (uint32_t)(((D - i) * SLICE + ks * 256) >> 4);
+      if (i == (D < kIbDig ? 0 : D - kIbDig + 1) && ks == 0) ib_mma<false>(dst, ao, bo, hi, idesc);
       else ib_mma<true>(dst, ao, bo, hi, idesc);
     }
 }
 
-template <int NC>
+template <int NC, int KP>
 __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
-  using Sh = IbShape<NC>;
+  using Sh = IbShape<NC, KP>;
+  using Num = IbNumbers<KP>;
   constexpr int RN = Sh::RN, PN = Sh::PN, WN = PN / 4;  // WN rows n1 per warp and pass
   extern __shared__ __align__(1024) unsigned char ib_raw[];
-  unsigned char *As = ib_raw, *Bs = ib_raw + kIbOperand;
-  IbSmem &S = *reinterpret_cast<IbSmem *>(Bs + Sh::BBYTES);
+  unsigned char *As = ib_raw, *Bs = ib_raw + Sh::OPERAND;
+  IbSmem<KP> &S = *reinterpret_cast<IbSmem<KP> *>(Bs + Sh::BSMEM);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bs = a.bs;
   const int ntiles = a.t1 - a.t0;
@@ -237,7 +257,7 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
   const int NT = a.t0 + (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x) - T0;  // this CTA's tiles
   const int passes = (bs + PN - 1) / PN;
 
-  if (tid < kIbK) S.mofn[tid] = tid < bs ? a.mofn[tid] : 0;
+  if (tid < KP) S.mofn[tid] = tid < bs ? a.mofn[tid] : 0;
   if (tid == 0) {
     auto init = [](uint64_t *b, int n) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n) : "memory");
@@ -289,8 +309,8 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
       S.next[ti & 1][1] = lb;
       S.next[ti & 1][2] = p0;
     }
-    if (lane < 8)
-      cp_async16(&S.exps[ti & 1][32 * look_half + 4 * lane], a.exps + (size_t)lb * 64 + 32 * look_half + 4 * lane);
+    if (lane < KP / 4)
+      cp_async16(&S.exps[ti & 1][KP * look_half + 4 * lane], a.exps + (size_t)lb * 2 * KP + KP * look_half + 4 * lane);
     const int c = look_half * 32 + lane;
     if (c < (p1 - p0) * a.rt) {
       const IbRec *r = a.rec + p0 + c / a.rt;
@@ -301,20 +321,20 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
   // the words of its t and phases
   auto look_form = [&](int ti) {
     if (look_half < 0 || ti >= NT) return;
-    IbTile &t = S.tile[ti & 3];
+    IbTile<KP> &t = S.tile[ti & 3];
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
     const int c = look_half * 32 + lane;
     const IbRec rc = S.rec[ti & 1][c];  // unused columns hold an old record
     if (look_half == 0) {
-      t.eb[lane] = S.exps[ti & 1][lane];
+      for (int e = lane; e < KP; e += 32) t.eb[e] = S.exps[ti & 1][e];
       if (lane == 0) {
         t.ncol = S.next[ti & 1][0];
         t.bucket = S.next[ti & 1][1];
         t.pair0 = S.next[ti & 1][2] - a.s0;
       }
     } else {
-      t.ea[lane] = S.exps[ti & 1][32 + lane];
+      for (int e = lane; e < KP; e += 32) t.ea[e] = S.exps[ti & 1][KP + e];
     }
     auto words = [](double v, int up) {  // v in units of 2^-up, |v| <= 1
       return ib_split_signed(min(ib_fixed<10>(v, 1023 + 62 - up - ib_field(v)), kIbBelowOne));
@@ -339,7 +359,7 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
   // the tensor core takes its MMAs (73 cycles each) is spread over the warps. Its accumulator is free once every warp
   // has read job g - 4.
   const uint32_t idesc = (1u << 4) | ((uint32_t)(kIbN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);  // F16 in, F32 out
-  const uint64_t da = tc_desc<kIbKC>(smem_u32(As)), db = tc_desc<kIbKC>(smem_u32(Bs));
+  const uint64_t da = tc_desc<Sh::KC>(smem_u32(As)), db = tc_desc<Sh::KC>(smem_u32(Bs));
   const uint32_t dal = (uint32_t)da, dbl = (uint32_t)db, dhi = (uint32_t)(da >> 32);
   auto issue = [&](uint32_t g, int pass, auto weight) {
     int ok = 1;
@@ -347,7 +367,8 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
       if (g >= 4) ok = tc_wait1(smem_u32(&S.dempty[g & 3]), ((g >> 2) - 1) & 1);
       if (ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        ib_issue<decltype(weight)::value>(tmem + (g & 3) * kIbN, dal, dbl + (uint32_t)(pass * (kIbOperand >> 4)), dhi, idesc);
+        ib_issue<decltype(weight)::value, KP>(tmem + (g & 3) * kIbN, dal, dbl + (Sh::STREAM ? 0u : (uint32_t)(pass * (Sh::OPERAND >> 4))),
+                                              dhi, idesc);
         tc_commit(smem_u32(&S.dfull[g & 3]));
       }
     }
@@ -355,7 +376,7 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
   };
     // x_j of this warp's four columns of tile ti on their way to shared memory
     auto fetch = [&](int ti) {
-      const IbTile &t = S.tile[ti & 3];
+      const IbTile<KP> &t = S.tile[ti & 3];
       const int chunk = lane >> 3, q = lane & 7, n2 = chunk * 8 + q;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -364,56 +385,71 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
           cp_async16(&S.x[col * kIbXPitch + q * 4 + chunk], a.x + t.xoff[col] + 2 * (size_t)n2 * a.R);
       }
     };
-    // rotate the columns of tile ti and cut them into digits
+    // rotate the columns of tile ti and cut them into digits; a lane owns a row (column and part) and every fourth
+    // core column of eight n2
     auto form = [&](int ti) {
-      IbTile &t = S.tile[ti & 3];
+      IbTile<KP> &t = S.tile[ti & 3];
       const int rl = lane & 7, chunk = lane >> 3, row = warp * 8 + rl, col = row >> 1, part = row & 1;
       const bool have = col < t.ncol;
       if (warp * 4 < t.ncol) {
-        const double *xp = reinterpret_cast<const double *>(S.x + col * kIbXPitch + chunk) + part;
-        double xv[8];
+        constexpr int CH = (Sh::KC + 3) / 4;
+        double xv[CH][8];
         int emax = 0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) xv[q] = have && chunk * 8 + q < bs ? xp[8 * q] : 0.0;
+        for (int k = 0; k < CH; ++k) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int f = ib_field(xv[q]);
-          if (f != 0) emax = max(emax, f == 0x7FF ? 1 << 20 : f + t.eb[chunk * 8 + q] + 4096);  // Inf, NaN: see below
+          for (int q = 0; q < 8; ++q) {
+            const int n2 = (chunk + 4 * k) * 8 + q;
+            if (Sh::STREAM) xv[k][q] = have && n2 < bs ? __ldg(a.x + t.xoff[col] + part + 2 * (size_t)n2 * a.R) : 0.0;
+            else xv[k][q] = have && n2 < bs ? reinterpret_cast<const double *>(S.x + col * kIbXPitch + chunk)[8 * q + part] : 0.0;
+          }
         }
+#pragma unroll
+        for (int k = 0; k < CH; ++k)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int f = ib_field(xv[k][q]);  // zero beyond the block; Inf, NaN: see below
+            if (f != 0) emax = max(emax, f == 0x7FF ? 1 << 20 : f + t.eb[(chunk + 4 * k) * 8 + q] + 4096);
+          }
         emax = max(emax, __shfl_xor_sync(kTcFull, emax, 1));
         emax = max(emax, __shfl_xor_sync(kTcFull, emax, 8));
         emax = max(emax, __shfl_xor_sync(kTcFull, emax, 16));
         if (part == 0 && chunk == 0) t.cexp[col] = emax;
         const int es = emax - 4096;  // |Re x|, |Im x| < 2^(es - 1022) under the column exponents
         const int4 *pc = t.ph[have ? col : 0];
-        unsigned char *dst = As + (size_t)(row >> 3) * (kIbKC * 128) + (row & 7) * 16 +
-                             chunk * 128;
-        uint32_t o[kIbDig][4];
 #pragma unroll
-        for (int q = 0; q < 8; q += 2) {
-          long long u[2];
+        for (int k = 0; k < CH; ++k) {
+          const int core = min(chunk + 4 * k, Sh::KC - 1);
+          unsigned char *dst = As + (size_t)(row >> 3) * (Sh::KC * 128) + (row & 7) * 16 + core * 128;
+          uint32_t o[kIbDig][4];
 #pragma unroll
-          for (int w = 0; w < 2; ++w) {
-            const int n2 = chunk * 8 + q + w, m = S.mofn[n2];
-            const IbWords f = ib_split(ib_fixed<9>(xv[q + w], es - t.eb[n2] - ib_field(xv[q + w])));
-            const int oh = __shfl_xor_sync(kTcFull, f.h, 1), ol = __shfl_xor_sync(kTcFull, f.l, 1);
-            // half of Re = c xr - s xi or Im = c xi + s xr
-            int4 p = pc[m < 0 ? -m : m];
-            if ((m < 0) == (part != 0)) {
-              p.z = -p.z;
-              p.w = -p.w;
+          for (int q = 0; q < 8; q += 2) {
+            long long u[2];
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+              const int n2 = core * 8 + q + w, m = S.mofn[n2];
+              const double x = xv[k][q + w];
+              const IbWords f = ib_split(ib_fixed<Num::UP>(x, es - t.eb[n2] - ib_field(x)));
+              const int oh = __shfl_xor_sync(kTcFull, f.h, 1), ol = __shfl_xor_sync(kTcFull, f.l, 1);
+              // half of Re = c xr - s xi or Im = c xi + s xr
+              int4 p = pc[m < 0 ? -m : m];
+              if ((m < 0) == (part != 0)) {
+                p.z = -p.z;
+                p.w = -p.w;
+              }
+              const long long mid = ib_mad(f.h, p.y, ib_mad(f.l, p.x, ib_mad(oh, p.w, ib_mad(ol, p.z, 0x40000000ll))));
+              u[w] = ib_mad(f.h, p.x, ib_mad(oh, p.z, mid >> 31));
             }
-            const long long mid = ib_mad(f.h, p.y, ib_mad(f.l, p.x, ib_mad(oh, p.w, ib_mad(ol, p.z, 0x40000000ll))));
-            u[w] = ib_mad(f.h, p.x, ib_mad(oh, p.z, mid >> 31));
+            uint32_t dg[kIbDig];
+            ib_digits<KP>(u[0], u[1], dg);
+#pragma unroll
+            for (int s = 0; s < kIbDig; ++s) o[s][q >> 1] = dg[s];
           }
-          uint32_t dg[kIbDig];
-          ib_digits(u[0], u[1], dg);
+          if (chunk + 4 * k < Sh::KC)
 #pragma unroll
-          for (int s = 0; s < kIbDig; ++s) o[s][q >> 1] = dg[s];
+            for (int s = 0; s < kIbDig; ++s)
+              *reinterpret_cast<uint4 *>(dst + (size_t)s * Sh::SLICE) = make_uint4(o[s][0], o[s][1], o[s][2], o[s][3]);
         }
-#pragma unroll
-        for (int s = 0; s < kIbDig; ++s)
-          *reinterpret_cast<uint4 *>(dst + (size_t)s * kIbSlice) = make_uint4(o[s][0], o[s][1], o[s][2], o[s][3]);
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -426,7 +462,7 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
     // waits for the next job (weight D of pass p); read() gets 16 of this warp's 32 columns at a time; then the
     // buffer is free for the job after next three, whose issuing warp sends it off
     auto job = [&](auto weight, int p, bool work, auto &&read) {
-      constexpr int D = decltype(weight)::value, DN = D <= 2 ? D + 4 : D - 3;
+      constexpr int D = decltype(weight)::value, DN = D + 4 < Num::JOBS ? D + 4 : D + 4 - Num::JOBS;
       if (!tc_waitw(smem_u32(&S.dfull[g & 3]), (g >> 2) & 1)) return false;
       if (work) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -443,34 +479,52 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
       __syncwarp();
       if (lane == 0) tc_arrive(smem_u32(&S.dempty[g & 3]));
       ++g;
-      const int pn = D <= 2 ? p : p + 1;
+      const int pn = D + 4 < Num::JOBS ? p : p + 1;
+      if (Sh::STREAM && D + 4 >= Num::JOBS) return true;  // the next pass starts when its operand is there
       return ((g + 3) & (kIbWarps - 1)) != warp || pn >= passes || issue(g + 3, pn, std::integral_constant<int, DN>());
     };
     int cur_b = -1, bloads = 0;
     auto wait_meta = [&](int ti) { return tc_waitw(smem_u32(&S.meta[ti & 3]), (uint32_t)((ti >> 2) & 1)); };
+    // the B operand of a bucket (STREAM: one pass of it), once every MMA that read the last one has completed
+    auto load_b = [&](int bucket, int pass) {
+      ++bloads;
+      if (warp == 0 && lane == 0) {
+        const uint32_t bar = smem_u32(&S.bfull), bytes = (uint32_t)((Sh::STREAM ? 1 : passes) * Sh::OPERAND);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(Bs)),
+            "l"(a.B + (size_t)bucket * Sh::BBYTES + (size_t)pass * Sh::OPERAND), "r"(bytes), "r"(bar)
+            : "memory");
+      }
+    };
+    // the first four jobs of a pass of tile ti
+    auto start = [&](int ti, int pass) {
+      const int mine = (int)((uint32_t)warp - g) & (kIbWarps - 1);
+      if (mine >= 4) return true;
+      if (pass == 0 && !tc_waitw(smem_u32(&S.afull), (uint32_t)(ti & 1))) return false;
+      if (!tc_waitw(smem_u32(&S.bfull), (uint32_t)((bloads - 1) & 1))) return false;
+      if (mine == 0) return issue(g, pass, std::integral_constant<int, 0>());
+      if (mine == 1) return issue(g + 1, pass, std::integral_constant<int, 1>());
+      if (mine == 2) return issue(g + 2, pass, std::integral_constant<int, 2>());
+      return issue(g + 3, pass, std::integral_constant<int, 3>());
+    };
     look_fetch(0);
     look_form(0);
     look_fetch(1);
     look_form(1);
     look_fetch(2);
     good = NT == 0 || wait_meta(0);
-    if (good && NT > 0) fetch(0);
+    if (good && NT > 0) {
+      if (!Sh::STREAM) fetch(0);
+      if (Sh::STREAM) load_b(S.tile[0].bucket, 0);
+    }
     for (int ti = 0; ti < NT && good; ++ti) {
-      IbTile &t = S.tile[ti & 3];
+      IbTile<KP> &t = S.tile[ti & 3];
       look_form(ti + 2);
       // every job of the last tile has been read: its operands are free
-      if (t.bucket != cur_b) {
+      if (!Sh::STREAM && t.bucket != cur_b) {
         cur_b = t.bucket;
-        ++bloads;
-        if (warp == 0 && lane == 0) {
-          const uint32_t bar = smem_u32(&S.bfull), bytes = (uint32_t)(passes * kIbOperand);
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-          asm volatile(
-              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                  smem_u32(Bs)),
-              "l"(a.B + (size_t)cur_b * Sh::BBYTES), "r"(bytes), "r"(bar)
-              : "memory");
-        }
+        load_b(cur_b, 0);
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncwarp();
@@ -479,26 +533,24 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
       if (ti + 1 < NT) {
         good = wait_meta(ti + 1);
         if (!good) break;
-        fetch(ti + 1);
+        if (!Sh::STREAM) fetch(ti + 1);
       }
-      const int mine = (int)((uint32_t)warp - g) & (kIbWarps - 1);  // the tile's first four jobs
-      if (mine < 4) {
-        good = tc_waitw(smem_u32(&S.afull), (uint32_t)(ti & 1)) &&
-               tc_waitw(smem_u32(&S.bfull), (uint32_t)((bloads - 1) & 1));
-        if (good) {
-          if (mine == 0) good = issue(g, 0, std::integral_constant<int, 0>());
-          else if (mine == 1) good = issue(g + 1, 0, std::integral_constant<int, 1>());
-          else if (mine == 2) good = issue(g + 2, 0, std::integral_constant<int, 2>());
-          else good = issue(g + 3, 0, std::integral_constant<int, 3>());
-        }
-      }
+      good = start(ti, 0);
       for (int p = 0; p < passes && good; ++p) {
+        if (Sh::STREAM && p > 0) {
+          good = start(ti, p);
+          if (!good) break;
+        }
         const int n0 = p * PN + grp * WN;
         const bool work = sp * 16 < t.ncol && n0 < bs;
-        // The digits in units of 2^-55 of the scales; the Im rows of C are negated in the Im u lanes. What is
+        // The digits in units of 2^-UNIT of the scales; the Im rows of C are negated in the Im u lanes. What is
         // below 2^22 becomes an integer by an FP32 addition of 1.5 2^23, whose exponent bits stay in the sum
-        // and are taken off it (kIbOffset) below.
+        // and are taken off it (OFFSET) below.
         auto unit = [&](int c, int u) { return c & 1 ? sg * u : u; };
+        auto bits = [](float f) { return __float_as_int(f + kIbMagic); };
+        auto high = [&](int c, float f, int u) {
+          return (long long)((unsigned long long)((unsigned)bits(f) * (unsigned)unit(c, u)) << 32);
+        };
         long long w[32];
         std::integral_constant<int, 0> w0;
         std::integral_constant<int, 1> w1;
@@ -507,28 +559,39 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
         std::integral_constant<int, 4> w4;
         std::integral_constant<int, 5> w5;
         std::integral_constant<int, 6> w6;
-        good = job(w0, p, work, [&](int c, float f) {
-          w[c] = (long long)((unsigned long long)(__float_as_uint(f + kIbMagic) * (unsigned)unit(c, 1 << 7)) << 32);
-        });
-        good = good && job(w1, p, work, [&](int c, float f) {
-          w[c] = ib_mad(__float_as_int(f + kIbMagic), unit(c, 1 << 30), w[c]);
-        });
-        good = good && job(w2, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 21), w[c]); });
-        good = good && job(w3, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 12), w[c]); });
-        good = good && job(w4, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 8), w[c]); });
-        good = good && job(w5, p, work, [&](int c, float f) {
-          w[c] = ib_mad(__float_as_int(fmaf(f, 0x1p-6f, kIbMagic)), unit(c, 1), w[c]);
-        });
-        good = good && job(w6, p, work, [&](int c, float f) {
-          w[c] = ib_mad(__float_as_int(fmaf(f, 0x1p-15f, kIbMagic)), unit(c, 1), w[c]);
-        });
+        if constexpr (KP == 32) {
+          good = job(w0, p, work, [&](int c, float f) { w[c] = high(c, f, 1 << 7); });
+          good = good && job(w1, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f), unit(c, 1 << 30), w[c]); });
+          good = good && job(w2, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 21), w[c]); });
+          good = good && job(w3, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 12), w[c]); });
+          good = good && job(w4, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 8), w[c]); });
+          good = good && job(w5, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f * 0x1p-6f), unit(c, 1), w[c]); });
+          good = good && job(w6, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f * 0x1p-15f), unit(c, 1), w[c]); });
+        } else {
+          good = job(w0, p, work, [&](int c, float f) { w[c] = high(c, f, 1 << 8); });
+          good = good && job(w1, p, work, [&](int c, float f) {
+            w[c] = (long long)((unsigned long long)w[c] + (unsigned long long)high(c, f, 1));
+          });
+          good = good && job(w2, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f), unit(c, 1 << 24), w[c]); });
+          good = good && job(w3, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f), unit(c, 1 << 16), w[c]); });
+          good = good && job(w4, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f), unit(c, 1 << 8), w[c]); });
+          good = good && job(w5, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1), w[c]); });
+          good = good && job(w6, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f * 0x1p-8f), unit(c, 1), w[c]); });
+          good = good && job(std::integral_constant<int, 7>(), p, work, [&](int c, float f) {
+            w[c] = ib_mad(bits(f * 0x1p-16f), unit(c, 1), w[c]);
+          });
+        }
+        if (Sh::STREAM && good) {  // every MMA of this pass has completed
+          if (p + 1 < passes) load_b(t.bucket, p + 1);
+          else if (ti + 1 < NT) load_b(S.tile[(ti + 1) & 3].bucket, 0);
+        }
         if (!good || !work) continue;
         const bool have = col < t.ncol;
         const int2 tw = have ? t.t[col] : make_int2(0, 0);
         const int ce = have ? t.cexp[col] : 0;
-        const int cs = ce - 4096 - 1022 + 1 - 55;  // scale of x, half of its rotation, units
+        const int cs = ce - 4096 - 1022 + 1 - Num::UNIT;  // scale of x, half of its rotation, units
         // the Re lane receives the negated Im sum (offsets cancel), the Im lane adds two positive ones
-        const unsigned long long offset = part ? 0ull - 2ull * kIbOffset : 0ull;
+        const unsigned long long offset = part ? 0ull - 2ull * Num::OFFSET : 0ull;
         const int4 *pc = t.ph[have ? col : 0];
         double *vo = a.V + 2 * ((t.pair0 * a.rt + (have ? col : 0)) * bs) + part;
 #pragma unroll
@@ -544,7 +607,7 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
           }
           const IbWords v = ib_split(acc);
           const int oh = __shfl_xor_sync(kTcFull, v.h, 1), ol = __shfl_xor_sync(kTcFull, v.l, 1);
-          const int m = S.mofn[n & 31];
+          const int nc = min(n, KP - 1), m = S.mofn[nc];
           int4 ph = pc[m < 0 ? -m : m];
           if ((m < 0) != (part != 0)) {
             ph.z = -ph.z;
@@ -553,7 +616,7 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
           // e^{-i m phi} times the value: c v +- s (other part)
           const long long mid = ib_mad(v.h, ph.y, ib_mad(v.l, ph.x, ib_mad(oh, ph.w, ib_mad(ol, ph.z, 0x20000000ll))));
           const long long out = 2 * ib_mad(v.h, ph.x, (long long)oh * ph.z) + (mid >> 30);
-          double res = ib_to_double(out, cs + t.ea[n & 31]);
+          double res = ib_to_double(out, cs + t.ea[nc]);
           if (ce >= (1 << 20)) res = __longlong_as_double(0x7FF8000000000000ll);  // Inf or NaN in x
           if (have && n < bs) vo[2 * n] = res;
         }
@@ -586,7 +649,7 @@ struct IbSum {
 
 // One block per receiver: `groups` thread groups take contiguous emitter ranges, each thread owns one
 // (right-hand side, n1) and adds the emitters in index order; the groups' sums are added in order.
-__global__ void __launch_bounds__(512) ib_sum_kernel(const CouplingLaunch L, const IbSum s) {
+__global__ void __launch_bounds__(768) ib_sum_kernel(const CouplingLaunch L, const IbSum s) {
   extern __shared__ __align__(16) unsigned char ib_sum_smem[];
   double2 *part = reinterpret_cast<double2 *>(ib_sum_smem);  // [groups][bs * rt]
   const int i = blockIdx.x, N = L.n, bs = L.bs, E = bs * s.rt;
@@ -681,14 +744,14 @@ __global__ void ib_records_kernel(const double2 *pos, int n, double rho_min, dou
 }
 
 // B operand and exponents of one non-empty interval per block
-template <int NC>
+template <int NC, int KP>
 __global__ void __launch_bounds__(256) ib_operand_kernel(const double2 *coef, const int *bk, int bs, unsigned char *B,
                                                          int *exps) {
-  using Sh = IbShape<NC>;
-  __shared__ int eb[kIbK], ea[kIbK];
+  using Sh = IbShape<NC, KP>;
+  __shared__ int eb[KP], ea[KP];
   const int tid = threadIdx.x, b = blockIdx.x, bs2 = bs * bs;
   const double2 *C = coef + (size_t)bk[b] * NC * bs2;
-  if (tid < kIbK) {
+  if (tid < KP) {
     eb[tid] = ea[tid] = -(1 << 20);
   }
   __syncthreads();
@@ -697,23 +760,23 @@ __global__ void __launch_bounds__(256) ib_operand_kernel(const double2 *coef, co
     if (f) atomicMax(&eb[(e % bs2) / bs], f - 1022);
   }
   __syncthreads();
-  if (tid < kIbK && eb[tid] == -(1 << 20)) eb[tid] = 0;
+  if (tid < KP && eb[tid] == -(1 << 20)) eb[tid] = 0;
   __syncthreads();
   for (int e = tid; e < NC * bs2; e += blockDim.x) {
     const int f = max(ib_field(C[e].x), ib_field(C[e].y));
     if (f) atomicMax(&ea[e % bs], f - 1022 - eb[(e % bs2) / bs]);
   }
   __syncthreads();
-  if (tid < kIbK && ea[tid] == -(1 << 20)) ea[tid] = 0;
+  if (tid < KP && ea[tid] == -(1 << 20)) ea[tid] = 0;
   __syncthreads();
-  if (tid < kIbK) {
-    exps[(size_t)b * 64 + tid] = eb[tid];
-    exps[(size_t)b * 64 + 32 + tid] = ea[tid];
+  if (tid < KP) {
+    exps[(size_t)b * 2 * KP + tid] = eb[tid];
+    exps[(size_t)b * 2 * KP + KP + tid] = ea[tid];
   }
   unsigned char *out = B + (size_t)b * Sh::BBYTES;
   // one thread per row (n1, power, part) and pair of n2
-  for (int e = tid; e < Sh::PASSES * kIbN * kIbK / 2; e += blockDim.x) {
-    const int row = e / (kIbK / 2), k = 2 * (e - row * (kIbK / 2));
+  for (int e = tid; e < Sh::PASSES * kIbN * KP / 2; e += blockDim.x) {
+    const int row = e / (KP / 2), k = 2 * (e - row * (KP / 2));
     const int n1 = row / Sh::RN, c = (row % Sh::RN) >> 1, im = row & 1;
     long long f[2];
     for (int w = 0; w < 2; ++w) {
@@ -723,14 +786,14 @@ __global__ void __launch_bounds__(256) ib_operand_kernel(const double2 *coef, co
         const double2 cv = C[(size_t)c * bs2 + n2 * bs + n1];
         v = im ? cv.y : cv.x;
       }
-      f[w] = ib_fixed<9>(v, n1 < bs && n2 < bs ? ea[n1] + eb[n2] + 1022 - ib_field(v) : 0);
+      f[w] = ib_fixed<IbNumbers<KP>::UP>(v, n1 < bs && n2 < bs ? ea[n1] + eb[n2] + 1022 - ib_field(v) : 0);
     }
     uint32_t dg[kIbDig];
-    ib_digits(f[0], f[1], dg);
+    ib_digits<KP>(f[0], f[1], dg);
     const int pass = row / kIbN, r = row % kIbN;
     for (int s = 0; s < kIbDig; ++s)
-      *reinterpret_cast<uint32_t *>(out + (size_t)pass * kIbOperand + (size_t)s * kIbSlice +
-                                    ((size_t)(r >> 3) * kIbKC + (k >> 3)) * 128 + (r & 7) * 16 + (k & 7) * 2) = dg[s];
+      *reinterpret_cast<uint32_t *>(out + (size_t)pass * Sh::OPERAND + (size_t)s * Sh::SLICE +
+                                    ((size_t)(r >> 3) * Sh::KC + (k >> 3)) * 128 + (r & 7) * 16 + (k & 7) * 2) = dg[s];
   }
 }
 
@@ -738,12 +801,32 @@ static constexpr int kIbMinParticles = 32;
 static constexpr long long kIbMaxPairs = 1ll << 27;      // 4 GB of pair records
 static constexpr size_t kIbWorkspace = (size_t)2 << 30;  // bytes of V per chunk
 
+// padded blocksize
+static int ib_kp(const sg_context *c) { return c->bs <= IbNumbers<32>::MAXB ? 32 : 48; }
+
 bool ib_supported(const sg_context *c) {
-  if (c->vol || c->kind < 0 || c->bs > kIbMaxB) return false;
+  if (c->vol || c->kind < 0 || c->bs > IbNumbers<48>::MAXB) return false;
   if ((long long)c->n * c->n > kIbMaxPairs || c->n < kIbMinParticles) return false;
+  const int mmax = ib_kp(c) == 32 ? IbNumbers<32>::MAXM : IbNumbers<48>::MAXM;
   for (int m : c->h_mofn)
-    if (m > kIbMaxM || m < -kIbMaxM) return false;
+    if (m > mmax || m < -mmax) return false;
   return true;
+}
+
+// f(NC, KP) as compile-time constants
+template <class F>
+static void ib_dispatch(const sg_context *c, F &&f) {
+  std::integral_constant<int, 2> two;
+  std::integral_constant<int, 4> four;
+  std::integral_constant<int, 32> small;
+  std::integral_constant<int, 48> large;
+  if (ib_kp(c) == 32) {
+    if (c->ncoef == 2) f(two, small);
+    else f(four, small);
+  } else {
+    if (c->ncoef == 2) f(two, large);
+    else f(four, large);
+  }
 }
 
 static void ib_build_plan(sg_context *c, cudaStream_t st) {
@@ -786,12 +869,14 @@ static void ib_build_plan(sg_context *c, cudaStream_t st) {
   DevBuf<int> dbk;
   dbk.reserve(P.nb);
   P.boff.reserve(P.nb + 1);
-  P.exps.reserve((size_t)P.nb * 64);
-  P.B.reserve((size_t)P.nb * (c->ncoef == 2 ? IbShape<2>::BBYTES : IbShape<4>::BBYTES));
+  P.exps.reserve((size_t)P.nb * 2 * ib_kp(c));
+  ib_dispatch(c, [&](auto nc, auto kp) { P.B.reserve((size_t)P.nb * IbShape<decltype(nc)::value, decltype(kp)::value>::BBYTES); });
   SG_CUDA(cudaMemcpyAsync(dbk.ptr, bk.data(), P.nb * sizeof(int), cudaMemcpyHostToDevice, st));
   SG_CUDA(cudaMemcpyAsync(P.boff.ptr, P.h_boff.data(), (P.nb + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-  if (c->ncoef == 2) ib_operand_kernel<2><<<P.nb, 256, 0, st>>>(c->coef64.ptr, dbk.ptr, c->bs, P.B.ptr, P.exps.ptr);
-  else ib_operand_kernel<4><<<P.nb, 256, 0, st>>>(c->coef64.ptr, dbk.ptr, c->bs, P.B.ptr, P.exps.ptr);
+  ib_dispatch(c, [&](auto nc, auto kp) {
+    ib_operand_kernel<decltype(nc)::value, decltype(kp)::value>
+        <<<P.nb, 256, 0, st>>>(c->coef64.ptr, dbk.ptr, c->bs, P.B.ptr, P.exps.ptr);
+  });
   SG_CUDA(cudaGetLastError());
   P.err.reserve(1);
   SG_CUDA(cudaMemsetAsync(P.err.ptr, 0, sizeof(int), st));
@@ -818,12 +903,13 @@ static sg_context::IbTiles &ib_tiles(sg_context *c, int per, cudaStream_t st) {
   return *P.tiles.back();
 }
 
-template <int NC>
+template <int NC, int KP>
 static void ib_launch(const IbArgs &a, cudaStream_t st) {
   static bool attr_done[64] = {};
+  constexpr int smem = (int)ib_smem<NC, KP>();
   if (first_on_device(attr_done))
-    SG_CUDA(cudaFuncSetAttribute(ib_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ib_smem<NC>()));
-  ib_kernel<NC><<<std::min(sm_count(), a.t1 - a.t0), kIbThreads, ib_smem<NC>(), st>>>(a);
+    SG_CUDA(cudaFuncSetAttribute(ib_kernel<NC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  ib_kernel<NC, KP><<<std::min(sm_count(), a.t1 - a.t0), kIbThreads, smem, st>>>(a);
   SG_CUDA(cudaGetLastError());
 }
 
@@ -894,9 +980,8 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
       s.s1 = first_pair(a.t1);
       s.first = t0 == 0;
       s.last = a.t1 == ntiles;
-      if (c->ncoef == 2) ib_launch<2>(a, st);
-      else ib_launch<4>(a, st);
-      ib_sum_kernel<<<c->n, 512, smem, st>>>(L, s);
+      ib_dispatch(c, [&](auto nc, auto kp) { ib_launch<decltype(nc)::value, decltype(kp)::value>(a, st); });
+      ib_sum_kernel<<<c->n, std::max(512, s.width), smem, st>>>(L, s);
       SG_CUDA(cudaGetLastError());
       launched += 2;
     }

@@ -17,7 +17,7 @@ RES = 40.0
 def _system(ctx, n, bs, kind, seed, l_values=None):
     rng = np.random.default_rng(seed)
     xy = rng.uniform(0, 900.0, (n, 2))
-    m = rng.integers(-3, 4, bs)
+    m = rng.integers(-3, 4, bs) if bs <= 30 else rng.integers(-4, 5, bs)
     rho = np.arange(-3 * RES, 900.0 * 1.5 + 4 * RES, RES)
     table = rng.standard_normal((len(rho), bs, bs)) + 1j * rng.standard_normal((len(rho), bs, bs))
     table *= 10.0 ** -rng.uniform(0, 3, bs)[None, None, :]   # columns of different size
@@ -44,7 +44,9 @@ def _direct(xy, m, rho, table, kind, x):
 
 @pytest.mark.parametrize("n,bs,R,kind", [(32, 1, 1, "linear"), (33, 30, 1, "cubic"), (40, 6, 3, "cubic_hermite"),
                                          (47, 30, 16, "cubic"), (64, 17, 17, "linear"), (65, 30, 64, "cubic"),
-                                         (101, 30, 2, "linear"), (35, 9, 13, "cubic")])
+                                         (101, 30, 2, "linear"), (35, 9, 13, "cubic"), (34, 31, 1, "cubic"),
+                                         (50, 48, 3, "cubic"), (65, 48, 1, "linear"), (33, 36, 16, "cubic_hermite"),
+                                         (40, 47, 21, "linear")])
 def test_matches_direct_evaluation(n, bs, R, kind, gpu_context):
     xy, m, rho, table = _system(gpu_context, n, bs, kind, 100 * n + bs)
     rng = np.random.default_rng(n)
