@@ -134,8 +134,10 @@ __device__ __forceinline__ typename VC<Real>::T table_value(const typename VC<Re
         const cplx frrzz = vld(rows[a] + b * zs + 3 * qs);
         vr += wzm[b] * fzz.x;
         vi += wzm[b] * fzz.y;
-        mr += wz[b] * frr.x + wzm[b] * frrzz.x;
-        mi += wz[b] * frr.y + wzm[b] * frrzz.y;
+        mr += wz[b] * frr.x;
+        mi += wz[b] * frr.y;
+        mr += wzm[b] * frrzz.x;
+        mi += wzm[b] * frrzz.y;
       }
     }
     sr += wr[a] * vr;
@@ -341,7 +343,7 @@ __global__ void __launch_bounds__(kVolThreads) volume_kernel(const VolumeLaunch 
     const double2 pj = L.pos[j];
     const double dx = pi.x - pj.x, dy = pi.y - pj.y;
     const double rho = sqrt(dx * dx + dy * dy);
-    const double phi = atan2(dy, dx);
+    const double cphi = rho > 0.0 ? dx / rho : 1.0, sphi = rho > 0.0 ? dy / rho : 0.0;
     const double zj = V.z[j];
     double wv[4], wm[2];
     Real wr[NT], wrm[2], wp[NT], wpm[2], wn[NT], wnm[2];
@@ -364,7 +366,17 @@ __global__ void __launch_bounds__(kVolThreads) volume_kernel(const VolumeLaunch 
     // e^{i m phi} of the lane's rows; x_j staged with e^{i m2 phi}
     double ec[NB1], es[NB1];
 #pragma unroll
-    for (int s = 0; s < NB1; ++s) sincos((double)m1[s] * phi, &es[s], &ec[s]);
+    for (int s = 0; s < NB1; ++s) {  // by repeated multiplication: atan2 and sincos took a fifth of a pair's time
+      const int am = m1[s] < 0 ? -m1[s] : m1[s];
+      double pr = 1.0, pim = 0.0;
+      for (int q = 0; q < am; ++q) {
+        const double na = pr * cphi - pim * sphi;
+        pim = pr * sphi + pim * cphi;
+        pr = na;
+      }
+      ec[s] = pr;
+      es[s] = m1[s] < 0 ? -pim : pim;
+    }
 #pragma unroll
     for (int s = 0; s < NB1; ++s) {
       const int n2 = lane + 32 * s;
@@ -393,6 +405,17 @@ __global__ void __launch_bounds__(kVolThreads) volume_kernel(const VolumeLaunch 
       rp[a] = Tp + (size_t)(ir + a) * rs + (size_t)ip * zs;
       rm[a] = Tm + (size_t)(ir + a) * rs + (size_t)im * zs;
     }
+    // bilinear: the products of the axis weights, formed once per pair, leave one multiply-add per tap and part
+    Real w2[2][2][2];
+    if constexpr (KIND == SG_LINEAR) {
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          w2[0][a][b] = wr[a] * wp[b];
+          w2[1][a][b] = wr[a] * wn[b];
+        }
+    }
     cplx acc[NB1][RT];
 #pragma unroll
     for (int s = 0; s < NB1; ++s)
@@ -412,14 +435,28 @@ __global__ void __launch_bounds__(kVolThreads) volume_kernel(const VolumeLaunch 
             pa[a] = rp[a] + n2 * bs + n1;
             ma[a] = rm[a] + n2 * bs + n1;
           }
-          const cplx wpl = table_value<Real, KIND, NT>(pa, zs, qs, wr, wrm, wp, wpm);
-          const cplx wmn = table_value<Real, KIND, NT>(ma, zs, qs, wr, wrm, wn, wnm);
-          const Real wre = wpl.x + wmn.x, wim = wpl.y + wmn.y;
+          Real wre, wim;
+          if constexpr (KIND == SG_LINEAR) {
+            wre = wim = 0;
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+              for (int b = 0; b < 2; ++b) {
+                const cplx p = vld(pa[a] + b * zs), q = vld(ma[a] + b * zs);
+                wre = fma(w2[0][a][b], p.x, fma(w2[1][a][b], q.x, wre));
+                wim = fma(w2[0][a][b], p.y, fma(w2[1][a][b], q.y, wim));
+              }
+          } else {
+            const cplx wpl = table_value<Real, KIND, NT>(pa, zs, qs, wr, wrm, wp, wpm);
+            const cplx wmn = table_value<Real, KIND, NT>(ma, zs, qs, wr, wrm, wn, wnm);
+            wre = wpl.x + wmn.x;
+            wim = wpl.y + wmn.y;
+          }
 #pragma unroll
           for (int r = 0; r < RT; ++r) {
             const cplx xv = xs[n2 * RT + r];
-            acc[s][r].x += wre * xv.x - wim * xv.y;
-            acc[s][r].y += wre * xv.y + wim * xv.x;
+            acc[s][r].x = fma(wre, xv.x, fma(-wim, xv.y, acc[s][r].x));
+            acc[s][r].y = fma(wre, xv.y, fma(wim, xv.x, acc[s][r].y));
           }
         }
       }
