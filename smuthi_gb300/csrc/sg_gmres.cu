@@ -29,45 +29,55 @@ struct VecList {
   const double2 *v[kMaxVec];
 };
 
-// partial[blk][k][r] = sum_{rows in blk} conj(V_k[row][r]) * w[row][r]
-__global__ void dots_partial_kernel(VecList V, int nvec, const double2 *w, size_t rows, int R, double2 *partial) {
-  extern __shared__ double2 sd[];
-  const int tpr = blockDim.x / R;  // threads per rhs column (blockDim.x is a multiple of R)
-  const int r = threadIdx.x % R, lr = threadIdx.x / R;
-  const size_t nblk = gridDim.x;
-  for (int k = 0; k < nvec; ++k) {
-    double sr = 0.0, si = 0.0;
-    for (size_t row = blockIdx.x * (size_t)tpr + lr; row < rows; row += nblk * tpr) {
-      const double2 a = V.v[k][row * R + r], b = w[row * R + r];
-      sr = fma(a.x, b.x, fma(a.y, b.y, sr));
-      si = fma(a.x, b.y, fma(-a.y, b.x, si));
+// sums of the threads of equal r = threadIdx.x mod R into sd[r]; blockDim.x = tpr R, tpr a power of two
+__device__ __forceinline__ void reduce_columns(double2 *sd, double2 v, int R) {
+  const int tpr = blockDim.x / R, lr = threadIdx.x / R;
+  sd[threadIdx.x] = v;
+  __syncthreads();
+  for (int s = tpr / 2; s > 0; s >>= 1) {
+    if (lr < s) {
+      const double2 o = sd[threadIdx.x + s * R];
+      sd[threadIdx.x].x += o.x;
+      sd[threadIdx.x].y += o.y;
     }
-    sd[threadIdx.x] = make_double2(sr, si);
-    __syncthreads();
-    // reduce over lr for each r (tree over the lr index)
-    for (int s = tpr / 2; s > 0; s >>= 1) {
-      if (lr < s) {
-        const double2 o = sd[threadIdx.x + s * R];
-        sd[threadIdx.x].x += o.x;
-        sd[threadIdx.x].y += o.y;
-      }
-      __syncthreads();
-    }
-    if (lr == 0) partial[((size_t)blockIdx.x * nvec + k) * R + r] = sd[r];
     __syncthreads();
   }
 }
 
-__global__ void dots_final_kernel(const double2 *partial, int nblk, int nvec, int R, double2 *out) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nvec * R) return;
+// partial[blk][k][r] = sum_{rows in blk} conj(V_k[row][r]) * w[row][r]; block (blk, k). One vector per block: with all
+// vectors in turn a block spent nvec load latencies and tree reductions in series.
+__global__ void dots_partial_kernel(VecList V, int nvec, const double2 *w, size_t rows, int R, double2 *partial) {
+  extern __shared__ double2 sd[];
+  const int tpr = blockDim.x / R;  // threads per rhs column (blockDim.x is a multiple of R)
+  const int r = threadIdx.x % R, lr = threadIdx.x / R, k = blockIdx.y;
+  const double2 *v = V.v[k];
+  const size_t step = (size_t)gridDim.x * tpr;
   double sr = 0.0, si = 0.0;
-  for (int b = 0; b < nblk; ++b) {
-    const double2 v = partial[(size_t)b * nvec * R + e];
+#pragma unroll 4
+  for (size_t row = blockIdx.x * (size_t)tpr + lr; row < rows; row += step) {
+    const double2 a = v[row * R + r], b = w[row * R + r];
+    sr = fma(a.x, b.x, fma(a.y, b.y, sr));
+    si = fma(a.x, b.y, fma(-a.y, b.x, si));
+  }
+  reduce_columns(sd, make_double2(sr, si), R);
+  if (lr == 0) partial[((size_t)blockIdx.x * nvec + k) * R + r] = sd[r];
+}
+
+// out[e] = sum over blk of partial[blk][e], one warp per e (one thread per e took 24-72 us for 304 blocks)
+__global__ void dots_final_kernel(const double2 *partial, int nblk, int n, double2 *out) {
+  const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (e >= n) return;
+  double sr = 0.0, si = 0.0;
+  for (int b = lane; b < nblk; b += 32) {
+    const double2 v = partial[(size_t)b * n + e];
     sr += v.x;
     si += v.y;
   }
-  out[e] = make_double2(sr, si);
+  for (int o = 16; o > 0; o >>= 1) {
+    sr += __shfl_xor_sync(0xffffffffu, sr, o);
+    si += __shfl_xor_sync(0xffffffffu, si, o);
+  }
+  if (lane == 0) out[e] = make_double2(sr, si);
 }
 
 // y[row][r] += sign * sum_k V_k[row][r] * c[k][r]
@@ -84,11 +94,34 @@ __global__ void combine_kernel(VecList V, int nvec, const double2 *c, double sig
   y[e] = acc;
 }
 
-// y = x * s[r] (real scale per rhs)
-__global__ void scale_kernel(const double2 *x, const double *s, double2 *y, size_t rows, int R) {
+// the same with partial[blk][r] = sum of |y|^2 over the block's rows, so that the norm needs no pass of its own
+__global__ void combine_norm_kernel(VecList V, int nvec, const double2 *c, double sign, double2 *y, size_t rows, int R,
+                                    double2 *partial) {
+  extern __shared__ double2 sd[];
+  const int tpr = blockDim.x / R, r = threadIdx.x % R, lr = threadIdx.x / R;
+  const size_t step = (size_t)gridDim.x * tpr;
+  double s2 = 0.0;
+  for (size_t row = blockIdx.x * (size_t)tpr + lr; row < rows; row += step) {
+    const size_t e = row * R + r;
+    double2 acc = y[e];
+    for (int k = 0; k < nvec; ++k) {
+      const double2 a = V.v[k][e], h = c[k * R + r];
+      acc.x = fma(sign * a.x, h.x, fma(-sign * a.y, h.y, acc.x));
+      acc.y = fma(sign * a.x, h.y, fma(sign * a.y, h.x, acc.y));
+    }
+    y[e] = acc;
+    s2 = fma(acc.x, acc.x, fma(acc.y, acc.y, s2));
+  }
+  reduce_columns(sd, make_double2(s2, 0.0), R);
+  if (lr == 0) partial[(size_t)blockIdx.x * R + r] = sd[r];
+}
+
+// y = x / sqrt(s2[r]), zero where s2[r] is zero: the next basis vector, without a round trip to the host
+__global__ void normalise_kernel(const double2 *x, const double2 *s2, double2 *y, size_t rows, int R) {
   const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= rows * R) return;
-  const double f = s[e % R];
+  const double h = sqrt(fmax(0.0, s2[e % R].x));
+  const double f = h > 0.0 ? 1.0 / h : 0.0;
   y[e] = make_double2(x[e].x * f, x[e].y * f);
 }
 
@@ -163,20 +196,50 @@ struct Solver {
     else apply_padded(c, x, y, R, true, false, st);
   }
 
-  // out[k][r] = <V_k, w> for k < nvec (device), copied to host h (nvec * R)
-  void dots(const VecList &V, int nvec, const double2 *w, double2 *dout) {
-    int tpb = 256;
-    const int tpr = std::max(1, tpb / R);
+  // threads and blocks of the reductions: a power of two of rows side by side, eight rows and more per thread
+  void reduction_shape(int nvec, int &tpb, int &nblk) const {
+    const int tpr = std::max(1, 256 / R);
     int p2 = 1;
     while (p2 * 2 <= tpr) p2 *= 2;
     tpb = p2 * R;
-    const int nblk = (int)std::min<size_t>((size_t)sm_count() * 2, (rows + p2 - 1) / p2);
+    const size_t most = std::max<size_t>(1, (size_t)sm_count() * 8 / nvec), want = (rows + (size_t)p2 * 8 - 1) / ((size_t)p2 * 8);
+    nblk = (int)std::max<size_t>(1, std::min(want, std::min<size_t>(most, (size_t)sm_count() * 2)));
+  }
+
+  // out[k][r] = <V_k, w> for k < nvec (device)
+  void dots(const VecList &V, int nvec, const double2 *w, double2 *dout) {
+    int tpb, nblk;
+    reduction_shape(nvec, tpb, nblk);
     c->w_tmp.reserve((size_t)nblk * nvec * R);
-    dots_partial_kernel<<<nblk, tpb, tpb * sizeof(double2), st>>>(V, nvec, w, rows, R, c->w_tmp.ptr);
+    dots_partial_kernel<<<dim3(nblk, nvec), tpb, tpb * sizeof(double2), st>>>(V, nvec, w, rows, R, c->w_tmp.ptr);
     SG_CUDA(cudaGetLastError());
-    dots_final_kernel<<<nblocks((size_t)nvec * R), 256, 0, st>>>(c->w_tmp.ptr, nblk, nvec, R, dout);
-    SG_CUDA(cudaGetLastError());
+    final_sum(nblk, nvec * R, dout);
     *launches += 2;
+  }
+
+  void final_sum(int nblk, int n, double2 *dout) {
+    dots_final_kernel<<<(n + 3) / 4, 128, 0, st>>>(c->w_tmp.ptr, nblk, n, dout);
+    SG_CUDA(cudaGetLastError());
+  }
+
+  // y += sign sum_k V_k coef_k and dn[r] = |y_r|^2
+  void combine_norm(const VecList &V, int nvec, const double2 *coef, double sign, double2 *y, double2 *dn) {
+    int tpb, nblk;
+    reduction_shape(1, tpb, nblk);
+    nblk = (int)std::min<size_t>((rows * R + tpb - 1) / tpb, (size_t)sm_count() * 8);
+    c->w_tmp.reserve((size_t)nblk * R);
+    combine_norm_kernel<<<nblk, tpb, tpb * sizeof(double2), st>>>(V, nvec, coef, sign, y, rows, R, c->w_tmp.ptr);
+    SG_CUDA(cudaGetLastError());
+    final_sum(nblk, R, dn);
+    *launches += 2;
+  }
+
+  // device scalars to the host (pinned, kept with the context)
+  const double2 *fetch(const double2 *d, size_t n) {
+    c->h_scalars.reserve(n);
+    SG_CUDA(cudaMemcpyAsync(c->h_scalars.ptr, d, n * sizeof(double2), cudaMemcpyDeviceToHost, st));
+    SG_CUDA(cudaStreamSynchronize(st));
+    return c->h_scalars.ptr;
   }
 
   void combine(const VecList &V, int nvec, const double2 *coef, double sign, double2 *y) {
@@ -237,6 +300,7 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
   c->w_r.reserve(len);
   c->w_hcol.reserve((size_t)kHcol * R);
   c->w_red.reserve((size_t)4 * R + 4);
+  c->w_tmp.reserve((size_t)(sm_count() * 8 + kMaxVec) * R);  // all reductions of the solve
   double2 *V0 = c->w_basis.ptr;
   double2 *w = c->w_w.ptr;
   double2 *r = c->w_r.ptr;
@@ -252,8 +316,7 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
   VecList L1{};
   L1.v[0] = b;
   S.dots(L1, 1, b, dh);
-  SG_CUDA(cudaMemcpyAsync(hb.data(), dh, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-  SG_CUDA(cudaStreamSynchronize(S.st));
+  std::copy_n(S.fetch(dh, R), R, hb.begin());
   std::vector<double> bnrm(R), atol(R), ptol(R), pfac(R, 1.0), presid(R, 0.0), rnorm(R, 0.0);
   std::vector<char> active(R, 1);
   for (int q = 0; q < R; ++q) {
@@ -268,8 +331,7 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
   if (!zero_x0) {
     L1.v[0] = x;
     S.dots(L1, 1, x, dh);
-    SG_CUDA(cudaMemcpyAsync(hb.data(), dh, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-    SG_CUDA(cudaStreamSynchronize(S.st));
+    std::copy_n(S.fetch(dh, R), R, hb.begin());
     bool allzero = true;
     for (int q = 0; q < R; ++q) allzero &= hb[q].x == 0.0;
     zero_x0 = allzero;
@@ -284,8 +346,7 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
     // already converged at x0?
     L1.v[0] = r;
     S.dots(L1, 1, r, dh);
-    SG_CUDA(cudaMemcpyAsync(hb.data(), dh, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-    SG_CUDA(cudaStreamSynchronize(S.st));
+    std::copy_n(S.fetch(dh, R), R, hb.begin());
     for (int q = 0; q < R; ++q) {
       rnorm[q] = std::sqrt(std::max(0.0, hb[q].x));
       if (active[q] && rnorm[q] < atol[q]) {
@@ -298,7 +359,6 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
 
   std::vector<cd> H((size_t)restart * (restart + 1) * R), G((size_t)restart * R), Sv((size_t)(restart + 1) * R);
   std::vector<double> Gc((size_t)restart * R);
-  std::vector<double> hscale(R), hmask(R);
   std::vector<int> colstop(R);
   std::vector<char> inner_done(R), breakdown(R);
   std::vector<int> stalls(R, 0);
@@ -313,11 +373,11 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
     // v0 = r / ||r||
     L1.v[0] = r;
     S.dots(L1, 1, r, dh);
-    SG_CUDA(cudaMemcpyAsync(hb.data(), dh, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-    SG_CUDA(cudaStreamSynchronize(S.st));
+    normalise_kernel<<<nblocks(len), 256, 0, S.st>>>(r, dh, Vk(0), S.rows, R);
+    SG_CUDA(cudaGetLastError());
+    const double2 *hr = S.fetch(dh, R);
     for (int q = 0; q < R; ++q) {
-      const double nr = std::sqrt(std::max(0.0, hb[q].x));
-      hscale[q] = nr > 0 ? 1.0 / nr : 0.0;
+      const double nr = std::sqrt(std::max(0.0, hr[q].x));
       for (int k = 0; k <= restart; ++k) Sv[(size_t)k * R + q] = 0.0;
       Sv[q] = nr;
       inner_done[q] = active[q] ? 0 : 1;
@@ -325,10 +385,6 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
       colstop[q] = -1;
       if (active[q] && nr == 0.0) inner_done[q] = 1;
     }
-    double *dscale = c->w_red.ptr;
-    SG_CUDA(cudaMemcpyAsync(dscale, hscale.data(), R * sizeof(double), cudaMemcpyHostToDevice, S.st));
-    scale_kernel<<<nblocks(len), 256, 0, S.st>>>(r, dscale, Vk(0), S.rows, R);
-    SG_CUDA(cudaGetLastError());
 
     int col = 0;
     for (col = 0; col < restart; ++col) {
@@ -352,24 +408,22 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
       // pass 2: re-orthogonalise, then ||w||^2
       double2 *dh2 = dh + (size_t)(col + 2) * R;
       S.dots(L, col + 1, w, dh2);
-      S.combine(L, col + 1, dh2, -1.0, w);
       double2 *dn = dh2 + (size_t)(col + 1) * R;
-      L1.v[0] = w;
-      S.dots(L1, 1, w, dn);
-      const size_t nh = (size_t)(2 * col + 4) * R;
-      SG_CUDA(cudaMemcpyAsync(hb.data(), dh, nh * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-      SG_CUDA(cudaStreamSynchronize(S.st));
+      S.combine_norm(L, col + 1, dh2, -1.0, w, dn);
+      // v_{col+1} = w / h1
+      normalise_kernel<<<nblocks(len), 256, 0, S.st>>>(w, dn, Vk(col + 1), S.rows, R);
+      SG_CUDA(cudaGetLastError());
+      const double2 *hv = S.fetch(dh, (size_t)(2 * col + 4) * R);
       inner_iter++;
       for (int q = 0; q < R; ++q) {
         cd *h = &H[((size_t)q * restart + col) * (restart + 1)];
-        const double h0 = std::sqrt(std::max(0.0, hb[(size_t)(col + 1) * R + q].x));
+        const double h0 = std::sqrt(std::max(0.0, hv[(size_t)(col + 1) * R + q].x));
         for (int k = 0; k <= col; ++k) {
-          const double2 a = hb[(size_t)k * R + q], a2 = hb[(size_t)(col + 2 + k) * R + q];
+          const double2 a = hv[(size_t)k * R + q], a2 = hv[(size_t)(col + 2 + k) * R + q];
           h[k] = cd(a.x + a2.x, a.y + a2.y);
         }
-        const double h1 = std::sqrt(std::max(0.0, hb[(size_t)(2 * col + 3) * R + q].x));
+        const double h1 = std::sqrt(std::max(0.0, hv[(size_t)(2 * col + 3) * R + q].x));
         h[col + 1] = h1;
-        hscale[q] = (h1 > 0) ? 1.0 / h1 : 0.0;
         if (inner_done[q]) continue;
         bool bd = false;
         if (h1 <= eps * h0) {
@@ -401,10 +455,6 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
           breakdown[q] = bd;
         }
       }
-      // v_{col+1} = w / h1
-      SG_CUDA(cudaMemcpyAsync(dscale, hscale.data(), R * sizeof(double), cudaMemcpyHostToDevice, S.st));
-      scale_kernel<<<nblocks(len), 256, 0, S.st>>>(w, dscale, Vk(col + 1), S.rows, R);
-      SG_CUDA(cudaGetLastError());
     }
     // y = H^{-1} S per rhs; x += V y
     std::vector<double2> ycoef((size_t)(restart + 1) * R, make_double2(0, 0));
@@ -441,8 +491,7 @@ static GmresResult gmres_lockstep(Solver &S, const double2 *b, double2 *x, doubl
     SG_CUDA(cudaGetLastError());
     L1.v[0] = r;
     S.dots(L1, 1, r, dh);
-    SG_CUDA(cudaMemcpyAsync(hb.data(), dh, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-    SG_CUDA(cudaStreamSynchronize(S.st));
+    std::copy_n(S.fetch(dh, R), R, hb.begin());
     for (int q = 0; q < R; ++q) {
       const double before = rnorm[q];
       rnorm[q] = std::sqrt(std::max(0.0, hb[q].x));
@@ -726,8 +775,7 @@ static GmresResult block_gmres(Solver &S, const double2 *b, double2 *x, double r
     VecList L{};
     L.v[0] = v;
     S.dots(L, 1, v, c->w_hcol.ptr);
-    SG_CUDA(cudaMemcpyAsync(hb.data(), c->w_hcol.ptr, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-    SG_CUDA(cudaStreamSynchronize(S.st));
+    std::copy_n(S.fetch(c->w_hcol.ptr, R), R, hb.begin());
     out.resize(R);
     for (int q = 0; q < R; ++q) out[q] = std::sqrt(std::max(0.0, hb[q].x));
   };
@@ -889,8 +937,7 @@ static GmresResult refine_mixed(Solver &S, const double2 *b, double2 *x, double 
   VecList L1{};
   L1.v[0] = b;
   S.dots(L1, 1, b, dh);
-  SG_CUDA(cudaMemcpyAsync(hb.data(), dh, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-  SG_CUDA(cudaStreamSynchronize(S.st));
+  std::copy_n(S.fetch(dh, R), R, hb.begin());
   std::vector<double> bnrm(R);
   for (int q = 0; q < R; ++q) bnrm[q] = std::sqrt(std::max(0.0, hb[q].x));
   std::vector<char> done(R, 0);
@@ -901,8 +948,7 @@ static GmresResult refine_mixed(Solver &S, const double2 *b, double2 *x, double 
   double prev_worst = 0.0;
   L1.v[0] = x;
   S.dots(L1, 1, x, dh);
-  SG_CUDA(cudaMemcpyAsync(hb.data(), dh, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-  SG_CUDA(cudaStreamSynchronize(S.st));
+  std::copy_n(S.fetch(dh, R), R, hb.begin());
   bool x0_zero = true;
   for (int q = 0; q < R; ++q) x0_zero &= hb[q].x == 0.0;
   for (steps = 0; steps <= max_steps; ++steps) {
@@ -917,8 +963,7 @@ static GmresResult refine_mixed(Solver &S, const double2 *b, double2 *x, double 
     }
     L1.v[0] = rr;
     S.dots(L1, 1, rr, dh);
-    SG_CUDA(cudaMemcpyAsync(hb.data(), dh, R * sizeof(double2), cudaMemcpyDeviceToHost, S.st));
-    SG_CUDA(cudaStreamSynchronize(S.st));
+    std::copy_n(S.fetch(dh, R), R, hb.begin());
     double worst = 0.0;
     std::vector<double> rn(R);
     for (int q = 0; q < R; ++q) {

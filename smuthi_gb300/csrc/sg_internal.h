@@ -61,6 +61,27 @@ struct DevBuf {
   }
 };
 
+// pinned host memory, the same way
+template <typename T>
+struct PinnedBuf {
+  T *ptr = nullptr;
+  size_t n = 0;
+  PinnedBuf() = default;
+  PinnedBuf(const PinnedBuf &) = delete;
+  PinnedBuf &operator=(const PinnedBuf &) = delete;
+  ~PinnedBuf() {
+    if (ptr) cudaFreeHost(ptr);
+  }
+  void reserve(size_t count) {
+    if (count <= n && ptr) return;
+    if (ptr) cudaFreeHost(ptr);
+    ptr = nullptr;
+    n = 0;
+    SG_CUDA(cudaMallocHost(&ptr, count * sizeof(T)));
+    n = count;
+  }
+};
+
 // ---------------------------------------------------------------- coupling launch parameters
 // Vectors handled by the kernels are "padded": [particle][blocksize][nrhs] complex double.
 struct CouplingLaunch {
@@ -310,6 +331,7 @@ struct sg_context {
   sg::DevBuf<double> w_red;
   sg::DevBuf<double2> w_hcol;
   std::vector<double> h_red;
+  sg::PinnedBuf<double2> h_scalars;  // Arnoldi scalars on the host
 
   // learned preconditioner: k-nearest-neighbour graphs with their near-field blocks T_i W_ij
   struct PGraph {
