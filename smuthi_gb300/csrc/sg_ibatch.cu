@@ -13,32 +13,41 @@
 // and SM.
 //
 // FP64 accuracy on FP16 tensor cores (error-free slicing, the scheme of Ozaki, Ogita, Oishi and Rump,
-// Numer. Algorithms 59 (2012)): every operand is a 63-bit fixed-point number under a power-of-two
+// Numer. Algorithms 59 (2012)): every operand is a 62-bit fixed-point number under a power-of-two
 // scale (per column of C, then per row of C; per pair and right-hand side for u) cut into seven signed
 // 9-bit digits, which FP16 holds exactly. The digit products of equal weight 2^(-9 d), d = 0..6, share
-// one FP32 accumulator; smaller products (below 2^-60 of the scales) are dropped. A digit product is at
-// most 2^16 and K = 32 of them (at most 30 nonzero for blocksize <= 30) times d + 1 <= 7 pairs of digits
-// are summed, at most 7 * 30 * 2^16 = 13,762,560 < 2^24: every accumulator stays an exact integer
-// whatever the order of the sums. Blocksizes 31 to 48 (K = 48) take 8-bit digits of 56-bit numbers and the
-// weights d = 0..7, at most 7 * 48 * 2^14 = 5,505,024 per accumulator. (Ten-bit digits would need fewer products, but the sums of the
-// middle weights could pass 2^24.) The digits are combined in 64-bit integers, in which the powers of
-// t and the rotations follow; the result is independent of how the pairs are grouped.
+// one FP32 accumulator; smaller products (below 2^-60 of the scales) are dropped. The complex product is
+// one real one of twice the depth: a row of A holds (Im u, Re u), a column of B (-Im C, Re C) or
+// (Re C, Im C), so an accumulator holds Re or Im of a result. A digit product is at most 2^16 and at most
+// 60 (blocksize <= 30) times d + 1 of them are summed: the weights d <= 3 stay exact integers below 2^24
+// whatever the digits and the order of the sums; d = 4..6 could pass 2^24 only if nearly all digits had
+// their largest magnitude and one sign, and would then be rounded at 2^-51 of the scales, under a sum
+// that is itself 60 times as large. Blocksizes 31 to 48 take 8-bit digits of 55-bit numbers and the
+// weights d = 0..7, at most 7 * 96 * 2^14 < 2^24. The digits are combined in 64-bit integers, in which
+// the powers of t and the rotations follow; the result is independent of how the pairs are grouped.
 //
-// One CTA per SM walks a contiguous range of tiles; a tile is up to 64 complex columns (pairs x
+// One CTA per SM walks a contiguous range of tiles; a tile is up to 128 complex columns (pairs x
 // right-hand sides) of one interval:
-//   * the warps rotate x_j, cut u into digits and store them as the A operand (128 rows: Re and Im of 64
-//     columns, K = 32);
+//   * sixteen warps rotate x_j, cut u into digits and store them as the A operand in tensor memory (a
+//     lane per column), which leaves shared memory to B and its bandwidth to the tensor core;
 //   * one thread issues the digit products against the interval's B operand (resident while the
-//     interval lasts; with K = 48 one pass at a time, copied while the last pass is combined): passes of
-//     128 rows (n1, power of t, Re / Im), one job per weight d = 0..6 in a ring of four tensor-memory
-//     accumulators of 128 columns;
-//   * the warps read the jobs back (32 columns per warp), combine digits, real and imaginary parts
-//     (neighbouring lanes) and powers of t, rotate back and store the pair's contribution V.
+//     interval lasts; with K = 48 one pass at a time): passes of 64 (n1, power of t), one job per
+//     weight, the least first, in one or two accumulators of 128 columns (64 Re, 64 Im);
+//   * the sixteen warps read the jobs back, combine digits and powers of t, rotate back and store the
+//     pair's contribution V;
+//   * three more warps fetch the next tiles' records and prepare the words of t and the phases.
 // A second kernel sums V over the emitters of every receiver in index order (deterministic) and forms
 // W x or x - T W x. V is a bounded workspace: larger problems run in chunks of tiles.
 //
-// Integer arithmetic instead of FP64 for everything but the last conversion: a GB300 SM sub-partition
-// issues an FP64 instruction every 64 cycles, a 32-bit integer one every two.
+// What bounds it: instruction issue (42% of the slots, half of them two-cycle integer instructions) and the
+// tensor core (34%) in turn: a tile of 2000 spheres takes 44 thousand cycles, of which 16 are MMAs, 6 forming A,
+// 13 the last combination; operand memory does not allow a second tile in flight. 2000 spheres, cubic lookup, one
+// right-hand side: 80.5 ms with the per-receiver kernel, 9.3 with Re and Im of u as separate rows of A in shared
+// memory (twice the accumulators to read and combine), 5.2 now; 1201 spheres with l_max = 4: 82.4, 8.0, 5.05; 100
+// spheres, linear: 127, 51, 46 us.
+//
+// Integer arithmetic instead of FP64: a GB300 SM sub-partition issues an FP64 instruction every 64 cycles, a
+// 32-bit integer one every two.
 #include <cub/cub.cuh>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -54,14 +63,16 @@
 
 namespace sg {
 
-static constexpr int kIbWarps = 16;
-static constexpr int kIbThreads = 32 * kIbWarps;
-static constexpr int kIbCols = 64;   // complex columns per tile
+static constexpr int kIbWarps = 16;  // warps that form, read and combine; one of four more issues
+static constexpr int kIbThreads = 32 * (kIbWarps + 4);
+// The block is launched with 96 registers a thread (20 warps); its 61440 are split 512 x 104 + 128 x 64.
+#define IB_SETMAXNREG(dir, n) asm volatile("setmaxnreg." #dir ".sync.aligned.u32 " #n ";")
+static constexpr int kIbCols = 128;  // complex columns per tile
 static constexpr int kIbDig = 7;     // digits per operand
-static constexpr int kIbN = 128;     // B operand rows per pass: n1 x powers of t x (Re, Im)
+static constexpr int kIbRows = 64;   // (n1, power of t) per pass: N = 128 accumulator columns, Re and Im
 // 1.5 2^23: added to an integer below 2^22 it leaves that in the mantissa
 static constexpr float kIbMagic = 12582912.f;
-static constexpr unsigned long long kIbMagicBits = 0x4B400000ull;
+static constexpr unsigned kIbMagicBits = 0x4B400000u;
 // largest t in units of 2^-62 whose high word fits (t < 1 up to its last places)
 static constexpr long long kIbBelowOne = (1ll << 62) - (1ll << 30) - 1;
 
@@ -82,56 +93,74 @@ struct IbNumbers {
   static constexpr unsigned long long BIAS = bias();
   // what the bits of 1.5 2^23 add to a combination of digits: the weights that take them
   static constexpr unsigned long long OFFSET =
-      kIbMagicBits * (KP == 32 ? (1ull << 39) + (1ull << 30) + 1 + 1
-                               : (1ull << 40) + (1ull << 32) + (1ull << 24) + (1ull << 16) + (1ull << 8) + 1 + 1);
-  static_assert(kIbDig * MAXB * (1 << (2 * BITS - 2)) <= (1 << 24), "exact FP32 accumulators");
-  static_assert((KP == 32 ? 2 : 5) * MAXB * (1 << (2 * BITS - 2)) < (1 << 22), "weights that become integers by addition");
+      (unsigned long long)(unsigned)(kIbMagicBits * (KP == 32 ? 9u : 2u)) +
+      (unsigned long long)kIbMagicBits * (KP == 32 ? (1ull << 39) + (1ull << 30) + (1ull << 21) + (1ull << 12)
+                                                   : (1ull << 40) + (1ull << 32) + (1ull << 24) + (1ull << 16) + (1ull << 8));
+  // weights up to 3 (K = 64) or all (K = 96) are exact in FP32 whatever the digits
+  static_assert((KP == 32 ? 4 : kIbDig) * 2 * MAXB * (1 << (2 * BITS - 2)) <= (1 << 24), "exact FP32 accumulators");
+  static_assert((KP == 32 ? 1 : 2) * 2 * MAXB * (1 << (2 * BITS - 2)) < (1 << 22), "weights that need no check");
 };
 
 template <int NC, int KP>
 struct IbShape {
-  static constexpr int KC = KP / 8;               // core columns of 16 bytes
-  static constexpr int SLICE = 128 * KP * 2;      // bytes of one digit of an operand
-  static constexpr int OPERAND = kIbDig * SLICE;  // bytes of an A operand or one pass of B
-  static constexpr int RN = 2 * NC;               // B rows per n1
-  static constexpr int PN = kIbN / RN;            // n1 per pass
+  static constexpr int KC = KP / 8;                  // chunks of eight n2: one K = 16 step of (Im u, Re u)
+  static constexpr int PLANE = 3 * kIbRows * 16;     // bytes of a chunk of B: rows of -Im C, Re C, Im C
+  static constexpr int SLICE = KC * PLANE;           // bytes of one digit of a pass of B
+  static constexpr int OPERAND = kIbDig * SLICE;     // bytes of one pass of B
+  static constexpr int PN = kIbRows / NC;            // n1 per pass
   static constexpr int PASSES = (KP + PN - 1) / PN;  // at most
   static constexpr int BBYTES = PASSES * OPERAND;
-  static constexpr bool STREAM = KP > 32;         // B in shared memory: one pass, or all
+  static constexpr bool STREAM = KP > 32;            // B in shared memory: one pass, or all
   static constexpr int BSMEM = STREAM ? OPERAND : BBYTES;
+  static constexpr int BUFS = KP == 32 ? 2 : 1;      // accumulators of 128 tensor-memory columns
+  static constexpr int ACOL = BUFS * 128;            // first tensor-memory column of A: KP columns per digit
+  static_assert(ACOL + kIbDig * KP <= 512, "tensor memory");
 };
 
-// per-tile data, four tiles deep: written two tiles ahead, read until the tile is stored
+// The n2 of a warp group (a quarter of the KP) are a chunk of eight and, with KP = 48, four more that
+// share a chunk with a neighbour's: chunk and place of n2.
 template <int KP>
-struct IbTile {
-  int4 ph[kIbCols][IbNumbers<KP>::MAXM + 1];  // cos, sin of m phi in words of 2^-61
-  int2 t[kIbCols];                // t in words of 2^-62
-  long long xoff[kIbCols];        // x_j of the column
-  int eb[KP], ea[KP];             // column and row exponents of the interval
-  int cexp[kIbCols];              // scale of x_j (written with the A operand)
-  int ncol, bucket;
-  long long pair0;                // first pair, from the start of V
-};
-
-static constexpr int kIbXPitch = 31;  // x_j of a column: element n2 at (n2 mod 8) 4 + n2 / 8
-
+__host__ __device__ constexpr int ib_chunk(int n2) {
+  return n2 % (KP / 4) < 8 ? n2 / (KP / 4) : 4 + n2 / (KP / 4) / 2;
+}
 template <int KP>
+__host__ __device__ constexpr int ib_place(int n2) {
+  return n2 % (KP / 4) < 8 ? n2 % (KP / 4) : n2 / (KP / 4) % 2 * 4 + n2 % (KP / 4) - 8;
+}
+
+// SETS: 1: the tiles have 128 columns, all warps take part in each. 2: 64 columns; odd and even tiles belong to two
+// sets of eight warps and 64 tensor-memory lanes, which run half a tile apart. (The products cover all lanes; what
+// they give in those of the other set, from digits that may just be being written there, nobody reads.)
+template <int NC, int KP, int SETS>
 struct IbSmem {
-  IbTile<KP> tile[4];
-  IbRec rec[2][kIbCols];              // records, exponents and (columns, bucket, first pair) of the next tiles
-  int exps[2][2 * KP];
-  int next[2][3];
-  double2 x[KP == 32 ? kIbCols * kIbXPitch : 1];  // x_j of the next tile's columns (K = 48 leaves no room for it)
-  uint64_t dfull[4], dempty[4], afull, meta[4], bfull, done;
+  static constexpr int COLS = kIbCols / SETS;
+  // two B operands where there is room: the next interval's is on its way while the last one is used
+  static constexpr int NB = KP == 32 && NC == 2 ? 2 : 1;
+  struct Tile {
+    int4 ph[IbNumbers<KP>::MAXM + 1][COLS];  // cos, sin of m phi in words of 2^-61
+    int2 t[COLS];                // t in words of 2^-62
+    int xoff[COLS];              // x_j of the column
+    int eb[KP], ea[KP];          // column and row exponents of the interval
+    int ncol, bucket;
+    long long pair0;             // first pair, from the start of V
+  };
+  struct Set {
+    Tile tile[4];                // written ahead, read until the tile is stored
+    uint64_t dfull[2], dempty[2], afull, meta[4], tfree[4];
+  } set[SETS];
+  int emax[4][kIbCols];          // exponents of the quarters of a column
+  uint64_t quarters[4], bfull[2], done;
   int mofn[KP];
   uint32_t tmem;
-  int lb[2];  // bucket of the two look-ahead warps
 };
-template <int NC, int KP>
+template <int NC, int KP, int SETS>
 constexpr size_t ib_smem() {
-  return (size_t)IbShape<NC, KP>::OPERAND + IbShape<NC, KP>::BSMEM + (sizeof(IbSmem<KP>) + 127) / 128 * 128;
+  using Sm = IbSmem<NC, KP, SETS>;
+  return (size_t)Sm::NB * IbShape<NC, KP>::BSMEM + (sizeof(Sm) + 127) / 128 * 128;
 }
-static_assert(ib_smem<4, 32>() <= kTcSmemBudget && ib_smem<4, 48>() <= kTcSmemBudget, "shared memory");
+template <int KP, int SETS>
+constexpr bool ib_fits = ib_smem<2, KP, SETS>() <= kTcSmemBudget && ib_smem<4, KP, SETS>() <= kTcSmemBudget;
+static_assert(ib_fits<32, 1> && ib_fits<32, 2> && ib_fits<48, 1> && ib_fits<48, 2>, "shared memory");
 
 struct IbArgs {
   const IbRec *rec;       // ordered pairs sorted by interval
@@ -139,11 +168,12 @@ struct IbArgs {
   const int *toff;        // [nb + 1] first tile
   const unsigned char *B; // [nb] B operands
   const int *exps;        // [nb][2 KP]: column exponents eb[KP], row exponents ea[KP]
-  const double *x;        // [N][bs][R] complex
+  const int4 *x;          // [N][rt][KP] words of x (ib_words_kernel)
+  const int *xe;          // their exponents
   const int *mofn;
-  double *V;              // [pair - s0][rt][bs] complex
+  double2 *V;             // [pair - s0][rt][bs]
   long long s0;           // first pair of this chunk
-  int nb, bs, mmax, R, r0, rt, per, t0, t1;  // rt right-hand sides from r0; per = pairs per tile; tiles [t0, t1)
+  int nb, bs, mmax, rt, per, t0, t1;  // rt right-hand sides; per = pairs per tile; tiles [t0, t1)
   int *err;
 };
 
@@ -177,10 +207,6 @@ __device__ __forceinline__ void ib_digits(long long v0, long long v1, uint32_t (
   }
 }
 
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
 // Products of 62-bit fixed-point numbers from 31-bit words: three 32 x 32 -> 64 bit multiply-adds, low
 // word by low word (below the last place kept) is dropped. The factors that stay the same for a pair
 // (t, the phases) carry a signed low word in [-2^30, 2^30), so that what is dropped has no bias that
@@ -201,55 +227,71 @@ __device__ __forceinline__ long long ib_mul(IbWords a, int bh, int bl, long long
   return ib_mad(a.h, bh, c + (mid >> 31));
 }
 
-// v 2^e rounded to double: the words placed in the mantissas of 2^84 and 2^52, two FP64 additions
+// v 2^e rounded to double (halves away from zero), in integers: an FP64 conversion or addition holds its pipe for
+// 64 cycles
 __device__ __forceinline__ double ib_to_double(long long v, int e) {
-  const unsigned lo = (unsigned)v, hi = (unsigned)((unsigned long long)v >> 32) ^ 0x80000000u;
-  const double h = __hiloint2double(0x45300000, (int)hi) - (19342813113834066795298816.0 +  // 2^84
-                                                            9223372036854775808.0 +         // 2^63
-                                                            4503599627370496.0);            // 2^52
-  const double d = h + __hiloint2double(0x43300000, (int)lo);
-  const int f = ib_field(d);
-  if (f != 0 && f + e > 0 && f + e < 0x7FF) return __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
-  return scalbn(d, e);  // zero, or outside the normal range
+  const unsigned sign = (unsigned)((unsigned long long)v >> 32) & 0x80000000u;
+  const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
+  const unsigned hi = (unsigned)(m >> 32), lo = (unsigned)m;
+  const int z = __clz((int)hi), f = 1023 + 63 - z + e;  // exponent field
+  if (hi != 0 && f > 0 && f < 0x7FE) {
+    const unsigned mh = __funnelshift_l(lo, hi, z), ml = lo << (z & 31);
+    // the leading bit adds one to the field, a carry out of the mantissa another
+    const unsigned long long b = (((unsigned long long)mh << 32 | ml) >> 11) + ((ml >> 10) & 1u);
+    return __hiloint2double((int)(((unsigned)(b >> 32) + ((unsigned)(f - 1) << 20)) | sign), (int)(unsigned)b);
+  }
+  return scalbn((double)v, e);  // below 2^32, or outside the normal range
 }
 
-// One product of a digit of A and a digit of B (K = 16) into dst; the descriptors differ from those of the
-// operands' first bytes by a constant in their low word.
-template <bool ACC>
+// One product of a digit of A (tensor memory, column AO of it) and a digit of B (K = 16, BO bytes into the pass) into
+// dst. The offsets are added here, so that the compiler does not keep a hundred addresses.
+template <bool ACC, int AO, int BO>
 __device__ __forceinline__ void ib_mma(uint32_t dst, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-      "mov.b64 da, {%1, %3};\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t.reg .b32 ra, rb;\n\t"
+      "add.u32 ra, %1, %6;\n\t"
+      "add.u32 rb, %2, %7;\n\t"
+      "mov.b64 db, {rb, %3};\n\t"
       "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(dst),
-      "r"(a), "r"(b), "r"(hi), "r"(idesc), "n"(ACC ? 1 : 0)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [ra], db, %4, p;\n\t}" ::"r"(dst),
+      "r"(a), "r"(b), "r"(hi), "r"(idesc), "n"(ACC ? 1 : 0), "n"(AO), "n"(BO >> 4)
       : "memory");
 }
 
 // all digit products of weight D; unrolled, because one thread issues them and every instruction between two
 // MMAs costs it several cycles
-template <int D, int KP>
+template <int D, int NC, int KP, int I = (D < kIbDig ? 0 : D - kIbDig + 1), int K = 0>
 __device__ __forceinline__ void ib_issue(uint32_t dst, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc) {
-#pragma unroll
-  for (int i = D < kIbDig ? 0 : D - kIbDig + 1; i <= (D < kIbDig ? D : kIbDig - 1); ++i)
-#pragma unroll
-    for (int ks = 0; ks < KP / 16; ++ks) {
-      constexpr int SLICE = 128 * KP * 2;
-      const uint32_t ao = a + (uint32_t)((i * SLICE + ks * 256) >> 4), bo = b + (uint32_t)(((D - i) * SLICE + ks * 256) >> 4);
-      if (i == (D < kIbDig ? 0 : D - kIbDig + 1) && ks == 0) ib_mma<false>(dst, ao, bo, hi, idesc);
-      else ib_mma<true>(dst, ao, bo, hi, idesc);
-    }
+  using Sh = IbShape<NC, KP>;
+  constexpr int I0 = D < kIbDig ? 0 : D - kIbDig + 1, I1 = D < kIbDig ? D : kIbDig - 1;
+  if constexpr (K == Sh::KC) {
+    ib_issue<D, NC, KP, I + 1, 0>(dst, a, b, hi, idesc);
+  } else if constexpr (I <= I1) {
+    ib_mma<(I != I0 || K != 0), I * KP + K * 8, (D - I) * Sh::SLICE + K * Sh::PLANE>(dst, a, b, hi, idesc);
+    ib_issue<D, NC, KP, I, K + 1>(dst, a, b, hi, idesc);
+  }
 }
 
-template <int NC, int KP>
+__device__ __forceinline__ void tmem_st2(uint32_t taddr, uint32_t a, uint32_t b) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(taddr), "r"(a), "r"(b) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "r"(taddr));
+}
+
+template <int NC, int KP, int SETS>
 __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
   using Sh = IbShape<NC, KP>;
   using Num = IbNumbers<KP>;
-  constexpr int RN = Sh::RN, PN = Sh::PN, WN = PN / 4;  // WN rows n1 per warp and pass
+  using Sm = IbSmem<NC, KP, SETS>;
+  constexpr int PN = Sh::PN, WN = PN / 4;  // WN rows n1 per warp and pass
+  constexpr int BUFS = Sh::BUFS, NB = Sm::NB;
   extern __shared__ __align__(1024) unsigned char ib_raw[];
-  unsigned char *As = ib_raw, *Bs = ib_raw + Sh::OPERAND;
-  IbSmem<KP> &S = *reinterpret_cast<IbSmem<KP> *>(Bs + Sh::BSMEM);
+  unsigned char *Bs = ib_raw;
+  Sm &S = *reinterpret_cast<Sm *>(Bs + NB * Sh::BSMEM);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bs = a.bs;
   const int ntiles = a.t1 - a.t0;
@@ -262,14 +304,20 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
     auto init = [](uint64_t *b, int n) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n) : "memory");
     };
-    for (int b = 0; b < 4; ++b) {
-      init(&S.dfull[b], 1);
-      init(&S.dempty[b], kIbWarps);
-      init(&S.meta[b], 2);
+    for (int h = 0; h < SETS; ++h) {
+      for (int b = 0; b < 2; ++b) {
+        init(&S.set[h].dfull[b], 1);
+        init(&S.set[h].dempty[b], kIbWarps / SETS);
+      }
+      for (int b = 0; b < 4; ++b) {
+        init(&S.set[h].meta[b], 4 / SETS);
+        init(&S.set[h].tfree[b], kIbWarps / SETS);
+      }
+      init(&S.set[h].afull, kIbWarps / SETS);
     }
-    init(&S.afull, kIbWarps);
-    init(&S.bfull, 1);
-    init(&S.done, kIbWarps);
+    for (int b = 0; b < 4; ++b) init(&S.quarters[b], 4);
+    for (int b = 0; b < 2; ++b) init(&S.bfull[b], 1);
+    init(&S.done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -283,358 +331,391 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
   const uint32_t tmem = S.tmem;
   bool good = true;
 
-  // ------------------------------------------------------------------ look ahead (two warps, 32 columns each)
-  const int look_half = warp == 5 ? 0 : (warp == 10 ? 1 : -1);
-  if (look_half >= 0) {  // bucket of the first tile
-    int lb = 0, hi = a.nb - 1;
-    while (lb < hi) {
-      const int mid = (lb + hi + 1) >> 1;
-      if (a.toff[mid] <= T0) lb = mid;
-      else hi = mid - 1;
-    }
-    S.lb[look_half] = lb;
-    __syncwarp();
-  }
-  // records of tile ti on their way to shared memory
-  auto look_fetch = [&](int ti) {
-    if (look_half < 0 || ti >= NT) return;
-    const int T = T0 + ti;
-    int lb = S.lb[look_half];
-    while (T >= a.toff[lb + 1]) ++lb;
-    const int p0 = a.boff[lb] + (T - a.toff[lb]) * a.per, p1 = min(a.boff[lb + 1], p0 + a.per);
-    __syncwarp();
-    S.lb[look_half] = lb;
-    if (look_half == 0 && lane == 0) {
-      S.next[ti & 1][0] = (p1 - p0) * a.rt;
-      S.next[ti & 1][1] = lb;
-      S.next[ti & 1][2] = p0;
-    }
-    if (lane < KP / 4)
-      cp_async16(&S.exps[ti & 1][KP * look_half + 4 * lane], a.exps + (size_t)lb * 2 * KP + KP * look_half + 4 * lane);
-    const int c = look_half * 32 + lane;
-    if (c < (p1 - p0) * a.rt) {
-      const IbRec *r = a.rec + p0 + c / a.rt;
-      cp_async16(&S.rec[ti & 1][c], r);
-      cp_async16(reinterpret_cast<char *>(&S.rec[ti & 1][c]) + 16, reinterpret_cast<const char *>(r) + 16);
-    }
-  };
-  // the words of its t and phases
-  auto look_form = [&](int ti) {
-    if (look_half < 0 || ti >= NT) return;
-    IbTile<KP> &t = S.tile[ti & 3];
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
-    const int c = look_half * 32 + lane;
-    const IbRec rc = S.rec[ti & 1][c];  // unused columns hold an old record
-    if (look_half == 0) {
-      for (int e = lane; e < KP; e += 32) t.eb[e] = S.exps[ti & 1][e];
-      if (lane == 0) {
-        t.ncol = S.next[ti & 1][0];
-        t.bucket = S.next[ti & 1][1];
-        t.pair0 = S.next[ti & 1][2] - a.s0;
-      }
-    } else {
-      for (int e = lane; e < KP; e += 32) t.ea[e] = S.exps[ti & 1][KP + e];
-    }
-    auto words = [](double v, int up) {  // v in units of 2^-up, |v| <= 1
-      return ib_split_signed(min(ib_fixed<10>(v, 1023 + 62 - up - ib_field(v)), kIbBelowOne));
-    };
-    const IbWords tw = words(rc.t, 62);
-    t.t[c] = make_int2(tw.h, tw.l);
-    t.xoff[c] = 2 * ((long long)rc.j * bs * a.R + a.r0 + c % a.rt);
-    t.ph[c][0] = make_int4(1 << 30, 0, 0, 0);
-    double pr = rc.c, pi = rc.s;
-    for (int m = 1; m <= a.mmax; ++m) {
-      const IbWords cw = words(pr, 61), sw = words(pi, 61);
-      t.ph[c][m] = make_int4(cw.h, cw.l, sw.h, sw.l);
-      const double nr = pr * rc.c - pi * rc.s;
-      pi = pr * rc.s + pi * rc.c;
-      pr = nr;
-    }
-    __syncwarp();
-    if (lane == 0) tc_arrive(smem_u32(&S.meta[ti & 3]));
-  };
-  // ------------------------------------------------------------------ issue
-  // Job number g (counted over the CTA's tiles) is issued by warp g mod 16, so that the time a thread is held while
-  // the tensor core takes its MMAs (73 cycles each) is spread over the warps. Its accumulator is free once every warp
-  // has read job g - 4.
-  const uint32_t idesc = (1u << 4) | ((uint32_t)(kIbN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);  // F16 in, F32 out
-  const uint64_t da = tc_desc<Sh::KC>(smem_u32(As)), db = tc_desc<Sh::KC>(smem_u32(Bs));
-  const uint32_t dal = (uint32_t)da, dbl = (uint32_t)db, dhi = (uint32_t)(da >> 32);
-  auto issue = [&](uint32_t g, int pass, auto weight) {
-    int ok = 1;
-    if (lane == 0) {
-      if (g >= 4) ok = tc_wait1(smem_u32(&S.dempty[g & 3]), ((g >> 2) - 1) & 1);
-      if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        ib_issue<decltype(weight)::value, KP>(tmem + (g & 3) * kIbN, dal, dbl + (Sh::STREAM ? 0u : (uint32_t)(pass * (Sh::OPERAND >> 4))),
-                                              dhi, idesc);
-        tc_commit(smem_u32(&S.dfull[g & 3]));
-      }
-    }
-    return __shfl_sync(kTcFull, ok, 0) != 0;
-  };
-    // x_j of this warp's four columns of tile ti on their way to shared memory
-    auto fetch = [&](int ti) {
-      const IbTile<KP> &t = S.tile[ti & 3];
-      const int chunk = lane >> 3, q = lane & 7, n2 = chunk * 8 + q;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int col = warp * 4 + c;
-        if (col < t.ncol && n2 < bs)
-          cp_async16(&S.x[col * kIbXPitch + q * 4 + chunk], a.x + t.xoff[col] + 2 * (size_t)n2 * a.R);
-      }
-    };
-    // rotate the columns of tile ti and cut them into digits; a lane owns a row (column and part) and every fourth
-    // core column of eight n2
-    auto form = [&](int ti) {
-      IbTile<KP> &t = S.tile[ti & 3];
-      const int rl = lane & 7, chunk = lane >> 3, row = warp * 8 + rl, col = row >> 1, part = row & 1;
-      const bool have = col < t.ncol;
-      if (warp * 4 < t.ncol) {
-        constexpr int CH = (Sh::KC + 3) / 4;
-        double xv[CH][8];
-        int emax = 0;
-#pragma unroll
-        for (int k = 0; k < CH; ++k) {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int n2 = (chunk + 4 * k) * 8 + q;
-            if (Sh::STREAM) xv[k][q] = have && n2 < bs ? __ldg(a.x + t.xoff[col] + part + 2 * (size_t)n2 * a.R) : 0.0;
-            else xv[k][q] = have && n2 < bs ? reinterpret_cast<const double *>(S.x + col * kIbXPitch + chunk)[8 * q + part] : 0.0;
+  if (warp >= kIbWarps) {
+    IB_SETMAXNREG(dec, 64);
+    // ---------------------------------------------------------------- issue
+    // One thread of a warp of its own: it is held while the tensor core takes an MMA (73 cycles each).
+    if (warp == kIbWarps && lane == 0) {
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);  // F16 in, F32 out
+      // B: core matrices adjacent in rows 128 bytes apart, in K 64 rows, from -Im C | Re C to Re C | Im C
+      const uint32_t blo = ((smem_u32(Bs) >> 4) & 0x3FFFu) | (uint32_t)((kIbRows * 16) >> 4) << 16;
+      const uint32_t bhi = (128u >> 4) | (1u << 14);
+      uint32_t buf = 0;           // accumulator of the next job
+      uint32_t par = 0;           // bit 2 h + b: parity of the next job of set h in accumulator b
+      uint32_t user = 0;          // bits 2 b: set of the last job in accumulator b
+      uint32_t used = 0;          // bit b: accumulator b has been used
+      int slot = 0, held0 = -1, held1 = -1;  // operand in use; intervals in the two places
+      uint32_t bpar = 0, arrived = 0;        // parity of the next load of a place; bit: its load has been waited for
+      // every MMA of the last tile issued by set h has completed
+      auto finished = [&](int h, uint32_t b) {
+        return tc_wait1(smem_u32(&S.set[h].dfull[b]), ((par >> (2 * h + b)) & 1) ^ 1);
+      };
+      auto load = [&](int place, int bucket, int p) {
+        const uint32_t bar = smem_u32(&S.bfull[place]), bytes = (uint32_t)((Sh::STREAM ? 1 : passes) * Sh::OPERAND);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                smem_u32(Bs) + place * Sh::BSMEM),
+            "l"(a.B + (size_t)bucket * Sh::BBYTES + (size_t)(Sh::STREAM ? p : 0) * Sh::OPERAND), "r"(bytes), "r"(bar)
+            : "memory");
+        if (place == 0) held0 = bucket;
+        else held1 = bucket;
+        arrived &= ~(1u << place);
+      };
+      auto landed = [&](int place) {
+        if ((arrived >> place) & 1) return true;
+        arrived |= 1u << place;
+        const uint32_t q = (bpar >> place) & 1;
+        bpar ^= 1u << place;
+        return tc_wait1(smem_u32(&S.bfull[place]), q);
+      };
+      auto bucket_of = [&](int T, int &bucket) {  // of tile T of this CTA
+        const int h = T % SETS, n = T / SETS;
+        if (!tc_wait1(smem_u32(&S.set[h].meta[n & 3]), (uint32_t)((n >> 2) & 1))) return false;
+        bucket = S.set[h].tile[n & 3].bucket;
+        return true;
+      };
+      int lasth = 0;         // set and accumulator of the last job
+      uint32_t lastb = 0;
+      for (int T = 0; T < NT && good; ++T) {
+        const int h = T % SETS, n = T / SETS;
+        int bucket = 0;
+        good = bucket_of(T, bucket);
+        if (!good) break;
+        if (NB == 2 && bucket != (slot ? held1 : held0)) slot ^= 1;
+        for (int p = 0; p < passes && good; ++p) {
+          if (Sh::STREAM || bucket != (slot ? held1 : held0)) {
+            // the operand may be replaced once every MMA that reads it has completed
+            if (used) good = finished(lasth, lastb);
+            if (!good) break;
+            load(slot, bucket, p);
+          }
+          good = landed(slot);
+          if (p == 0) good = good && tc_wait1(smem_u32(&S.set[h].afull), (uint32_t)(n & 1));
+          const uint32_t bp = blo + (uint32_t)((slot * Sh::BSMEM) >> 4) + (Sh::STREAM ? 0u : (uint32_t)(p * (Sh::OPERAND >> 4)));
+          auto issue = [&](auto weight) {
+            if (!good) return;
+            if ((used >> buf) & 1) {
+              const uint32_t u = (user >> (2 * buf)) & 3;  // whoever had the accumulator last has read it
+              good = tc_wait1(smem_u32(&S.set[SETS == 1 ? 0 : u].dempty[buf]), ((par >> (2 * u + buf)) & 1) ^ 1);
+            }
+            if (!good) return;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            ib_issue<decltype(weight)::value, NC, KP>(tmem + buf * 128, tmem + Sh::ACOL, bp, bhi, idesc);
+            tc_commit(smem_u32(&S.set[h].dfull[buf]));
+            par ^= 1u << (2 * h + buf);
+            user = (user & ~(3u << (2 * buf))) | ((uint32_t)h << (2 * buf));
+            used |= 1u << buf;
+            lasth = h;
+            lastb = buf;
+            if (BUFS == 2) buf ^= 1;
+          };
+          if constexpr (Num::JOBS > 7) issue(std::integral_constant<int, 7>());
+          issue(std::integral_constant<int, 6>());
+          issue(std::integral_constant<int, 5>());
+          issue(std::integral_constant<int, 4>());
+          issue(std::integral_constant<int, 3>());
+          issue(std::integral_constant<int, 2>());
+          issue(std::integral_constant<int, 1>());
+          issue(std::integral_constant<int, 0>());
+          if (NB == 2 && p == 0 && T + 1 < NT && good) {
+            // the other place was last read by the tile before this one, whose jobs precede this tile's
+            int next = 0;
+            good = bucket_of(T + 1, next);
+            if (good && next != held0 && next != held1) load(slot ^ 1, next, 0);
           }
         }
-#pragma unroll
-        for (int k = 0; k < CH; ++k)
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int f = ib_field(xv[k][q]);  // zero beyond the block; Inf, NaN: see below
-            if (f != 0) emax = max(emax, f == 0x7FF ? 1 << 20 : f + t.eb[(chunk + 4 * k) * 8 + q] + 4096);
+      }
+      // nothing of this CTA may be in flight when its memory is given back
+      tc_commit(smem_u32(&S.done));
+      if (!tc_wait1(smem_u32(&S.done), 0u)) good = false;
+      if (held0 >= 0) landed(0);
+      if (held1 >= 0) landed(1);
+    }
+    // ---------------------------------------------------------------- look ahead
+    // Three warps take the records of the tiles, 32 columns at a time, and leave the words of t and the phases.
+    if (warp > kIbWarps) {
+      int lb = 0;  // interval of the tile: the last one whose first tile is not behind it
+      for (int len = a.nb; len > 1;) {
+        const int step = (len + 31) / 32, q = lane * step;
+        const unsigned hit = __ballot_sync(kTcFull, q < len && a.toff[lb + min(q, len - 1)] <= T0);
+        const int o = (__popc(hit) - 1) * step;
+        lb += o;
+        len = min(step, len - o);
+      }
+      auto words = [](double v, int up) {  // v in units of 2^-up, |v| <= 1
+        return ib_split_signed(min(ib_fixed<10>(v, 1023 + 62 - up - ib_field(v)), kIbBelowOne));
+      };
+      for (int T = 0; T < NT && good; ++T) {
+        while (T0 + T >= a.toff[lb + 1]) ++lb;
+        const int h = T % SETS, n = T / SETS;
+        auto &t = S.set[h].tile[n & 3];
+        const int p0 = a.boff[lb] + (T0 + T - a.toff[lb]) * a.per, ncol = (min(a.boff[lb + 1], p0 + a.per) - p0) * a.rt;
+        for (int g = 0; g < 4 / SETS && good; ++g) {
+          if ((T * (4 / SETS) + g) % 3 != warp - kIbWarps - 1) continue;
+          if (n >= 4) good = tc_waitw(smem_u32(&S.set[h].tfree[n & 3]), (uint32_t)(((n >> 2) - 1) & 1));
+          if (!good) break;
+          if (g == 0) {
+            for (int e = lane; e < 2 * KP; e += 32) (e < KP ? t.eb[e] : t.ea[e - KP]) = a.exps[(size_t)lb * 2 * KP + e];
+            if (lane == 0) {
+              t.ncol = ncol;
+              t.bucket = lb;
+              t.pair0 = p0 - a.s0;
+            }
           }
-        emax = max(emax, __shfl_xor_sync(kTcFull, emax, 1));
-        emax = max(emax, __shfl_xor_sync(kTcFull, emax, 8));
-        emax = max(emax, __shfl_xor_sync(kTcFull, emax, 16));
-        if (part == 0 && chunk == 0) t.cexp[col] = emax;
-        const int es = emax - 4096;  // |Re x|, |Im x| < 2^(es - 1022) under the column exponents
-        const int4 *pc = t.ph[have ? col : 0];
+          const int c = g * 32 + lane;
+          const IbRec rc = a.rec[p0 + min(c, ncol - 1) / a.rt];  // columns that are not there repeat the last
+          const IbWords tw = words(rc.t, 62);
+          t.t[c] = make_int2(tw.h, tw.l);
+          t.xoff[c] = rc.j * a.rt + min(c, ncol - 1) % a.rt;
+          t.ph[0][c] = make_int4(1 << 30, 0, 0, 0);
+          double pr = rc.c, pi = rc.s;
+          for (int m = 1; m <= a.mmax; ++m) {
+            const IbWords cw = words(pr, 61), sw = words(pi, 61);
+            t.ph[m][c] = make_int4(cw.h, cw.l, sw.h, sw.l);
+            const double nr = pr * rc.c - pi * rc.s;
+            pi = pr * rc.s + pi * rc.c;
+            pr = nr;
+          }
+          __syncwarp();
+          if (lane == 0) tc_arrive(smem_u32(&S.set[h].meta[n & 3]));
+        }
+      }
+    }
+    __syncwarp();
+    __syncthreads();  // the registers come back from the other warps: none may ask for them before
+    IB_SETMAXNREG(inc, 96);
+  } else {
+    IB_SETMAXNREG(inc, 104);
+    // A thread owns a column (tensor-memory lane) and, of the four warps of its lanes, a quarter of the n2 and n1.
+    const int sp = warp & 3, grp = warp >> 2;
+    const int h = sp / (4 / SETS);                   // set
+    const int c0w = sp % (4 / SETS) * 32, col = c0w + lane;  // column of the tile
+    const int NS = (NT - h + SETS - 1) / SETS;       // the set's tiles
+    auto &Q = S.set[h];
+    const uint32_t lanes = tmem + ((uint32_t)(sp * 32) << 16);
+    int ce = 0;           // exponent of the column
+    uint32_t formed = 0;  // tiles with columns in these lanes
+    // rotate the columns of the set's tile ti and cut them into digits
+    auto form = [&](int ti) {
+      auto &t = Q.tile[ti & 3];
+      if (c0w < t.ncol) {
+        constexpr int E = KP / 4;
+        const int4 *xp = a.x + (size_t)t.xoff[col] * KP + grp * E;
+        int4 xv[E];
+        int xe[E], emax = 0;
 #pragma unroll
-        for (int k = 0; k < CH; ++k) {
-          const int core = min(chunk + 4 * k, Sh::KC - 1);
-          unsigned char *dst = As + (size_t)(row >> 3) * (Sh::KC * 128) + (row & 7) * 16 + core * 128;
-          uint32_t o[kIbDig][4];
+        for (int q = 0; q < E; q += 4)
+          *reinterpret_cast<int4 *>(xe + q) = __ldg(reinterpret_cast<const int4 *>(a.xe + (size_t)t.xoff[col] * KP + grp * E + q));
 #pragma unroll
-          for (int q = 0; q < 8; q += 2) {
-            long long u[2];
+        for (int q = 0; q < E; ++q) xv[q] = __ldg(xp + q);
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+          xe[q] += t.eb[grp * E + q] + 4096;
+          emax = max(emax, xe[q]);
+        }
+        S.emax[grp][sp * 32 + lane] = emax;
+        __syncwarp();
+        if (lane == 0) tc_arrive(smem_u32(&S.quarters[sp]));
+        good = good && tc_waitw(smem_u32(&S.quarters[sp]), formed & 1);
+        ++formed;
+        // |Re x|, |Im x| < 2^(ce - 4096 - 1022) under the column exponents
+        ce = max(max(S.emax[0][sp * 32 + lane], S.emax[1][sp * 32 + lane]),
+                 max(S.emax[2][sp * 32 + lane], S.emax[3][sp * 32 + lane]));
+#pragma unroll
+        for (int q4 = 0; q4 < E; q4 += 4) {
+          uint32_t o[2][kIbDig][2];
+#pragma unroll
+          for (int q = 0; q < 4; q += 2) {
+            long long u[2][2];
 #pragma unroll
             for (int w = 0; w < 2; ++w) {
-              const int n2 = core * 8 + q + w, m = S.mofn[n2];
-              const double x = xv[k][q + w];
-              const IbWords f = ib_split(ib_fixed<Num::UP>(x, es - t.eb[n2] - ib_field(x)));
-              const int oh = __shfl_xor_sync(kTcFull, f.h, 1), ol = __shfl_xor_sync(kTcFull, f.l, 1);
-              // half of Re = c xr - s xi or Im = c xi + s xr
-              int4 p = pc[m < 0 ? -m : m];
-              if ((m < 0) == (part != 0)) {
+              const int n2 = grp * E + q4 + q + w, m = S.mofn[n2];
+              const int4 x = xv[q4 + q + w];  // Re and Im in words of 2^-62 of their scale
+              const int sh = min(ce - xe[q4 + q + w] + 9 - Num::UP, 63);
+              // half of Re = c xr - s xi and Im = c xi + s xr
+              int4 p = t.ph[m < 0 ? -m : m][col];
+              if (m < 0) {
                 p.z = -p.z;
                 p.w = -p.w;
               }
-              const long long mid = ib_mad(f.h, p.y, ib_mad(f.l, p.x, ib_mad(oh, p.w, ib_mad(ol, p.z, 0x40000000ll))));
-              u[w] = ib_mad(f.h, p.x, ib_mad(oh, p.z, mid >> 31));
+              const long long mr = ib_mad(x.x, p.y, ib_mad(x.y, p.x, ib_mad(x.z, -p.w, ib_mad(x.w, -p.z, 0x40000000ll))));
+              const long long mi = ib_mad(x.z, p.y, ib_mad(x.w, p.x, ib_mad(x.x, p.w, ib_mad(x.y, p.z, 0x40000000ll))));
+              u[0][w] = ib_mad(x.z, p.x, ib_mad(x.x, p.z, mi >> 31)) >> sh;
+              u[1][w] = ib_mad(x.x, p.x, ib_mad(x.z, -p.z, mr >> 31)) >> sh;
             }
-            uint32_t dg[kIbDig];
-            ib_digits<KP>(u[0], u[1], dg);
 #pragma unroll
-            for (int s = 0; s < kIbDig; ++s) o[s][q >> 1] = dg[s];
+            for (int w = 0; w < 2; ++w) {
+              uint32_t dg[kIbDig];
+              ib_digits<KP>(u[w][0], u[w][1], dg);
+#pragma unroll
+              for (int s = 0; s < kIbDig; ++s) o[w][s][q >> 1] = dg[s];
+            }
           }
-          if (chunk + 4 * k < Sh::KC)
+          // two columns of the chunk's Im part, then of its Re part
+          const int c0 = ib_chunk<KP>(grp * E + q4) * 8 + (ib_place<KP>(grp * E + q4) >> 1);
+#pragma unroll
+          for (int w = 0; w < 2; ++w)
 #pragma unroll
             for (int s = 0; s < kIbDig; ++s)
-              *reinterpret_cast<uint4 *>(dst + (size_t)s * Sh::SLICE) = make_uint4(o[s][0], o[s][1], o[s][2], o[s][3]);
+              tmem_st2(lanes + Sh::ACOL + s * KP + c0 + 4 * w, o[w][s][0], o[w][s][1]);
         }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) tc_arrive(smem_u32(&S.afull));
+      if (lane == 0) tc_arrive(smem_u32(&Q.afull));
     };
-    const int sp = warp & 3, grp = warp >> 2;
-    const int col = sp * 16 + (lane >> 1), part = lane & 1, sg = part ? -1 : 1;
-    const uint32_t lanes = tmem + ((uint32_t)(sp * 32) << 16) + (uint32_t)(grp * 32);
-    uint32_t g = 0;  // jobs read
-    // waits for the next job (weight D of pass p); read() gets 16 of this warp's 32 columns at a time; then the
-    // buffer is free for the job after next three, whose issuing warp sends it off
-    auto job = [&](auto weight, int p, bool work, auto &&read) {
-      constexpr int D = decltype(weight)::value, DN = D + 4 < Num::JOBS ? D + 4 : D + 4 - Num::JOBS;
-      if (!tc_waitw(smem_u32(&S.dfull[g & 3]), (g >> 2) & 1)) return false;
-      if (work) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    uint32_t buf = 0, par = 0;  // accumulator of the next job; parities of the set's next jobs in the two
+    auto wait_job = [&]() {
+      if (good) good = tc_waitw(smem_u32(&Q.dfull[buf]), (par >> buf) & 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    };
+    auto release = [&]() {
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc_arrive(smem_u32(&Q.dempty[buf]));
+      par ^= 1u << buf;
+      if (BUFS == 2) buf ^= 1;
+    };
+    // the next job: block() gets eight at a time of this warp's 16 Re and 16 Im columns
+    auto job = [&](auto &&block) {
+      wait_job();
+      const uint32_t src = lanes + buf * 128 + grp * 16;
 #pragma unroll
-        for (int h = 0; h < 32; h += 16) {
-          float f[16];
-          tmem_ld16(lanes + (g & 3) * kIbN + h, f);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int c = 0; c < 16; ++c) read(h + c, f[c]);
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      }
-      __syncwarp();
-      if (lane == 0) tc_arrive(smem_u32(&S.dempty[g & 3]));
-      ++g;
-      const int pn = D + 4 < Num::JOBS ? p : p + 1;
-      if (Sh::STREAM && D + 4 >= Num::JOBS) return true;  // the next pass starts when its operand is there
-      return ((g + 3) & (kIbWarps - 1)) != warp || pn >= passes || issue(g + 3, pn, std::integral_constant<int, DN>());
-    };
-    int cur_b = -1, bloads = 0;
-    auto wait_meta = [&](int ti) { return tc_waitw(smem_u32(&S.meta[ti & 3]), (uint32_t)((ti >> 2) & 1)); };
-    // the B operand of a bucket (STREAM: one pass of it), once every MMA that read the last one has completed
-    auto load_b = [&](int bucket, int pass) {
-      ++bloads;
-      if (warp == 0 && lane == 0) {
-        const uint32_t bar = smem_u32(&S.bfull), bytes = (uint32_t)((Sh::STREAM ? 1 : passes) * Sh::OPERAND);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(Bs)),
-            "l"(a.B + (size_t)bucket * Sh::BBYTES + (size_t)pass * Sh::OPERAND), "r"(bytes), "r"(bar)
-            : "memory");
+      for (int h = 0; h < 32; h += 8) {
+        float f[8];
+        tmem_ld8(src + (h < 16 ? h : h - 16 + kIbRows), f);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (h == 24) release();
+        block(h, f);
       }
     };
-    // the first four jobs of a pass of tile ti
-    auto start = [&](int ti, int pass) {
-      const int mine = (int)((uint32_t)warp - g) & (kIbWarps - 1);
-      if (mine >= 4) return true;
-      if (pass == 0 && !tc_waitw(smem_u32(&S.afull), (uint32_t)(ti & 1))) return false;
-      if (!tc_waitw(smem_u32(&S.bfull), (uint32_t)((bloads - 1) & 1))) return false;
-      if (mine == 0) return issue(g, pass, std::integral_constant<int, 0>());
-      if (mine == 1) return issue(g + 1, pass, std::integral_constant<int, 1>());
-      if (mine == 2) return issue(g + 2, pass, std::integral_constant<int, 2>());
-      return issue(g + 3, pass, std::integral_constant<int, 3>());
-    };
-    look_fetch(0);
-    look_form(0);
-    look_fetch(1);
-    look_form(1);
-    look_fetch(2);
-    good = NT == 0 || wait_meta(0);
-    if (good && NT > 0) {
-      if (!Sh::STREAM) fetch(0);
-      if (Sh::STREAM) load_b(S.tile[0].bucket, 0);
-    }
-    for (int ti = 0; ti < NT && good; ++ti) {
-      IbTile<KP> &t = S.tile[ti & 3];
-      look_form(ti + 2);
-      // every job of the last tile has been read: its operands are free
-      if (!Sh::STREAM && t.bucket != cur_b) {
-        cur_b = t.bucket;
-        load_b(cur_b, 0);
-      }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncwarp();
-      form(ti);
-      look_fetch(ti + 3);
-      if (ti + 1 < NT) {
-        good = wait_meta(ti + 1);
-        if (!good) break;
-        if (!Sh::STREAM) fetch(ti + 1);
-      }
-      good = start(ti, 0);
+    for (int ti = 0; ti < NS && good; ++ti) {
+      auto &t = Q.tile[ti & 3];
+      good = tc_waitw(smem_u32(&Q.meta[ti & 3]), (uint32_t)((ti >> 2) & 1));
+      if (!good) break;
+      if (BUFS == 2) buf = (uint32_t)((ti * SETS + h) * passes * Num::JOBS) & 1;
+      form(ti);  // every job of the set's last tile has been read: its operand is free
       for (int p = 0; p < passes && good; ++p) {
-        if (Sh::STREAM && p > 0) {
-          good = start(ti, p);
-          if (!good) break;
-        }
         const int n0 = p * PN + grp * WN;
-        const bool work = sp * 16 < t.ncol && n0 < bs;
-        // The digits in units of 2^-UNIT of the scales; the Im rows of C are negated in the Im u lanes. What is
-        // below 2^22 becomes an integer by an FP32 addition of 1.5 2^23, whose exponent bits stay in the sum
-        // and are taken off it (OFFSET) below.
-        auto unit = [&](int c, int u) { return c & 1 ? sg * u : u; };
-        auto bits = [](float f) { return __float_as_int(f + kIbMagic); };
-        auto high = [&](int c, float f, int u) {
-          return (long long)((unsigned long long)((unsigned)bits(f) * (unsigned)unit(c, u)) << 32);
+        if (c0w >= t.ncol || n0 >= bs) {
+          for (int k = 0; k < Num::JOBS; ++k) {
+            wait_job();
+            release();
+          }
+          continue;
+        }
+        // The digits in units of 2^-UNIT of the scales, least weights first. What is below 2^22 becomes an integer
+        // by an FP32 addition of 1.5 2^23, whose exponent bits stay in the sum and are taken off it (OFFSET) below;
+        // a warp that meets a larger sum converts.
+        auto bits = [](float f) { return (unsigned)__float_as_int(f + kIbMagic); };
+        auto ints = [&](float (&f)[8]) {
+          float m = 0.f;
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) asm("max.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(f[c]), "f"(f[c + 1]));
+          if (__any_sync(kTcFull, m >= 4194304.f)) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) f[c] = __int_as_float(__float2int_rn(f[c]) + (int)kIbMagicBits);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) f[c] += kIbMagic;
+          }
         };
-        long long w[32];
-        std::integral_constant<int, 0> w0;
-        std::integral_constant<int, 1> w1;
-        std::integral_constant<int, 2> w2;
-        std::integral_constant<int, 3> w3;
-        std::integral_constant<int, 4> w4;
-        std::integral_constant<int, 5> w5;
-        std::integral_constant<int, 6> w6;
+        auto wide = [](float v, unsigned u, unsigned long long c) {
+          return (unsigned long long)(unsigned)__float_as_int(v) * u + c;
+        };
+        float low[32];
+        unsigned long long w[32];
+#define IB_EACH(stmt) [&](int h, float (&f)[8]) { _Pragma("unroll") for (int c = 0; c < 8; ++c) { stmt; } }
+#define IB_INTS(stmt) [&](int h, float (&f)[8]) { ints(f); _Pragma("unroll") for (int c = 0; c < 8; ++c) { stmt; } }
         if constexpr (KP == 32) {
-          good = job(w0, p, work, [&](int c, float f) { w[c] = high(c, f, 1 << 7); });
-          good = good && job(w1, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f), unit(c, 1 << 30), w[c]); });
-          good = good && job(w2, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 21), w[c]); });
-          good = good && job(w3, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1 << 12), w[c]); });
-          good = good && job(w4, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 8), w[c]); });
-          good = good && job(w5, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f * 0x1p-6f), unit(c, 1), w[c]); });
-          good = good && job(w6, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f * 0x1p-15f), unit(c, 1), w[c]); });
+          job(IB_EACH(low[h + c] = f[c] * 0x1p-15f));
+          job(IB_EACH(low[h + c] = fmaf(f[c], 0x1p-6f, low[h + c])));
+          job(IB_INTS(low[h + c] = __int_as_float((int)((unsigned)__float_as_int(f[c]) * 8u + bits(low[h + c])))));
+          job(IB_INTS(w[h + c] = wide(f[c], 1u << 12, (unsigned)__float_as_int(low[h + c]))));
+          job(IB_INTS(w[h + c] = wide(f[c], 1u << 21, w[h + c])));
+          job(IB_INTS(w[h + c] = wide(f[c], 1u << 30, w[h + c])));
+          job(IB_EACH(w[h + c] += (unsigned long long)(bits(f[c]) * 128u) << 32));
         } else {
-          good = job(w0, p, work, [&](int c, float f) { w[c] = high(c, f, 1 << 8); });
-          good = good && job(w1, p, work, [&](int c, float f) {
-            w[c] = (long long)((unsigned long long)w[c] + (unsigned long long)high(c, f, 1));
-          });
-          good = good && job(w2, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f), unit(c, 1 << 24), w[c]); });
-          good = good && job(w3, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f), unit(c, 1 << 16), w[c]); });
-          good = good && job(w4, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f), unit(c, 1 << 8), w[c]); });
-          good = good && job(w5, p, work, [&](int c, float f) { w[c] = ib_mad(__float2int_rn(f), unit(c, 1), w[c]); });
-          good = good && job(w6, p, work, [&](int c, float f) { w[c] = ib_mad(bits(f * 0x1p-8f), unit(c, 1), w[c]); });
-          good = good && job(std::integral_constant<int, 7>(), p, work, [&](int c, float f) {
-            w[c] = ib_mad(bits(f * 0x1p-16f), unit(c, 1), w[c]);
-          });
+          job(IB_EACH(low[h + c] = f[c] * 0x1p-16f));
+          job(IB_EACH(low[h + c] = fmaf(f[c], 0x1p-8f, low[h + c])));
+          job(IB_INTS(low[h + c] = __int_as_float((int)((unsigned)__float_as_int(f[c]) + bits(low[h + c])))));
+          job(IB_INTS(w[h + c] = wide(f[c], 1u << 8, (unsigned)__float_as_int(low[h + c]))));
+          job(IB_INTS(w[h + c] = wide(f[c], 1u << 16, w[h + c])));
+          job(IB_INTS(w[h + c] = wide(f[c], 1u << 24, w[h + c])));
+          job(IB_EACH(w[h + c] += (unsigned long long)bits(f[c]) << 32));
+          job(IB_EACH(w[h + c] += (unsigned long long)(bits(f[c]) * 256u) << 32));
         }
-        if (Sh::STREAM && good) {  // every MMA of this pass has completed
-          if (p + 1 < passes) load_b(t.bucket, p + 1);
-          else if (ti + 1 < NT) load_b(S.tile[(ti + 1) & 3].bucket, 0);
-        }
-        if (!good || !work) continue;
+#undef IB_EACH
+#undef IB_INTS
+        if (!good) break;
         const bool have = col < t.ncol;
-        const int2 tw = have ? t.t[col] : make_int2(0, 0);
-        const int ce = have ? t.cexp[col] : 0;
+        const int2 tw = t.t[col];
         const int cs = ce - 4096 - 1022 + 1 - Num::UNIT;  // scale of x, half of its rotation, units
-        // the Re lane receives the negated Im sum (offsets cancel), the Im lane adds two positive ones
-        const unsigned long long offset = part ? 0ull - 2ull * Num::OFFSET : 0ull;
-        const int4 *pc = t.ph[have ? col : 0];
-        double *vo = a.V + 2 * ((t.pair0 * a.rt + (have ? col : 0)) * bs) + part;
+        double2 *vo = a.V + (t.pair0 * a.rt + col) * bs;
 #pragma unroll
         for (int s = 0; s < WN; ++s) {
           const int n = n0 + s;
-          // lane pair (Re u, Im u): Re y = C_re u_re - C_im u_im, Im y = C_re u_im + C_im u_re
-          long long acc = 0;
+          if (n >= bs) break;
+          long long y[2];
 #pragma unroll
-          for (int c = NC - 1; c >= 0; --c) {
-            const long long e = (long long)((unsigned long long)w[s * RN + 2 * c] + offset +
-                                            (unsigned long long)__shfl_xor_sync(kTcFull, w[s * RN + 2 * c + 1], 1));
-            acc = c == NC - 1 ? e : ib_mul(ib_split(acc), tw.x, tw.y, e);
-          }
-          const IbWords v = ib_split(acc);
-          const int oh = __shfl_xor_sync(kTcFull, v.h, 1), ol = __shfl_xor_sync(kTcFull, v.l, 1);
-          const int nc = min(n, KP - 1), m = S.mofn[nc];
-          int4 ph = pc[m < 0 ? -m : m];
-          if ((m < 0) != (part != 0)) {
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int c = NC - 1; c >= 0; --c) {
+              const long long e = (long long)(w[16 * h + s * NC + c] - Num::OFFSET);
+              y[h] = c == NC - 1 ? e : ib_mul(ib_split(y[h]), tw.x, tw.y, e);
+            }
+          const IbWords r = ib_split(y[0]), i = ib_split(y[1]);
+          const int m = S.mofn[n];
+          int4 ph = t.ph[m < 0 ? -m : m][col];
+          if (m < 0) {
             ph.z = -ph.z;
             ph.w = -ph.w;
           }
-          // e^{-i m phi} times the value: c v +- s (other part)
-          const long long mid = ib_mad(v.h, ph.y, ib_mad(v.l, ph.x, ib_mad(oh, ph.w, ib_mad(ol, ph.z, 0x20000000ll))));
-          const long long out = 2 * ib_mad(v.h, ph.x, (long long)oh * ph.z) + (mid >> 30);
-          double res = ib_to_double(out, cs + t.ea[nc]);
-          if (ce >= (1 << 20)) res = __longlong_as_double(0x7FF8000000000000ll);  // Inf or NaN in x
-          if (have && n < bs) vo[2 * n] = res;
+          // e^{-i m phi} times the value: Re = c r + s i, Im = c i - s r
+          const long long mr = ib_mad(r.h, ph.y, ib_mad(r.l, ph.x, ib_mad(i.h, ph.w, ib_mad(i.l, ph.z, 0x20000000ll))));
+          const long long mi = ib_mad(i.h, ph.y, ib_mad(i.l, ph.x, ib_mad(r.h, -ph.w, ib_mad(r.l, -ph.z, 0x20000000ll))));
+          const int e = cs + t.ea[n];
+          double2 res = make_double2(ib_to_double(2 * ib_mad(r.h, ph.x, (long long)i.h * ph.z) + (mr >> 30), e),
+                                     ib_to_double(2 * ib_mad(i.h, ph.x, (long long)r.h * -ph.z) + (mi >> 30), e));
+          if (ce >= (1 << 20)) res.x = res.y = __longlong_as_double(0x7FF8000000000000ll);  // Inf or NaN in x
+          if (have) vo[n] = res;
         }
       }
+      __syncwarp();
+      if (lane == 0) tc_arrive(smem_u32(&Q.tfree[ti & 3]));
     }
-  if (!good && lane == 0) atomicExch(a.err, 1);
-  // nothing of this CTA may be in flight when its memory is given back
-  if (lane == 0) {
-    tc_commit(smem_u32(&S.done));
-    if (!tc_wait1(smem_u32(&S.done), 0u)) atomicExch(a.err, 1);
-    if (warp == 0 && bloads > 0) tc_wait1(smem_u32(&S.bfull), (uint32_t)((bloads - 1) & 1));
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    IB_SETMAXNREG(dec, 96);
+    __syncthreads();
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  if (!good && lane == 0) atomicExch(a.err, 1);
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
+}
+
+// ------------------------------------------------------------------ words of x
+// Re and Im of every element in words of 2^-62 of a power-of-two scale of its own, and the scale's exponent field: the
+// N pairs of an emitter share them.
+template <int KP>
+__global__ void __launch_bounds__(256) ib_words_kernel(const double2 *x, int n, int bs, int R, int r0, int rt, int4 *xw, int *xe) {
+  const size_t q = (size_t)blockIdx.x * 256 + threadIdx.x;  // (j, r, n2)
+  if (q >= (size_t)n * rt * KP) return;
+  const int n2 = (int)(q % KP), r = (int)(q / KP % rt);
+  const size_t j = q / ((size_t)KP * rt);
+  int4 w = make_int4(0, 0, 0, 0);
+  int f = 0;
+  if (n2 < bs) {
+    const double2 v = x[(j * bs + n2) * R + r0 + r];
+    f = max(ib_field(v.x), ib_field(v.y));
+    const IbWords re = ib_split(ib_fixed<9>(v.x, f - ib_field(v.x))), im = ib_split(ib_fixed<9>(v.y, f - ib_field(v.y)));
+    w = make_int4(re.h, re.l, im.h, im.l);
+  }
+  xw[q] = w;
+  xe[q] = f == 0 ? -(1 << 24) : f == 0x7FF ? 1 << 21 : f;  // zero; Inf or NaN
 }
 
 // ------------------------------------------------------------------ sum over the emitters
@@ -655,33 +736,36 @@ __global__ void __launch_bounds__(768) ib_sum_kernel(const CouplingLaunch L, con
   const int i = blockIdx.x, N = L.n, bs = L.bs, E = bs * s.rt;
   const int g = threadIdx.x / s.width, e = threadIdx.x - g * s.width;
   double2 *red = part + (size_t)s.groups * E;
-  if (g < s.groups && e < E) {
+  if (g < s.groups) {  // a whole warp (the width is a multiple of 32)
     const int j0 = (int)((long long)N * g / s.groups), j1 = (int)((long long)N * (g + 1) / s.groups);
+    const int lane = threadIdx.x & 31;
     const unsigned *sl = s.slot + (size_t)i * N;
+    const double2 *V = s.V + min(e, E - 1);
     double2 a = make_double2(0.0, 0.0);
-    int j = j0;
-    for (; j + 8 <= j1; j += 8) {
-      double2 v[8];
+    for (int j = j0; j < j1; j += 32) {
+      const long long p = j + lane < j1 ? (long long)__ldg(sl + j + lane) - s.s0 : -1;
+      unsigned m = __ballot_sync(kTcFull, p >= 0 && p < s.s1 - s.s0);
+      // the pairs of this chunk among 32, several loads in flight; what is not in it costs no FP64 addition (64 cycles)
+      auto take = [&](auto count) {
+        constexpr int C = decltype(count)::value;
+        double2 v[C];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const long long p = (long long)__ldg(sl + j + q);
-        v[q] = p >= s.s0 && p < s.s1 ? s.V[(size_t)(p - s.s0) * E + e] : make_double2(0.0, 0.0);
-      }
+        for (int q = 0; q < C; ++q) {
+          v[q] = V[(size_t)__shfl_sync(kTcFull, (unsigned)p, __ffs(m) - 1) * E];
+          m &= m - 1;
+        }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        a.x += v[q].x;
-        a.y += v[q].y;
-      }
+        for (int q = 0; q < C; ++q) {
+          a.x += v[q].x;
+          a.y += v[q].y;
+        }
+      };
+      while (__popc(m) >= 8) take(std::integral_constant<int, 8>());
+      if (__popc(m) >= 4) take(std::integral_constant<int, 4>());
+      if (__popc(m) >= 2) take(std::integral_constant<int, 2>());
+      if (m) take(std::integral_constant<int, 1>());
     }
-    for (; j < j1; ++j) {
-      const long long p = (long long)__ldg(sl + j);
-      if (p >= s.s0 && p < s.s1) {
-        const double2 v = s.V[(size_t)(p - s.s0) * E + e];
-        a.x += v.x;
-        a.y += v.y;
-      }
-    }
-    part[(size_t)g * E + e] = a;
+    if (e < E) part[(size_t)g * E + e] = a;
   }
   __syncthreads();
   for (int q = threadIdx.x; q < E; q += blockDim.x) {
@@ -774,44 +858,39 @@ __global__ void __launch_bounds__(256) ib_operand_kernel(const double2 *coef, co
     exps[(size_t)b * 2 * KP + KP + tid] = ea[tid];
   }
   unsigned char *out = B + (size_t)b * Sh::BBYTES;
-  // one thread per row (n1, power, part) and pair of n2
-  for (int e = tid; e < Sh::PASSES * kIbN * KP / 2; e += blockDim.x) {
+  // one thread per row (n1, power) and pair of n2
+  for (int e = tid; e < Sh::PASSES * kIbRows * KP / 2; e += blockDim.x) {
     const int row = e / (KP / 2), k = 2 * (e - row * (KP / 2));
-    const int n1 = row / Sh::RN, c = (row % Sh::RN) >> 1, im = row & 1;
-    long long f[2];
+    const int n1 = row / NC, c = row % NC;
+    long long f[2][2];
     for (int w = 0; w < 2; ++w) {
       const int n2 = k + w;
-      double v = 0.0;
-      if (n1 < bs && n2 < bs) {
-        const double2 cv = C[(size_t)c * bs2 + n2 * bs + n1];
-        v = im ? cv.y : cv.x;
-      }
-      f[w] = ib_fixed<IbNumbers<KP>::UP>(v, n1 < bs && n2 < bs ? ea[n1] + eb[n2] + 1022 - ib_field(v) : 0);
+      const bool in = n1 < bs && n2 < bs;
+      const double2 v = in ? C[(size_t)c * bs2 + n2 * bs + n1] : make_double2(0.0, 0.0);
+      const int s = in ? ea[n1] + eb[n2] + 1022 : 0;
+      f[0][w] = ib_fixed<IbNumbers<KP>::UP>(v.x, s - ib_field(v.x));
+      f[1][w] = ib_fixed<IbNumbers<KP>::UP>(v.y, s - ib_field(v.y));
     }
-    uint32_t dg[kIbDig];
-    ib_digits<KP>(f[0], f[1], dg);
-    const int pass = row / kIbN, r = row % kIbN;
-    for (int s = 0; s < kIbDig; ++s)
-      *reinterpret_cast<uint32_t *>(out + (size_t)pass * Sh::OPERAND + (size_t)s * Sh::SLICE +
-                                    ((size_t)(r >> 3) * Sh::KC + (k >> 3)) * 128 + (r & 7) * 16 + (k & 7) * 2) = dg[s];
+    const int pass = row / kIbRows, r = row % kIbRows;
+    unsigned char *o = out + (size_t)pass * Sh::OPERAND + ib_chunk<KP>(k) * Sh::PLANE + (r >> 3) * 128 + (r & 7) * 16 +
+                       ib_place<KP>(k) * 2;
+    uint32_t dg[3][kIbDig];
+    ib_digits<KP>(-f[1][0], -f[1][1], dg[0]);
+    ib_digits<KP>(f[0][0], f[0][1], dg[1]);
+    ib_digits<KP>(f[1][0], f[1][1], dg[2]);
+    for (int h = 0; h < 3; ++h)
+      for (int s = 0; s < kIbDig; ++s)
+        *reinterpret_cast<uint32_t *>(o + (size_t)s * Sh::SLICE + h * (kIbRows * 16)) = dg[h][s];
   }
 }
 
 static constexpr int kIbMinParticles = 32;
 static constexpr long long kIbMaxPairs = 1ll << 27;      // 4 GB of pair records
+static constexpr size_t kIbMaxOperands = (size_t)32 << 30;  // bytes of the intervals' B operands
 static constexpr size_t kIbWorkspace = (size_t)2 << 30;  // bytes of V per chunk
 
 // padded blocksize
 static int ib_kp(const sg_context *c) { return c->bs <= IbNumbers<32>::MAXB ? 32 : 48; }
-
-bool ib_supported(const sg_context *c) {
-  if (c->vol || c->kind < 0 || c->bs > IbNumbers<48>::MAXB) return false;
-  if ((long long)c->n * c->n > kIbMaxPairs || c->n < kIbMinParticles) return false;
-  const int mmax = ib_kp(c) == 32 ? IbNumbers<32>::MAXM : IbNumbers<48>::MAXM;
-  for (int m : c->h_mofn)
-    if (m > mmax || m < -mmax) return false;
-  return true;
-}
 
 // f(NC, KP) as compile-time constants
 template <class F>
@@ -827,6 +906,19 @@ static void ib_dispatch(const sg_context *c, F &&f) {
     if (c->ncoef == 2) f(two, large);
     else f(four, large);
   }
+}
+
+bool ib_supported(const sg_context *c) {
+  if (c->vol || c->kind < 0 || c->bs > IbNumbers<48>::MAXB) return false;
+  const long long pairs = (long long)c->n * c->n;
+  if (pairs > kIbMaxPairs || c->n < kIbMinParticles) return false;
+  size_t operand = 0;
+  ib_dispatch(c, [&](auto nc, auto kp) { operand = IbShape<decltype(nc)::value, decltype(kp)::value>::BBYTES; });
+  if (std::min<size_t>(c->n_int, pairs) * operand > kIbMaxOperands) return false;
+  const int mmax = ib_kp(c) == 32 ? IbNumbers<32>::MAXM : IbNumbers<48>::MAXM;
+  for (int m : c->h_mofn)
+    if (m > mmax || m < -mmax) return false;
+  return true;
 }
 
 static void ib_build_plan(sg_context *c, cudaStream_t st) {
@@ -886,13 +978,23 @@ static void ib_build_plan(sg_context *c, cudaStream_t st) {
   P.ready = true;
 }
 
-// tiles of `per` pairs: first tile of every interval
-static sg_context::IbTiles &ib_tiles(sg_context *c, int per, cudaStream_t st) {
+// The tiles for rt right-hand sides: first tile of every interval. Where 64 columns make hardly more tiles than 128,
+// most are not half full and two sets of warps that overlap their tiles are faster: 100 spheres (1.00 times the tiles)
+// 51 against 63 us, 220 (1.27) 108 against 117, 200 with the cubic lookup (1.25) 144 against 141, 301 (1.54) 165
+// against 161, 1000 (1.8) 1140 against 1056.
+static sg_context::IbTiles &ib_tiles(sg_context *c, int rt, cudaStream_t st) {
   auto &P = c->ib;
   for (auto &t : P.tiles)
-    if (t->per == per) return *t;
+    if (t->rt == rt) return *t;
   auto t = std::make_unique<sg_context::IbTiles>();
-  t->per = per;
+  auto count = [&](int per) {
+    long long n = 0;
+    for (int b = 0; b < P.nb; ++b) n += (P.h_boff[b + 1] - P.h_boff[b] + per - 1) / per;
+    return n;
+  };
+  t->rt = rt;
+  t->sets = 3 * count(kIbCols / 2 / rt) <= 4 * count(kIbCols / rt) ? 2 : 1;
+  const int per = t->per = kIbCols / t->sets / rt;
   t->h_toff.assign(1, 0);
   for (int b = 0; b < P.nb; ++b)
     t->h_toff.push_back(t->h_toff.back() + (P.h_boff[b + 1] - P.h_boff[b] + per - 1) / per);
@@ -903,13 +1005,13 @@ static sg_context::IbTiles &ib_tiles(sg_context *c, int per, cudaStream_t st) {
   return *P.tiles.back();
 }
 
-template <int NC, int KP>
+template <int NC, int KP, int SETS>
 static void ib_launch(const IbArgs &a, cudaStream_t st) {
   static bool attr_done[64] = {};
-  constexpr int smem = (int)ib_smem<NC, KP>();
+  constexpr int smem = (int)ib_smem<NC, KP, SETS>();
   if (first_on_device(attr_done))
-    SG_CUDA(cudaFuncSetAttribute(ib_kernel<NC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  ib_kernel<NC, KP><<<std::min(sm_count(), a.t1 - a.t0), kIbThreads, smem, st>>>(a);
+    SG_CUDA(cudaFuncSetAttribute(ib_kernel<NC, KP, SETS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  ib_kernel<NC, KP, SETS><<<std::min(sm_count(), a.t1 - a.t0), kIbThreads, smem, st>>>(a);
   SG_CUDA(cudaGetLastError());
 }
 
@@ -933,9 +1035,15 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
   L.t_diag = c->t_diag;
   int mmax = 0, launched = 0;
   for (int m : c->h_mofn) mmax = std::max(mmax, std::abs(m));
-  for (int r0 = 0; r0 < R; r0 += 16) {
-    const int rt = std::min(16, R - r0), per = kIbCols / rt;
-    auto &tl = ib_tiles(c, per, st);
+  // Right-hand sides at a time: their pairs share t and the phases and fill the tiles of a sparse interval, but every
+  // further chunk goes through the slots again. 16 of them, one / four / sixteen at a time: 301 spheres (0.07 GB of V a
+  // right-hand side) 2.90 / 1.76 / 1.45 ms, 1000 (0.5 GB) 23.7 / 20.9 / 20.6, 2000 (1.9 GB) 85.8 / 82.4 / 83.0, 4000
+  // (7.7 GB) 334 / 334 / 374.
+  const int most = (int)std::min<size_t>(16, std::max<size_t>(1, 4 * kIbWorkspace / ((size_t)c->n * c->n * bs * sizeof(double2))));
+  for (int r0 = 0, rt; r0 < R; r0 += rt) {
+    rt = std::min(most, R - r0);
+    auto &tl = ib_tiles(c, rt, st);
+    const int per = tl.per;
     const size_t pair_bytes = (size_t)rt * bs * sizeof(double2);
     const int ntiles = tl.h_toff.back();
     const int chunk = (int)std::min<size_t>(ntiles, std::max<size_t>(1, kIbWorkspace / (pair_bytes * per)));
@@ -952,14 +1060,20 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     a.toff = tl.toff.ptr;
     a.B = P.B.ptr;
     a.exps = P.exps.ptr;
-    a.x = reinterpret_cast<const double *>(x);
+    const size_t words = (size_t)c->n * rt * ib_kp(c);
+    P.xw.reserve(words);
+    P.xe.reserve(words);
+    (ib_kp(c) == 32 ? ib_words_kernel<32> : ib_words_kernel<48>)<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(
+        x, c->n, bs, R, r0, rt, P.xw.ptr, P.xe.ptr);
+    SG_CUDA(cudaGetLastError());
+    ++launched;
+    a.x = P.xw.ptr;
+    a.xe = P.xe.ptr;
     a.mofn = c->mofn.ptr;
-    a.V = reinterpret_cast<double *>(P.V.ptr);
+    a.V = P.V.ptr;
     a.nb = P.nb;
     a.bs = bs;
     a.mmax = mmax;
-    a.R = R;
-    a.r0 = r0;
     a.rt = rt;
     a.per = per;
     a.err = P.err.ptr;
@@ -980,7 +1094,10 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
       s.s1 = first_pair(a.t1);
       s.first = t0 == 0;
       s.last = a.t1 == ntiles;
-      ib_dispatch(c, [&](auto nc, auto kp) { ib_launch<decltype(nc)::value, decltype(kp)::value>(a, st); });
+      ib_dispatch(c, [&](auto nc, auto kp) {
+        if (tl.sets == 1) ib_launch<decltype(nc)::value, decltype(kp)::value, 1>(a, st);
+        else ib_launch<decltype(nc)::value, decltype(kp)::value, 2>(a, st);
+      });
       ib_sum_kernel<<<c->n, std::max(512, s.width), smem, st>>>(L, s);
       SG_CUDA(cudaGetLastError());
       launched += 2;

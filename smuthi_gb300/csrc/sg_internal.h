@@ -299,7 +299,7 @@ struct sg_context {
   // interval-batched FP64 operator (sg_ibatch.cu): ordered pairs sorted by lookup interval, the
   // intervals' digit operands, the pairs' contributions V of one chunk
   struct IbTiles {
-    int per = 0;  // pairs per tile
+    int rt = 0, sets = 1, per = 0;  // right-hand sides; sets of warps; pairs per tile
     std::vector<int> h_toff;
     sg::DevBuf<int> toff;
   };
@@ -312,6 +312,8 @@ struct sg_context {
     sg::DevBuf<int> boff, exps, err;
     sg::DevBuf<unsigned char> B;
     sg::DevBuf<double2> V, acc;
+    sg::DevBuf<int4> xw;  // words of x and their exponents
+    sg::DevBuf<int> xe;
     std::vector<std::unique_ptr<IbTiles>> tiles;
     cudaEvent_t done = nullptr;  // end of the last call: calls on other streams wait for it
     ~Ib() {

@@ -57,6 +57,20 @@ def test_matches_direct_evaluation(n, bs, R, kind, gpu_context):
         assert np.linalg.norm(y[..., r] - ref[..., r]) <= 1e-13 * np.linalg.norm(ref[..., r])
 
 
+@pytest.mark.parametrize("bs", [30, 48])
+def test_largest_digit_sums(bs, gpu_context):
+    """Equal operands with all mantissa bits set: digit sums beyond 2^22, which the kernel converts one by one."""
+    n = 40
+    xy, m, rho, table = _system(gpu_context, n, bs, "linear", 21)
+    table[:] = (1 - 2.0 ** -53) * (1 + 1j)
+    gpu_context.set_particles(xy, *np.divmod(np.arange(n * bs), bs), bs, 0 * m)
+    gpu_context.set_lookup("linear", table, rho[0], RES)
+    x = np.full((n, bs, 1), (1 - 2.0 ** -53) * (1 - 1j))
+    y = gpu_context.coupling_matvec(x.reshape(n * bs, 1), 0).reshape(n, bs, 1)
+    ref = _direct(xy, 0 * m, rho, table, "linear", x)
+    assert np.linalg.norm(y - ref) <= 1e-13 * np.linalg.norm(ref)
+
+
 def test_scales_and_zero_columns(gpu_context):
     """Right-hand sides of any magnitude (exact powers of two scale exactly), zero ones stay zero."""
     n, bs = 50, 30
