@@ -407,7 +407,7 @@ static int matvec_host(sg_context *ctx, const double *x, double *y, int nrhs, in
       throw sg::Error{SG_ERR_CUDA, "pair-symmetric FP32 operator: a bounded wait ran out"};
     if (precision == SG_FP32 && sg::tc_check_error(ctx, st))
       throw sg::Error{SG_ERR_CUDA, "tensor-core operator: a bounded wait ran out"};
-    if (precision == SG_FP64 && sg::ib_check_error(ctx, st))
+    if ((precision == SG_FP64 || precision == SG_DF64) && sg::ib_check_error(ctx, st))
       throw sg::Error{SG_ERR_CUDA, "interval-batched operator: a bounded wait ran out"};
     return SG_OK;
   });
