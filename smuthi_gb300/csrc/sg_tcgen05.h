@@ -56,19 +56,6 @@ __device__ __forceinline__ bool tc_poll(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// the same without waiting
-__device__ __forceinline__ bool tc_poll0(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // one thread: true when the phase of `parity` has completed, false when the budget ran out
 __device__ __forceinline__ bool tc_wait1(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
