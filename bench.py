@@ -262,13 +262,15 @@ def run_ours(args, rank, world, local_rank):
                 3: "sym_kernel (pair-symmetric, two warps per receiver, RHS tile %d)" % t32,
                 4: "tc_coupling_kernel (tcgen05 3xTF32, %d RHS)" % t32,
                 5: "tcsym_kernel (pair-symmetric tcgen05 3xTF32, %d RHS)" % t32}.get(v32, "FP32 operator")
+        if ctx.fp32_batched(R)[0]:
+            name = "ih_kernel (interval-batched, tcgen05 FP16 parts, %d RHS)" % R
         peak, bound = peak32, "fp32"
         byts = algorithmic_bytes(n, bs, kind, n_int, R, True)
     elif msdf >= ms64:
         # double-float kernel on the FP32 pipe: FP64-grade flops against the FP32 pipe's peak
         avg_ms = msdf / max(ndf, 1)
         fl = algorithmic_flops(n, bs, kind, R)
-        peak, bound, name = peak32, "fp32", "coupling_kernel<df64>"
+        peak, bound, name = peak32, "fp32", "SG_DF64 operator: ib_kernel (interval-batched) where it applies"
         byts = algorithmic_bytes(n, bs, kind, n_int, R, False)
     else:
         avg_ms = ms64 / max(n64, 1)
@@ -329,10 +331,12 @@ def run_ours(args, rank, world, local_rank):
                         "residual_arithmetic": args.residual,
                         "batched": True, "x0": "0",
                         "fp32_kernel": dict(zip(("variant", "rhs_tile", "ms_per_receiver", "ms_bucketed", "ms_symmetric",
-                                                 "ms_tensor_core", "ms_tensor_core_symmetric"), ctx.fp32_autotune(R))),
+                                                 "ms_tensor_core", "ms_tensor_core_symmetric"), ctx.fp32_autotune(R)),
+                            **dict(zip(("interval_batched", "ms_interval_batched"), ctx.fp32_batched(R)))),
                         "fp32_kernel_variants": "0 = per-receiver, 1 = interval-bucketed, 2 = pair-symmetric (one warp per "
                                                 "receiver), 3 = pair-symmetric (two warps per receiver), 4 = tensor "
-                                                "cores (tcgen05 3xTF32), 5 = pair-symmetric tensor cores; RHS tile "
+                                                "cores (tcgen05 3xTF32), 5 = pair-symmetric tensor cores; interval_batched: "
+                                                "that operator runs instead of 4 or 5; RHS tile "
                                                 "autotuned"},
         "prep_s": round(prep_s, 2),
         "e2e": {"value": round(e2e_value, 6), "unit": UNIT, "h2d_bytes_per_step": int(2 * rhs.nbytes),

@@ -45,11 +45,11 @@ extern "C" {
  * right-preconditioned flexible GMRES with the learned preconditioner selected by
  * sg_precond_select; a correction solve that fails to reduce its residual is redone without it */
 #define SG_PRECOND 4
-/* double-float arithmetic: every sum of the coupling operator in two FP32 words (about 48
- * significant bits) on the FP32 pipe, with the FP64 table split into two FP32 words. As a matvec
- * precision it is an FP64-grade operator (it agrees with SG_FP64 to ~1e-13 relative); OR-ed into
- * sg_gmres_solve's precision with SG_FP32, the refinement's true residuals use it in place of the
- * FP64 operator. No counterpart in the reference. */
+/* FP64-grade operator: with the radial lookup, 32 particles or more and blocksize <= 48 the
+ * interval-batched operator that SG_FP64 uses; otherwise, and under stream capture, double-float
+ * arithmetic: every sum in two FP32 words (about 48 significant bits) on the FP32 pipe, with the FP64
+ * table split into two FP32 words (it agrees with SG_FP64 to ~1e-13 relative). OR-ed into
+ * sg_gmres_solve's precision with SG_FP32, the refinement's true residuals use it. No counterpart in the reference. */
 #define SG_DF64 8
 /* matvec precision: the coupling operator on the tensor cores (tcgen05.mma kind::tf32, each
  * operand split into a TF32 high part and a remainder, three products), for the radial lookup with
@@ -193,6 +193,13 @@ int sg_fp32_autotune(sg_context *ctx, int nrhs, int *variant, int *rhs_tile, dou
  * that RHS count; set_particles / set_lookup clear it. For tests and measurements of one kernel; no
  * counterpart in the reference. */
 int sg_fp32_set_kernel(sg_context *ctx, int nrhs, int variant, int rhs_tile);
+
+/* The interval-batched FP32 operator (pairs grouped by lookup interval, tensor cores) takes the place of
+ * variants 4 and 5 for an RHS count >= 16 when the autotuner finds it faster: *taken = 1 then, and *ms its
+ * time (-1 when not timed; either pointer may be NULL). take != 0 fixes it for that RHS count (32 particles
+ * or more, blocksize <= 30 or 33 to 48) until the next set_particles, set_lookup or sg_fp32_set_kernel. Under
+ * stream capture the variant that sg_fp32_autotune reports runs. No counterpart in the reference. */
+int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms);
 
 /* Emitters accumulated into one tensor-memory accumulator of the tensor-core operator before it is
  * added into the FP32 total (default 8). Fewer emitters bound the tensor core's accumulation error

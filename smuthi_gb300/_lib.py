@@ -28,6 +28,7 @@ EXPORTS = ("sg_last_error", "sg_version", "sg_create", "sg_destroy", "sg_set_par
            "sg_set_tmatrix", "sg_coupling_matvec", "sg_master_matvec", "sg_coupling_matvec_dev",
            "sg_master_matvec_dev", "sg_gmres_solve", "sg_gmres_solve_dev", "sg_true_residual", "sg_profile",
            "sg_kernel_timing", "sg_launch_count", "sg_measure_fma_peak", "sg_fp32_autotune", "sg_fp32_set_kernel",
+           "sg_fp32_batched",
            "sg_tc_set_window", "sg_coupling_matvec_linear_noalloc", "sg_precond_param_count", "sg_precond_add_graph",
            "sg_precond_select", "sg_precond_clear", "sg_precond_set_params", "sg_precond_get_params",
            "sg_precond_apply_dev", "sg_precond_train_step", "sg_precond_export_blocks", "sg_bessel_jac_table",
@@ -90,6 +91,7 @@ def _declare(L):
         "sg_fp32_autotune": [_P, _I, ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_D), ctypes.POINTER(_D),
                              ctypes.POINTER(_D), ctypes.POINTER(_D), ctypes.POINTER(_D)],
         "sg_fp32_set_kernel": [_P, _I, _I, _I],
+        "sg_fp32_batched": [_P, _I, _I, ctypes.POINTER(_I), ctypes.POINTER(_D)],
         "sg_tc_set_window": [_P, _I],
         "sg_plane_wave_swe": [_P, _I, _P, _I, _I, _P, _I, _P, _P, _P],
         "sg_coupling_matvec_linear_noalloc": [_I, _I, _P, _I, _P, _I, _D, _D, _P, _P, _P, _I, _P],
@@ -274,6 +276,13 @@ class Context:
         """Fix the FP32 operator for an RHS count (0 per-receiver, 1 bucketed, 2 pair-symmetric, 3 pair-symmetric
         with two warps per receiver, 4 tensor cores and 5 pair-symmetric tensor cores with rhs_tile = nrhs)."""
         check(lib().sg_fp32_set_kernel(self.h, int(nrhs), int(variant), int(rhs_tile)))
+
+    def fp32_batched(self, nrhs, take=False):
+        """(taken, ms): whether the interval-batched FP32 operator replaces the autotuned tensor-core variant for an
+        RHS count, and its time (-1 if not timed); ``take`` fixes it."""
+        on, ms = ctypes.c_int(), ctypes.c_double()
+        check(lib().sg_fp32_batched(self.h, int(nrhs), int(take), ctypes.byref(on), ctypes.byref(ms)))
+        return bool(on.value), ms.value
 
     def tc_set_window(self, emitters):
         """Emitters per tensor-memory accumulator of the tensor-core operator before it is drained."""

@@ -1,6 +1,7 @@
 // C ABI of the smuthi_gb300 library: context, uploads, validation and entry points.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <exception>
@@ -407,7 +408,7 @@ static int matvec_host(sg_context *ctx, const double *x, double *y, int nrhs, in
       throw sg::Error{SG_ERR_CUDA, "pair-symmetric FP32 operator: a bounded wait ran out"};
     if (precision == SG_FP32 && sg::tc_check_error(ctx, st))
       throw sg::Error{SG_ERR_CUDA, "tensor-core operator: a bounded wait ran out"};
-    if ((precision == SG_FP64 || precision == SG_DF64) && sg::ib_check_error(ctx, st))
+    if (sg::ib_check_error(ctx, st))
       throw sg::Error{SG_ERR_CUDA, "interval-batched operator: a bounded wait ran out"};
     return SG_OK;
   });
@@ -615,6 +616,33 @@ int sg_fp32_autotune(sg_context *ctx, int nrhs, int *variant, int *rhs_tile, dou
         return SG_OK;
       }
     *variant = -1;
+    return SG_OK;
+  });
+}
+
+int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms) {
+  return guarded([&]() -> int {
+    SG_REQUIRE(ctx, "null context");
+    SG_REQUIRE(!ctx->vol && ctx->kind >= 0, "a radial lookup must be set");
+    if (take) {
+      use_device(ctx);
+      ensure_pairs(ctx, ctx->stream);  // builds the FP32 operator data now (it would clear the choice later)
+      SG_REQUIRE(sg::ib32_supported(ctx, nrhs),
+                 "the interval-batched FP32 operator needs nrhs >= 16, 32 particles or more and blocksize <= 30 or 33 to 48");
+      sg_context::Tuned t{nrhs, 0, 1, -1.f, -1.f, 0, -1.f, -1.f, -1.f, -1.f, true};
+      auto &v = ctx->tuned;
+      v.erase(std::remove_if(v.begin(), v.end(), [&](const sg_context::Tuned &o) { return o.nrhs == nrhs; }), v.end());
+      v.push_back(t);
+    }
+    int on = 0;
+    double time = -1.0;
+    for (const auto &t : ctx->tuned)
+      if (t.nrhs == nrhs) {
+        on = t.batched;
+        time = t.ms_batched;
+      }
+    if (taken) *taken = on;
+    if (ms) *ms = time;
     return SG_OK;
   });
 }

@@ -1119,6 +1119,14 @@ static void launch_receiver_fp32(sg_context *c, const double2 *x, double2 *y, in
   c->launches += launch_coupling(L, true, ns, st);
 }
 
+// The interval-batched operators keep a workspace and order their calls by an event, which a captured
+// graph could not follow: under stream capture the other kernels run.
+static bool ib_usable(const sg_context *c, cudaStream_t st) {
+  if (!ib_supported(c)) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   // candidates: the per-receiver kernel with the three largest RHS tiles that divide R (16 only for
   // the FP32 path), and the bucketed kernel when its plan exists; each is warmed once (first
@@ -1175,6 +1183,12 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
   if (tc_supported(c, R)) ms_tc = time_it([&] { c->launches += launch_tc_matvec(c, x, y, R, master, st); });
   if (tcsym_supported(c, R))
     ms_tcs = time_it([&] { c->launches += launch_tcsym_matvec(c, x, y, R, master, st); });
+  // The interval-batched operator replaces the tensor-core ones, whose error is larger (2000 spheres, 16 right-hand
+  // sides: 4.5e-7 against 2.7e-7; 13.6 against 7.2 ms); where an FP32-pipe kernel wins, that one rounds better
+  // (100 spheres: 4.5e-8 against 5.6e-8) and stays.
+  float ms_batched = -1.f;
+  if (ib32_supported(c, R) && ib_usable(c, st))
+    ms_batched = time_it([&] { c->launches += launch_ibatch32(c, x, y, R, master, st); });
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   int v = 0;
@@ -1191,17 +1205,13 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
     v = 4;
     best = ms_tc;
   }
-  if (ms_tcs >= 0.f && ms_tcs < best) v = 5;
-  c->tuned.push_back({R, v, best_rt, best_rec, ms_bucket, sym_rt, ms_sym, ms_tc, ms_tcs});
+  if (ms_tcs >= 0.f && ms_tcs < best) {
+    v = 5;
+    best = ms_tcs;
+  }
+  c->tuned.push_back({R, v, best_rt, best_rec, ms_bucket, sym_rt, ms_sym, ms_tc, ms_tcs, ms_batched,
+                      v >= 4 && ms_batched >= 0.f && ms_batched < best});
   return v;
-}
-
-// The interval-batched operator keeps a workspace and orders its calls by an event, which a captured
-// graph could not follow: under stream capture the per-receiver kernel runs.
-static bool ib_usable(const sg_context *c, cudaStream_t st) {
-  if (!ib_supported(c)) return false;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }
 
 void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool master, bool fp32, cudaStream_t st) {
@@ -1212,6 +1222,7 @@ void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     SG_CUDA(cudaEventRecord(e0, st));
   }
   int variant = 0, rt = 0, sym_rt = 0;
+  bool batched = false;
   if (c->vol) {
     c->launches += launch_volume(c, x, y, R, master, fp32, st);
     variant = -1;
@@ -1222,15 +1233,19 @@ void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool maste
         variant = t.variant;
         rt = t.rt;
         sym_rt = t.sym_rt;
+        batched = t.batched;
       }
     if (variant < 0) {
       variant = autotune_fp32(c, x, y, R, master, st);
       rt = c->tuned.back().rt;
       sym_rt = c->tuned.back().sym_rt;
+      batched = c->tuned.back().batched;
     }
   }
   if (variant == 0 && !fp32 && ib_usable(c, st)) {
     c->launches += launch_ibatch(c, x, y, R, master, st);
+  } else if (batched && ib_usable(c, st)) {
+    c->launches += launch_ibatch32(c, x, y, R, master, st);
   } else if (variant == 5) {
     c->launches += launch_tcsym_matvec(c, x, y, R, master, st);
   } else if (variant == 4) {

@@ -58,6 +58,7 @@
 #include <vector>
 
 #include "sg_epilogue.h"
+#include "sg_ibatch.h"
 #include "sg_internal.h"
 #include "sg_tcgen05.h"
 
@@ -176,8 +177,6 @@ struct IbArgs {
   int nb, bs, mmax, rt, per, t0, t1;  // rt right-hand sides; per = pairs per tile; tiles [t0, t1)
   int *err;
 };
-
-__device__ __forceinline__ int ib_field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
 
 // v 2^(53 + UP - scale) truncated, for an exponent of v that lies `below` under the scale's
 template <int UP>
@@ -835,24 +834,7 @@ __global__ void __launch_bounds__(256) ib_operand_kernel(const double2 *coef, co
   __shared__ int eb[KP], ea[KP];
   const int tid = threadIdx.x, b = blockIdx.x, bs2 = bs * bs;
   const double2 *C = coef + (size_t)bk[b] * NC * bs2;
-  if (tid < KP) {
-    eb[tid] = ea[tid] = -(1 << 20);
-  }
-  __syncthreads();
-  for (int e = tid; e < NC * bs2; e += blockDim.x) {
-    const int f = max(ib_field(C[e].x), ib_field(C[e].y));
-    if (f) atomicMax(&eb[(e % bs2) / bs], f - 1022);
-  }
-  __syncthreads();
-  if (tid < KP && eb[tid] == -(1 << 20)) eb[tid] = 0;
-  __syncthreads();
-  for (int e = tid; e < NC * bs2; e += blockDim.x) {
-    const int f = max(ib_field(C[e].x), ib_field(C[e].y));
-    if (f) atomicMax(&ea[e % bs], f - 1022 - eb[(e % bs2) / bs]);
-  }
-  __syncthreads();
-  if (tid < KP && ea[tid] == -(1 << 20)) ea[tid] = 0;
-  __syncthreads();
+  ib_exponents<NC, KP>(C, bs, eb, ea);
   if (tid < KP) {
     exps[(size_t)b * 2 * KP + tid] = eb[tid];
     exps[(size_t)b * 2 * KP + KP + tid] = ea[tid];
@@ -921,8 +903,9 @@ bool ib_supported(const sg_context *c) {
   return true;
 }
 
-static void ib_build_plan(sg_context *c, cudaStream_t st) {
+void ib_plan(sg_context *c, cudaStream_t st) {
   auto &P = c->ib;
+  if (P.ready) return;
   const int n = c->n, n_int = c->n_int;
   const size_t np = (size_t)n * n;
   DevBuf<unsigned> keys, keys2, vals, vals2;
@@ -958,34 +941,49 @@ static void ib_build_plan(sg_context *c, cudaStream_t st) {
       P.h_boff.push_back(P.h_boff.back() + cnt[k]);
     }
   P.nb = (int)bk.size();
-  DevBuf<int> dbk;
-  dbk.reserve(P.nb);
+  P.bk.reserve(P.nb);
   P.boff.reserve(P.nb + 1);
-  P.exps.reserve((size_t)P.nb * 2 * ib_kp(c));
-  ib_dispatch(c, [&](auto nc, auto kp) { P.B.reserve((size_t)P.nb * IbShape<decltype(nc)::value, decltype(kp)::value>::BBYTES); });
-  SG_CUDA(cudaMemcpyAsync(dbk.ptr, bk.data(), P.nb * sizeof(int), cudaMemcpyHostToDevice, st));
+  SG_CUDA(cudaMemcpyAsync(P.bk.ptr, bk.data(), P.nb * sizeof(int), cudaMemcpyHostToDevice, st));
   SG_CUDA(cudaMemcpyAsync(P.boff.ptr, P.h_boff.data(), (P.nb + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-  ib_dispatch(c, [&](auto nc, auto kp) {
-    ib_operand_kernel<decltype(nc)::value, decltype(kp)::value>
-        <<<P.nb, 256, 0, st>>>(c->coef64.ptr, dbk.ptr, c->bs, P.B.ptr, P.exps.ptr);
-  });
-  SG_CUDA(cudaGetLastError());
   P.err.reserve(1);
   SG_CUDA(cudaMemsetAsync(P.err.ptr, 0, sizeof(int), st));
   SG_CUDA(cudaStreamSynchronize(st));  // the temporaries are released on return
   P.tiles.clear();
-  c->launches += 3;
+  c->launches += 2;
   P.ready = true;
+  P.digits_ready = P.halves_ready = false;
 }
+
+static void ib_digit_operands(sg_context *c, cudaStream_t st) {
+  auto &P = c->ib;
+  if (P.digits_ready) return;
+  P.exps.reserve((size_t)P.nb * 2 * ib_kp(c));
+  ib_dispatch(c, [&](auto nc, auto kp) {
+    constexpr int NC = decltype(nc)::value, KP = decltype(kp)::value;
+    P.B.reserve((size_t)P.nb * IbShape<NC, KP>::BBYTES);
+    ib_operand_kernel<NC, KP><<<P.nb, 256, 0, st>>>(c->coef64.ptr, P.bk.ptr, c->bs, P.B.ptr, P.exps.ptr);
+  });
+  SG_CUDA(cudaGetLastError());
+  c->launches += 1;
+  P.digits_ready = true;
+}
+
+void ib_enter(sg_context *c, cudaStream_t st) {
+  auto &P = c->ib;
+  if (!P.done) SG_CUDA(cudaEventCreateWithFlags(&P.done, cudaEventDisableTiming));
+  else SG_CUDA(cudaStreamWaitEvent(st, P.done, 0));
+}
+
+void ib_leave(sg_context *c, cudaStream_t st) { SG_CUDA(cudaEventRecord(c->ib.done, st)); }
 
 // The tiles for rt right-hand sides: first tile of every interval. Where 64 columns make hardly more tiles than 128,
 // most are not half full and two sets of warps that overlap their tiles are faster: 100 spheres (1.00 times the tiles)
 // 51 against 63 us, 220 (1.27) 108 against 117, 200 with the cubic lookup (1.25) 144 against 141, 301 (1.54) 165
 // against 161, 1000 (1.8) 1140 against 1056.
-static sg_context::IbTiles &ib_tiles(sg_context *c, int rt, cudaStream_t st) {
+sg_context::IbTiles &ib_tiles(sg_context *c, int rt, int sets, cudaStream_t st) {
   auto &P = c->ib;
   for (auto &t : P.tiles)
-    if (t->rt == rt) return *t;
+    if (t->rt == rt && t->asked == sets) return *t;
   auto t = std::make_unique<sg_context::IbTiles>();
   auto count = [&](int per) {
     long long n = 0;
@@ -993,7 +991,8 @@ static sg_context::IbTiles &ib_tiles(sg_context *c, int rt, cudaStream_t st) {
     return n;
   };
   t->rt = rt;
-  t->sets = 3 * count(kIbCols / 2 / rt) <= 4 * count(kIbCols / rt) ? 2 : 1;
+  t->asked = sets;
+  t->sets = sets ? sets : 3 * count(kIbCols / 2 / rt) <= 4 * count(kIbCols / rt) ? 2 : 1;
   const int per = t->per = kIbCols / t->sets / rt;
   t->h_toff.assign(1, 0);
   for (int b = 0; b < P.nb; ++b)
@@ -1018,10 +1017,9 @@ static void ib_launch(const IbArgs &a, cudaStream_t st) {
 // y = M x or W x in FP64; returns the number of kernels launched
 int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   auto &P = c->ib;
-  if (!P.ready) ib_build_plan(c, st);
-  // the workspace is shared by all calls on this context: order them across streams
-  if (!P.done) SG_CUDA(cudaEventCreateWithFlags(&P.done, cudaEventDisableTiming));
-  else SG_CUDA(cudaStreamWaitEvent(st, P.done, 0));
+  ib_enter(c, st);
+  ib_plan(c, st);
+  ib_digit_operands(c, st);
   const int bs = c->bs;
   CouplingLaunch L{};
   L.n = c->n;
@@ -1042,7 +1040,7 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
   const int most = (int)std::min<size_t>(16, std::max<size_t>(1, 4 * kIbWorkspace / ((size_t)c->n * c->n * bs * sizeof(double2))));
   for (int r0 = 0, rt; r0 < R; r0 += rt) {
     rt = std::min(most, R - r0);
-    auto &tl = ib_tiles(c, rt, st);
+    auto &tl = ib_tiles(c, rt, 0, st);
     const int per = tl.per;
     const size_t pair_bytes = (size_t)rt * bs * sizeof(double2);
     const int ntiles = tl.h_toff.back();
@@ -1103,7 +1101,7 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
       launched += 2;
     }
   }
-  SG_CUDA(cudaEventRecord(P.done, st));
+  ib_leave(c, st);
   return launched;
 }
 

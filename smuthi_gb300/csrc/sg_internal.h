@@ -117,7 +117,16 @@ bool tc_check_error(sg_context *c, cudaStream_t st);  // reads and clears the ti
 bool tcsym_supported(const sg_context *c, int R);
 int launch_tcsym_matvec(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 // FP32 W x in c->sym_yacc -> FP64 W x or x - T (W x) (diagonal or dense T); one launch
-void launch_fp32_epilogue(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
+// top: largest exponent fields of x per right-hand side, by which x was scaled (null: not); err: flag of a wait that ran
+// out (null: none), which makes the result NaN
+void launch_fp32_epilogue(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st,
+                          const int *top = nullptr, const int *err = nullptr);
+#ifdef __CUDACC__
+// power of two that brings values with exponent field up to `top` below 1 (as far as it is a normal number)
+__device__ __forceinline__ double fp32_scale(int top) {
+  return __hiloint2double(max(1, min(2045, 2045 - top)) << 20, 0);
+}
+#endif
 // y = M x or W x in double-float arithmetic (FP64-grade; builds the df64 coefficients on first use)
 void apply_padded_df64(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 // padded-vector operator application and solver (sg_gmres.cu)
@@ -127,6 +136,8 @@ void solve_padded(sg_context *c, const double2 *b, double2 *x, int R, double rto
 void residual_norms(sg_context *c, const double2 *b, const double2 *x, int R, double *rel, cudaStream_t st);
 // FP64 operator batched by lookup interval on the tensor cores (sg_ibatch.cu)
 bool ib_supported(const sg_context *c);
+bool ib32_supported(const sg_context *c, int R);
+int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 bool ib_check_error(sg_context *c, cudaStream_t st);  // reads and clears the timeout flag (synchronises)
 struct IbRec {  // one ordered pair: fraction within its interval, direction, receiver i and emitter j
@@ -281,6 +292,8 @@ struct sg_context {
     float ms_sym;       // best pair-symmetric tile and layout (< 0: not a candidate)
     float ms_tc;        // tensor-core operator (< 0: not a candidate)
     float ms_tcs;       // pair-symmetric tensor-core operator (< 0: not a candidate)
+    float ms_batched = -1.f;  // interval-batched FP32 operator (< 0: not a candidate)
+    bool batched = false;     // it replaces the variant
   };
   std::vector<Tuned> tuned;
   std::vector<std::pair<int, int>> tuned_df;  // double-float kernel: (nrhs, RHS tile)
@@ -299,18 +312,20 @@ struct sg_context {
   // interval-batched FP64 operator (sg_ibatch.cu): ordered pairs sorted by lookup interval, the
   // intervals' digit operands, the pairs' contributions V of one chunk
   struct IbTiles {
-    int rt = 0, sets = 1, per = 0;  // right-hand sides; sets of warps; pairs per tile
+    int rt = 0, asked = 0, sets = 1, per = 0;  // right-hand sides; sets of warps, asked for (0: none) and taken; pairs per tile
     std::vector<int> h_toff;
     sg::DevBuf<int> toff;
   };
   struct Ib {
-    bool ready = false;
+    bool ready = false, digits_ready = false, halves_ready = false;
     int nb = 0;
     std::vector<int> h_boff;
     sg::DevBuf<sg::IbRec> rec;
     sg::DevBuf<unsigned> slot;
-    sg::DevBuf<int> boff, exps, err;
-    sg::DevBuf<unsigned char> B;
+    sg::DevBuf<int> bk, boff, exps, err;
+    sg::DevBuf<unsigned char> B, H;  // operands: digits (FP64), FP16 halves (FP32)
+    sg::DevBuf<float2> xh;           // FP32 copy of x for the FP32 form
+    sg::DevBuf<int> top;             // its scales
     sg::DevBuf<double2> V, acc;
     sg::DevBuf<int4> xw;  // words of x and their exponents
     sg::DevBuf<int> xe;

@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kSymThreads, SPLIT) sym_kernel(const SymLaunch
 
 // y = W x (FP64 from the FP32 sums) or x - T W x; one thread per padded element
 __global__ void sym_epilogue_kernel(const float2 *yacc, const double2 *x, double2 *y, int n, int bs, int R, int master,
-                                    const double2 *t, const int *ptype, int t_diag) {
+                                    const double2 *t, const int *ptype, int t_diag, const int *top, const int *err) {
   const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t total = (size_t)n * bs * R;
   if (e >= total) return;
@@ -503,6 +503,9 @@ __global__ void sym_epilogue_kernel(const float2 *yacc, const double2 *x, double
   const int i = (int)(ib / bs);
   const float2 w = yacc[e];
   double2 v = make_double2((double)w.x, (double)w.y);
+  // x was scaled by a power of two per right-hand side (fp32_scale)
+  const double u = err && *err ? __longlong_as_double(0x7FF8000000000000ll) : top ? 1.0 / fp32_scale(top[r]) : 1.0;
+  v = make_double2(v.x * u, v.y * u);
   if (master) {
     const int ty = ptype[i];
     double2 tw;
@@ -519,7 +522,7 @@ __global__ void sym_epilogue_kernel(const float2 *yacc, const double2 *x, double
         ar = fma(tt.x, (double)a.x, fma(-tt.y, (double)a.y, ar));
         ai = fma(tt.x, (double)a.y, fma(tt.y, (double)a.x, ai));
       }
-      tw = make_double2(ar, ai);
+      tw = make_double2(ar * u, ai * u);
     }
     const double2 xv = x[e];
     v = make_double2(xv.x - tw.x, xv.y - tw.y);
@@ -644,11 +647,12 @@ int launch_sym_matvec(sg_context *c, const double2 *x, double2 *y, int R, bool m
   return 3;  // conversion, coupling, epilogue (the memset is not a kernel of this library)
 }
 
-void launch_fp32_epilogue(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
+void launch_fp32_epilogue(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st, const int *top,
+                          const int *err) {
   const size_t len = (size_t)c->n * c->bs * R;
   sym_epilogue_kernel<<<(unsigned)((len + 255) / 256), 256, 0, st>>>(c->sym_yacc.ptr, x, y, c->n, c->bs, R,
                                                                      master ? 1 : 0, c->tmat.ptr, c->ptype.ptr,
-                                                                     c->t_diag);
+                                                                     c->t_diag, top, err);
   SG_CUDA(cudaGetLastError());
 }
 
