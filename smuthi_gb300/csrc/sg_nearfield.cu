@@ -17,7 +17,7 @@
 // shared memory; kappa ranges of a larger split go to further blocks and a reduce kernel sums them
 // in a fixed order. FP64 throughout, and the FP64 pipe bounds it: 31 operations per node with the
 // table-driven sine (sg_sincos.h) against about 60 with sincos(); 4096 points on 279 x 721 nodes
-// 86.4 ms before, now 66.
+// 86.4 ms before, now 67.
 #include <cuda_runtime.h>
 #include <math.h>
 
