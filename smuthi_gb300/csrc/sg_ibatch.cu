@@ -74,8 +74,8 @@ static constexpr int kIbRows = 64;   // (n1, power of t) per pass: N = 128 accum
 // 1.5 2^23: added to an integer below 2^22 it leaves that in the mantissa
 static constexpr float kIbMagic = 12582912.f;
 static constexpr unsigned kIbMagicBits = 0x4B400000u;
-// largest t in units of 2^-62 whose high word fits (t < 1 up to its last places)
-static constexpr long long kIbBelowOne = (1ll << 62) - (1ll << 30) - 1;
+// first t in units of 2^-62 whose high word would not fit beside a signed low one
+static constexpr long long kIbNearOne = (1ll << 62) - (1ll << 30);
 
 // KP: padded blocksize, 32 or 48
 template <int KP>
@@ -218,6 +218,12 @@ __device__ __forceinline__ IbWords ib_split(long long v) {
 }
 __device__ __forceinline__ IbWords ib_split_signed(long long v) {
   return {(int)((v + 0x40000000ll) >> 31), (int)((unsigned)v << 1) >> 1};
+}
+// t, in units of 2^-62. The last 2^-32 below one keep an unsigned low word: with |h|, l < 2^31 the middle products of
+// ib_mul still stay within 2^63, and the bias of what it drops, below one unit, is that of the few pairs that close to
+// the end of an interval.
+__device__ __forceinline__ IbWords ib_split_fraction(long long v) {
+  return v >= kIbNearOne ? ib_split(v) : ib_split_signed(v);
 }
 __device__ __forceinline__ long long ib_mad(int a, int b, long long c) { return (long long)a * b + c; }
 // a b / 2^62 + c
@@ -442,9 +448,7 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
         lb += o;
         len = min(step, len - o);
       }
-      auto words = [](double v, int up) {  // v in units of 2^-up, |v| <= 1
-        return ib_split_signed(min(ib_fixed<10>(v, 1023 + 62 - up - ib_field(v)), kIbBelowOne));
-      };
+      auto fixed = [](double v, int up) { return ib_fixed<10>(v, 1023 + 62 - up - ib_field(v)); };  // |v| <= 1 in units of 2^-up
       for (int T = 0; T < NT && good; ++T) {
         while (T0 + T >= a.toff[lb + 1]) ++lb;
         const int h = T % SETS, n = T / SETS;
@@ -464,13 +468,13 @@ __global__ void __launch_bounds__(kIbThreads, 1) ib_kernel(const IbArgs a) {
           }
           const int c = g * 32 + lane;
           const IbRec rc = a.rec[p0 + min(c, ncol - 1) / a.rt];  // columns that are not there repeat the last
-          const IbWords tw = words(rc.t, 62);
+          const IbWords tw = ib_split_fraction(fixed(rc.t, 62));
           t.t[c] = make_int2(tw.h, tw.l);
           t.xoff[c] = rc.j * a.rt + min(c, ncol - 1) % a.rt;
           t.ph[0][c] = make_int4(1 << 30, 0, 0, 0);
           double pr = rc.c, pi = rc.s;
           for (int m = 1; m <= a.mmax; ++m) {
-            const IbWords cw = words(pr, 61), sw = words(pi, 61);
+            const IbWords cw = ib_split_signed(fixed(pr, 61)), sw = ib_split_signed(fixed(pi, 61));
             t.ph[m][c] = make_int4(cw.h, cw.l, sw.h, sw.l);
             const double nr = pr * rc.c - pi * rc.s;
             pi = pr * rc.s + pi * rc.c;

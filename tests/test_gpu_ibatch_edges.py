@@ -1,0 +1,48 @@
+"""The interval-batched operators (csrc/sg_ibatch.cu, sg_ibatch32.cu) at the edges of their number ranges, against a
+direct FP64 evaluation.
+"""
+import numpy as np
+import pytest
+
+from smuthi_gb300 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _line(n, step, res, bs, seed, scale=1.0):
+    """Particles on a line, `step` apart, and a smooth random table on a grid from zero."""
+    rng = np.random.default_rng(seed)
+    xy = np.stack([step * np.arange(n), np.zeros(n)], 1)
+    m = rng.integers(-3, 4, bs)
+    rho = res * np.arange(int(np.ceil(step * n / res)) + 4)
+    table = np.exp(1j * rho[:, None, None] * rng.uniform(0.1, 1.0, (bs, bs))) * rng.standard_normal((bs, bs)) * scale
+    x = rng.standard_normal((n, bs)) + 1j * rng.standard_normal((n, bs))
+    return xy, m, table, x
+
+
+def _linear(xy, m, table, res, x):
+    d = xy[:, None] - xy[None]
+    s = np.sqrt((d ** 2).sum(-1)) / res
+    k = np.floor(s).astype(int)
+    t = (s - k)[..., None, None]
+    w = table[k] + t * (table[k + 1] - table[k])
+    w = w * np.exp(1j * (m[None, :] - m[:, None]) * np.arctan2(d[..., 1], d[..., 0])[..., None, None])
+    return np.einsum("ijab,jb->ia", w, x), s - k
+
+
+def _upload(ctx, xy, m, table, res, bs):
+    ctx.set_particles(xy, *np.divmod(np.arange(len(xy) * bs), bs), bs, m)
+    ctx.set_lookup("linear", table, 0.0, res)
+
+
+@pytest.mark.parametrize("bs", [30, 48])
+def test_fraction_just_below_one(bs, gpu_context):
+    """Distances that fall a rounding error short of a grid point: t within 2^-32 of one. Bound as in
+    test_gpu_ibatch.py: n * blocksize <= 3100 products, each side rounds at 2^-53 of its partial sums."""
+    n, res = 64, 0.1
+    xy, m, table, x = _line(n, 0.3, res, bs, 1)
+    ref, t = _linear(xy, m, table, res, x)
+    assert (t > 1 - 2.0 ** -32).sum() > 1000
+    _upload(gpu_context, xy, m, table, res, bs)
+    y = gpu_context.coupling_matvec(x.reshape(-1), _lib.SG_FP64).reshape(n, bs)
+    assert np.linalg.norm(y - ref) <= 1e-13 * np.linalg.norm(ref)
