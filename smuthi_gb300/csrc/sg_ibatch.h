@@ -11,7 +11,8 @@ namespace sg {
 __device__ __forceinline__ int ib_field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
 
 // Scales of the NC coefficient matrices C [NC][n2][n1] of an interval, by a whole block: |Re|, |Im| of an element are
-// below 2^(ea[n1] + eb[n2]). Column exponents first, then row exponents of what they leave.
+// below 2^(ea[n1] + eb[n2]). Column exponents first, then row exponents of what they leave. A column of zeros keeps an
+// exponent below all others: nothing that x holds for it may take part in the scale of the products.
 template <int NC, int KP>
 __device__ __forceinline__ void ib_exponents(const double2 *C, int bs, int *eb, int *ea) {
   const int tid = threadIdx.x, bs2 = bs * bs;
@@ -21,8 +22,6 @@ __device__ __forceinline__ void ib_exponents(const double2 *C, int bs, int *eb, 
     const int f = max(ib_field(C[e].x), ib_field(C[e].y));
     if (f) atomicMax(&eb[(e % bs2) / bs], f - 1022);
   }
-  __syncthreads();
-  if (tid < KP && eb[tid] == -(1 << 20)) eb[tid] = 0;
   __syncthreads();
   for (int e = tid; e < NC * bs2; e += blockDim.x) {
     const int f = max(ib_field(C[e].x), ib_field(C[e].y));

@@ -46,3 +46,24 @@ def test_fraction_just_below_one(bs, gpu_context):
     _upload(gpu_context, xy, m, table, res, bs)
     y = gpu_context.coupling_matvec(x.reshape(-1), _lib.SG_FP64).reshape(n, bs)
     assert np.linalg.norm(y - ref) <= 1e-13 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("precision,R,tol", [(_lib.SG_FP64, 1, 1e-13), (_lib.SG_FP32, 16, 4e-6)])
+def test_zero_column_of_a_small_table(precision, R, tol, gpu_context):
+    """A table far below one with a multipole that couples to nothing: its part of x, which is not small, must not set
+    the scale of the products. Bounds as in test_gpu_ibatch.py and test_gpu_ibatch32.py."""
+    n, bs, res = 40, 30, 1.0
+    xy, m, table, x = _line(n, 7.3, res, bs, 2, 1e-9)
+    table[:, :, 3] = 0
+    ref, _ = _linear(xy, m, table, res, x)
+    _upload(gpu_context, xy, m, table, res, bs)
+    if precision == _lib.SG_FP32:
+        assert gpu_context.fp32_batched(R, take=True)[0]
+    y = gpu_context.coupling_matvec(np.repeat(x.reshape(-1, 1), R, axis=1), precision)
+    for r in range(R):
+        assert np.linalg.norm(y[:, r] - ref.reshape(-1)) <= tol * np.linalg.norm(ref)
+    table[:] = 0
+    _upload(gpu_context, xy, m, table, res, bs)
+    if precision == _lib.SG_FP32:
+        assert gpu_context.fp32_batched(R, take=True)[0]
+    assert not gpu_context.coupling_matvec(np.repeat(x.reshape(-1, 1), R, axis=1), precision).any()
