@@ -712,13 +712,21 @@ __global__ void __launch_bounds__(256) ib_words_kernel(const double2 *x, int n, 
   int4 w = make_int4(0, 0, 0, 0);
   int f = 0;
   if (n2 < bs) {
-    const double2 v = x[(j * bs + n2) * R + r0 + r];
+    double2 v = x[(j * bs + n2) * R + r0 + r];
     f = max(ib_field(v.x), ib_field(v.y));
+    const bool tiny = f < 64;  // a part of it may be subnormal: lifted by 2^128, its exponent below zero
+    if (tiny) {
+      v = make_double2(v.x * 0x1p128, v.y * 0x1p128);
+      f = max(ib_field(v.x), ib_field(v.y));
+    }
     const IbWords re = ib_split(ib_fixed<9>(v.x, f - ib_field(v.x))), im = ib_split(ib_fixed<9>(v.y, f - ib_field(v.y)));
     w = make_int4(re.h, re.l, im.h, im.l);
+    f = f == 0 ? -(1 << 24) : f == 0x7FF ? 1 << 21 : tiny ? f - 128 : f;  // zero; Inf or NaN
+  } else {
+    f = -(1 << 24);
   }
   xw[q] = w;
-  xe[q] = f == 0 ? -(1 << 24) : f == 0x7FF ? 1 << 21 : f;  // zero; Inf or NaN
+  xe[q] = f;
 }
 
 // ------------------------------------------------------------------ sum over the emitters

@@ -67,3 +67,19 @@ def test_zero_column_of_a_small_table(precision, R, tol, gpu_context):
     if precision == _lib.SG_FP32:
         assert gpu_context.fp32_batched(R, take=True)[0]
     assert not gpu_context.coupling_matvec(np.repeat(x.reshape(-1, 1), R, axis=1), precision).any()
+
+
+@pytest.mark.parametrize("e", [-1000, -1015, -1030, -1060])
+def test_subnormal_vectors(e, gpu_context):
+    """x in and below the last binades of FP64: the result scales with it, up to the rounding of each pair's
+    contribution and of their sum to a multiple of 2^-1074 (and FP64's own)."""
+    n, bs, res = 40, 30, 1.0
+    xy, m, table, x = _line(n, 7.3, res, bs, 3)
+    x = np.round(np.stack([x.real, x.imag], -1) * 2.0 ** 10) / 2.0 ** 10  # exact multiples of 2^(e - 10)
+    _upload(gpu_context, xy, m, table, res, bs)
+    big = gpu_context.coupling_matvec((x[..., 0] + 1j * x[..., 1]).reshape(-1), _lib.SG_FP64)
+    x = np.ldexp(x, e)
+    y = gpu_context.coupling_matvec((x[..., 0] + 1j * x[..., 1]).reshape(-1), _lib.SG_FP64)
+    for got, want in ((y.real, big.real), (y.imag, big.imag)):
+        got = np.ldexp(np.ldexp(got, 600), -e - 600)
+        assert (np.abs(got - want) <= 1e-13 * np.abs(big).max() + np.ldexp(n, -1074 - e)).all()
