@@ -128,8 +128,8 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
                : "memory");
 }
 
-// 2^e, zero below the normal range
-__device__ __forceinline__ float ih_pow2(int e) { return e < -126 ? 0.f : __int_as_float((min(e, 127) + 127) << 23); }
+// 2^e, zero below the normal range and Inf above it
+__device__ __forceinline__ float ih_pow2(int e) { return e < -126 ? 0.f : __int_as_float((min(e, 128) + 127) << 23); }
 
 // two floats as packed FP16 parts
 __device__ __forceinline__ void ih_split(float a, float b, uint32_t &hi, uint32_t &lo) {

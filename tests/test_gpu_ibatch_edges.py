@@ -83,3 +83,15 @@ def test_subnormal_vectors(e, gpu_context):
     for got, want in ((y.real, big.real), (y.imag, big.imag)):
         got = np.ldexp(np.ldexp(got, 600), -e - 600)
         assert (np.abs(got - want) <= 1e-13 * np.abs(big).max() + np.ldexp(n, -1074 - e)).all()
+
+
+def test_table_beyond_fp32(gpu_context):
+    """Coefficients too large for FP32 give no finite numbers, as with the other FP32 operators."""
+    n, bs, res, R = 40, 30, 1.0, 16
+    xy, m, table, x = _line(n, 7.3, res, bs, 2, 1e50)
+    _upload(gpu_context, xy, m, table, res, bs)
+    x = np.repeat(x.reshape(-1, 1), R, axis=1)
+    assert gpu_context.fp32_batched(R, take=True)[0]
+    assert not np.isfinite(gpu_context.coupling_matvec(x, _lib.SG_FP32)).any()
+    gpu_context.fp32_set_kernel(R, 0, 8)
+    assert not np.isfinite(gpu_context.coupling_matvec(x, _lib.SG_FP32)).any()
