@@ -11,8 +11,9 @@
 // interval. Even and odd tiles belong to two sets of eight warps that run half a tile apart: a set rotates x_j, splits
 // it and writes the A operand (a lane per column, K = 2 blocksize: Im and Re) to tensor memory, waits for the products
 // (one accumulator of 64 Re and 64 Im columns per set and pass), combines the powers of t, rotates back and adds the
-// contribution to y_i with vector atomics. One thread issues the MMAs against the interval's B operand in shared
-// memory (rows -Im C, Re C, Im C as in the FP64 form); three warps prepare the tiles' t and phases ahead.
+// contribution to y_i with vector atomics (in any order: the last bits of a product differ from run to run; with many
+// particles in chunks of tiles, kIhTerms). One thread issues the MMAs against the interval's B operand in shared memory
+// (rows -Im C, Re C, Im C as in the FP64 form); three warps prepare the tiles' t and phases ahead.
 //
 // Every wait is bounded; a wait that runs out sets the error flag, and all roles leave.
 //
@@ -92,7 +93,7 @@ struct IhArgs {
   const float2 *x;  // [N][KP][rt]
   const int *mofn;
   float2 *y;        // [N][bs][R]
-  int nb, bs, mmax, R, r0, rt, per, ntiles;
+  int nb, bs, mmax, R, r0, rt, per, t0, t1;  // tiles [t0, t1)
   int *err;
 };
 
@@ -150,8 +151,9 @@ __global__ void __launch_bounds__(kIhThreads, 1) ih_kernel(const IhArgs a) {
   Sm &S = *reinterpret_cast<Sm *>(Bs + NB * Sh::BBYTES);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bs = a.bs;
-  const int T0 = (int)((long long)a.ntiles * blockIdx.x / gridDim.x);
-  const int NT = (int)((long long)a.ntiles * (blockIdx.x + 1) / gridDim.x) - T0;  // this CTA's tiles
+  const int ntiles = a.t1 - a.t0;
+  const int T0 = a.t0 + (int)((long long)ntiles * blockIdx.x / gridDim.x);
+  const int NT = a.t0 + (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x) - T0;  // this CTA's tiles
   const int passes = (bs + PN - 1) / PN;
 
   if (tid < KP) S.mrow[tid] = ((tid < bs ? a.mofn[tid] : 0) + Sh::MAXM) * kIhCols;
@@ -482,6 +484,22 @@ __global__ void __launch_bounds__(256) ih_copy_kernel(const double2 *x, int n, i
   o[q] = v;
 }
 
+// FP32 sums of a chunk of pairs, columns r0 .. r0 + rt of R: into the FP64 totals, and zero again; the last chunk
+// leaves the total in their place
+__global__ void __launch_bounds__(256) ih_fold_kernel(float2 *y, double2 *total, size_t rows, int R, int r0, int rt, int first, int last) {
+  const size_t q = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (q >= rows * rt) return;
+  const size_t e = q / rt * R + r0 + q % rt;
+  const float2 v = y[e];
+  double2 s = make_double2(v.x, v.y);
+  if (!first) {
+    const double2 o = total[e];
+    s = make_double2(s.x + o.x, s.y + o.y);
+  }
+  if (!last) total[e] = s;
+  y[e] = last ? make_float2((float)s.x, (float)s.y) : make_float2(0.f, 0.f);
+}
+
 // B operand and exponents of one non-empty interval per block
 template <int NC, int KP>
 __global__ void __launch_bounds__(256) ih_operand_kernel(const double2 *coef, const int *bk, int bs, unsigned char *B, int *exps) {
@@ -515,6 +533,13 @@ __global__ void __launch_bounds__(256) ih_operand_kernel(const double2 *coef, co
 }
 
 static constexpr size_t kIhMaxOperands = (size_t)16 << 30;
+
+// Pairs of a receiver that are added one after the other in FP32, on average: n such roundings grow with sqrt(n) or
+// faster, so that larger systems run in chunks of tiles whose sums are added in FP64. Without chunks the error of a
+// film's product was 9.1e-7 with 2000 spheres, 1.3e-6 with 4001 and 2.1e-6 with 10000, where the pair-symmetric
+// tensor-core kernel has 1.7e-6 throughout; with chunks 6.4e-7, 6.4e-7 and 6.3e-7, in 6.03 ms instead of 6.01, 23.9
+// instead of 23.8 and 149.4 instead of 148.8.
+static constexpr int kIhTerms = 1024;
 
 template <class F>
 static void ih_dispatch(const sg_context *c, F &&f) {
@@ -584,22 +609,36 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
     auto &tl = ib_tiles(c, a.rt, 1, st);
     a.toff = tl.toff.ptr;
     a.per = tl.per;
-    a.ntiles = tl.h_toff.back();
+    const int ntiles = tl.h_toff.back(), chunks = (c->n + kIhTerms - 1) / kIhTerms;
+    if (chunks > 1) P.acc.reserve(len);
     const size_t elems = (size_t)c->n * kp * a.rt;
     P.xh.reserve(elems);
     ih_copy_kernel<<<(unsigned)((elems + 255) / 256), 256, 0, st>>>(x, c->n, bs, kp, R, r0, a.rt, P.top.ptr, P.xh.ptr);
     SG_CUDA(cudaGetLastError());
+    ++launched;
     a.x = P.xh.ptr;
-    ih_dispatch(c, [&](auto nc, auto kpc) {
-      constexpr int NC = decltype(nc)::value, KP = decltype(kpc)::value;
-      static bool attr_done[64] = {};
-      constexpr int smem = (int)ih_smem<NC, KP>();
-      if (first_on_device(attr_done))
-        SG_CUDA(cudaFuncSetAttribute(ih_kernel<NC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      ih_kernel<NC, KP><<<std::min(sm_count(), a.ntiles), kIhThreads, smem, st>>>(a);
-    });
-    SG_CUDA(cudaGetLastError());
-    launched += 2;
+    for (int q = 0; q < chunks; ++q) {
+      a.t0 = (int)((long long)ntiles * q / chunks);
+      a.t1 = (int)((long long)ntiles * (q + 1) / chunks);
+      if (a.t0 < a.t1) {
+        ih_dispatch(c, [&](auto nc, auto kpc) {
+          constexpr int NC = decltype(nc)::value, KP = decltype(kpc)::value;
+          static bool attr_done[64] = {};
+          constexpr int smem = (int)ih_smem<NC, KP>();
+          if (first_on_device(attr_done))
+            SG_CUDA(cudaFuncSetAttribute(ih_kernel<NC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+          ih_kernel<NC, KP><<<std::min(sm_count(), a.t1 - a.t0), kIhThreads, smem, st>>>(a);
+        });
+        SG_CUDA(cudaGetLastError());
+        ++launched;
+      }
+      if (chunks > 1) {
+        ih_fold_kernel<<<(unsigned)((rows * a.rt + 255) / 256), 256, 0, st>>>(a.y, P.acc.ptr, rows, R, r0, a.rt, q == 0,
+                                                                              q == chunks - 1);
+        SG_CUDA(cudaGetLastError());
+        ++launched;
+      }
+    }
   }
   launch_fp32_epilogue(c, x, y, R, master, st, P.top.ptr, P.err.ptr);
   ib_leave(c, st);

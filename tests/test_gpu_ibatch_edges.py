@@ -95,3 +95,27 @@ def test_table_beyond_fp32(gpu_context):
     assert not np.isfinite(gpu_context.coupling_matvec(x, _lib.SG_FP32)).any()
     gpu_context.fp32_set_kernel(R, 0, 8)
     assert not np.isfinite(gpu_context.coupling_matvec(x, _lib.SG_FP32)).any()
+
+
+@pytest.mark.parametrize("n,bs,R", [(1024, 4, 16), (1025, 4, 17), (3100, 3, 35)])
+def test_fp32_sums_in_chunks(n, bs, R, gpu_context):
+    """Systems of one, two and four chunks of tiles, groups of 16 right-hand sides with a remainder. Bound: 2.5e-6 of
+    the operands and products as in test_gpu_ibatch32.py, and sums over about 1024 pairs (sqrt(1024) 2^-24)."""
+    res = 40.0
+    rng = np.random.default_rng(n)
+    xy = rng.uniform(0, 2500.0, (n, 2))
+    m = rng.integers(-3, 4, bs)
+    table = rng.standard_normal((100, bs, bs)) + 1j * rng.standard_normal((100, bs, bs))
+    x = rng.standard_normal((n, bs, R)) + 1j * rng.standard_normal((n, bs, R))
+    _upload(gpu_context, xy, m, table, res, bs)
+    assert gpu_context.fp32_batched(R, take=True)[0]
+    y = gpu_context.coupling_matvec(x.reshape(n * bs, R), _lib.SG_FP32).reshape(n, bs, R)
+    rows = rng.choice(n, 40, replace=False)
+    d = xy[rows, None] - xy[None]
+    s = np.sqrt((d ** 2).sum(-1)) / res
+    k = np.floor(s).astype(int)
+    w = table[k] + (s - k)[..., None, None] * (table[k + 1] - table[k])
+    w = w * np.exp(1j * (m[None, :] - m[:, None]) * np.arctan2(d[..., 1], d[..., 0])[..., None, None])
+    ref = np.einsum("ijab,jbr->iar", w, x)
+    for r in range(R):
+        assert np.linalg.norm(y[rows, :, r] - ref[..., r]) <= 4.4e-6 * np.linalg.norm(ref[..., r])
