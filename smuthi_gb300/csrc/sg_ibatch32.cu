@@ -12,7 +12,7 @@
 // it and writes the A operand (a lane per column, K = 2 blocksize: Im and Re) to tensor memory, waits for the products
 // (one accumulator of 64 Re and 64 Im columns per set and pass), combines the powers of t, rotates back and adds the
 // contribution to y_i with vector atomics (in any order: the last bits of a product differ from run to run; with many
-// particles in chunks of tiles, kIhTerms). One thread issues the MMAs against the interval's B operand in shared memory
+// particles in chunks of tiles, ih_chunks). One thread issues the MMAs against the interval's B operand in shared memory
 // (rows -Im C, Re C, Im C as in the FP64 form); three warps prepare the tiles' t and phases ahead.
 //
 // Every wait is bounded; a wait that runs out sets the error flag, and all roles leave.
@@ -534,12 +534,15 @@ __global__ void __launch_bounds__(256) ih_operand_kernel(const double2 *coef, co
 
 static constexpr size_t kIhMaxOperands = (size_t)16 << 30;
 
-// Pairs of a receiver that are added one after the other in FP32, on average: n such roundings grow with sqrt(n) or
-// faster, so that larger systems run in chunks of tiles whose sums are added in FP64. Without chunks the error of a
-// film's product was 9.1e-7 with 2000 spheres, 1.3e-6 with 4001 and 2.1e-6 with 10000, where the pair-symmetric
-// tensor-core kernel has 1.7e-6 throughout; with chunks 6.4e-7, 6.4e-7 and 6.3e-7, in 6.03 ms instead of 6.01, 23.9
-// instead of 23.8 and 149.4 instead of 148.8.
-static constexpr int kIhTerms = 1024;
+// Pairs of a receiver that are added one after the other in FP32, on average. Larger systems run in chunks of tiles whose
+// sums are added in FP64, for two reasons. The error of n such roundings grows with n: films of 2000 / 4001 / 10000
+// spheres 9.1e-7 / 1.3e-6 / 2.1e-6 in one chunk (the pair-symmetric tensor-core kernel: 1.7e-6), now 4.4e-7 / 4.6e-7 /
+// 3.4e-7. And their order differs from product to product, so that the residual of a solve does not fall below what it
+// changes, which a film multiplies by five: with 2.3e-7 (1024 terms) 10000 spheres stood at 1.2e-6 before the correction's
+// 1e-6 for 302 to 362 iterations, with 1.4e-7 it takes 185. Every chunk costs a launch, a last wave and a pass over the
+// sums: 7.26 ms instead of 7.17 with 2000 spheres, cubic, 24.1 instead of 23.8 with 4001, 152.1 instead of 149.0 with
+// 10000. From 5000 particles on a chunk is long enough to halve the terms for 1%, which keeps what changes below 1.5e-7.
+static int ih_chunks(int n) { return (n + (n > 5000 ? 255 : 511)) / (n > 5000 ? 256 : 512); }
 
 template <class F>
 static void ih_dispatch(const sg_context *c, F &&f) {
@@ -609,7 +612,7 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
     auto &tl = ib_tiles(c, a.rt, 1, st);
     a.toff = tl.toff.ptr;
     a.per = tl.per;
-    const int ntiles = tl.h_toff.back(), chunks = (c->n + kIhTerms - 1) / kIhTerms;
+    const int ntiles = tl.h_toff.back(), chunks = ih_chunks(c->n);
     if (chunks > 1) P.acc.reserve(len);
     const size_t elems = (size_t)c->n * kp * a.rt;
     P.xh.reserve(elems);

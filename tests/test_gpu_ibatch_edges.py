@@ -97,9 +97,9 @@ def test_table_beyond_fp32(gpu_context):
     assert not np.isfinite(gpu_context.coupling_matvec(x, _lib.SG_FP32)).any()
 
 
-@pytest.mark.parametrize("n,bs,R", [(1024, 4, 16), (1025, 4, 17), (3100, 3, 35)])
+@pytest.mark.parametrize("n,bs,R", [(512, 4, 16), (513, 4, 16), (1024, 4, 16), (1025, 4, 17), (3100, 3, 35), (5001, 2, 16)])
 def test_fp32_sums_in_chunks(n, bs, R, gpu_context):
-    """Systems of one, two and four chunks of tiles, groups of 16 right-hand sides with a remainder. Bound: 2.5e-6 of
+    """Systems of one to twenty chunks of tiles, groups of 16 right-hand sides with a remainder. Bound: 2.5e-6 of
     the operands and products as in test_gpu_ibatch32.py, and sums over about 1024 pairs (sqrt(1024) 2^-24)."""
     res = 40.0
     rng = np.random.default_rng(n)
