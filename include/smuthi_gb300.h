@@ -186,7 +186,7 @@ int sg_fp32_autotune(sg_context *ctx, int nrhs, int *variant, int *rhs_tile, dou
 /* Fixes the FP32 operator for an RHS count instead of timing the candidates: variant 0 =
  * per-receiver kernel (rhs_tile 1, 2, 4, 8 or 16 dividing nrhs), 1 = interval-bucketed kernel
  * (rhs_tile ignored; needs its plan), 2 = pair-symmetric kernel (rhs_tile a power of two dividing
- * nrhs, at most 16 for blocksize <= 32 and 8 for blocksize <= 64), 3 = pair-symmetric kernel with two
+ * nrhs, at most 16 for even blocksizes <= 32 and 8 for even ones <= 64), 3 = pair-symmetric kernel with two
  * warps per receiver (the same tiles, at least 4), 4 = tensor-core operator (rhs_tile = nrhs, in
  * {16, 32, 64}; blocksize <= 48), 5 = pair-symmetric tensor-core operator (rhs_tile = nrhs, in
  * {16, 32}; blocksize <= 32). Replaces an earlier choice for

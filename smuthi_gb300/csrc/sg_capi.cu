@@ -680,7 +680,7 @@ int sg_fp32_set_kernel(sg_context *ctx, int nrhs, int variant, int rhs_tile) {
                  "the pair-symmetric tensor-core operator needs blocksize <= 32 and nrhs in {16, 32}");
       SG_REQUIRE(rhs_tile == nrhs, "the tensor-core operators take all right-hand sides at once (rhs_tile = nrhs)");
     } else {
-      SG_REQUIRE(sg::sym_supported(ctx), "the pair-symmetric kernel needs blocksize <= 64");
+      SG_REQUIRE(sg::sym_supported(ctx), "the pair-symmetric kernel needs an even blocksize <= 64");
       SG_REQUIRE(rhs_tile >= 1 && rhs_tile <= sg::sym_max_tile(ctx) && (rhs_tile & (rhs_tile - 1)) == 0,
                  "pair-symmetric RHS tile must be a power of two within the kernel's register budget");
       SG_REQUIRE(nrhs % rhs_tile == 0, "RHS tile must divide nrhs");

@@ -531,7 +531,8 @@ __global__ void sym_epilogue_kernel(const float2 *yacc, const double2 *x, double
 }
 
 // ------------------------------------------------------------------ plan and dispatch
-bool sym_supported(const sg_context *c) { return !c->vol && c->bs >= 2 && c->bs <= 64 && c->n >= 1; }
+// even blocksizes only: the bulk copies of coefficient columns (8 blocksize bytes each) must start on 16 bytes
+bool sym_supported(const sg_context *c) { return !c->vol && c->bs >= 2 && c->bs <= 64 && c->bs % 2 == 0 && c->n >= 1; }
 
 int sym_max_tile(const sg_context *c) { return c->bs <= 32 ? 16 : 8; }
 
@@ -610,7 +611,7 @@ static void launch_sym_r(sg_context *c, const SymLaunch &L, int rt, int split, c
 
 int launch_sym_matvec(sg_context *c, const double2 *x, double2 *y, int R, bool master, int rt, int split,
                       cudaStream_t st) {
-  SG_REQUIRE(sym_supported(c), "symmetric FP32 kernel: radial lookup with blocksize <= 64 required");
+  SG_REQUIRE(sym_supported(c), "symmetric FP32 kernel: radial lookup with an even blocksize <= 64 required");
   SG_REQUIRE(split == 1 || (split == 2 && rt >= 4), "symmetric FP32 kernel: two warps per receiver need a tile >= 4");
   SG_REQUIRE(c->pairs_ready, "symmetric FP32 kernel: the pair table is not built");
   SG_REQUIRE(rt >= 1 && R % rt == 0 && rt <= sym_max_tile(c), "symmetric FP32 kernel: bad RHS tile");
