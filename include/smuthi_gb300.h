@@ -46,10 +46,10 @@ extern "C" {
  * sg_precond_select; a correction solve that fails to reduce its residual is redone without it */
 #define SG_PRECOND 4
 /* FP64-grade operator: with the radial lookup, 32 particles or more and blocksize <= 48 the
- * interval-batched operator that SG_FP64 uses; otherwise, and under stream capture, double-float
- * arithmetic: every sum in two FP32 words (about 48 significant bits) on the FP32 pipe, with the FP64
- * table split into two FP32 words (it agrees with SG_FP64 to ~1e-13 relative). OR-ed into
- * sg_gmres_solve's precision with SG_FP32, the refinement's true residuals use it. No counterpart in the reference. */
+ * interval-batched operator that SG_FP64 uses; otherwise double-float arithmetic: every sum in two FP32
+ * words (about 48 significant bits) on the FP32 pipe, with the FP64 table split into two FP32 words (it
+ * agrees with SG_FP64 to ~1e-13 relative). OR-ed into sg_gmres_solve's precision with SG_FP32, the
+ * refinement's true residuals use it. No counterpart in the reference. */
 #define SG_DF64 8
 /* matvec precision: the coupling operator on the tensor cores (tcgen05.mma kind::tf32, each
  * operand split into a TF32 high part and a remainder, three products), for the radial lookup with
@@ -123,6 +123,10 @@ int sg_coupling_matvec(sg_context *ctx, const double *x, double *y, int nrhs, in
 /* y = x - T W x, the master operator (smuthi/linearsystem/linear_system.py:402-407). */
 int sg_master_matvec(sg_context *ctx, const double *x, double *y, int nrhs, int precision);
 
+/* Stream capture: make one uncaptured product of the same precision and nrhs first. The captured product then runs the
+ * same kernels with scratch memory that belongs to the graph (SG_FP32 variants 1 to 5: in the context's, which later
+ * products of other counts may move). Without it an FP64 product takes the per-receiver kernel, a double-float one of a
+ * context that has made FP64-grade products of another nrhs too, and an FP32 one fails. */
 /* Device-pointer variants: x, y are device buffers in the reference layout;
  * `stream` is a cudaStream_t (NULL = the context's stream). Asynchronous. */
 int sg_coupling_matvec_dev(sg_context *ctx, const void *x, void *y, int nrhs, int precision, void *stream);
@@ -197,8 +201,8 @@ int sg_fp32_set_kernel(sg_context *ctx, int nrhs, int variant, int rhs_tile);
 /* The interval-batched FP32 operator (pairs grouped by lookup interval, tensor cores) takes the place of
  * variants 4 and 5 for an RHS count >= 16 when the autotuner finds it faster: *taken = 1 then, and *ms its
  * time (-1 when not timed; either pointer may be NULL). take != 0 fixes it for that RHS count (32 particles
- * or more, blocksize <= 30 or 33 to 48) until the next set_particles, set_lookup or sg_fp32_set_kernel. Under
- * stream capture the variant that sg_fp32_autotune reports runs. No counterpart in the reference. */
+ * or more, blocksize <= 30 or 33 to 48) until the next set_particles, set_lookup or sg_fp32_set_kernel. No
+ * counterpart in the reference. */
 int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms);
 
 /* Emitters accumulated into one tensor-memory accumulator of the tensor-core operator before it is

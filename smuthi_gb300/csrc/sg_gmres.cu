@@ -1081,17 +1081,15 @@ void solve_padded(sg_context *c, const double2 *b, double2 *x, int R, double rto
   }
 }
 
-// y = M x or W x on padded vectors (public matvec entry points)
-// One CUDA-event-timed run of each FP32 kernel on the live operands; the faster one is cached per
-// RHS count. Runs once per (context, nrhs) and synchronises the stream, so it must not be reached
-// inside a stream capture.
-static void launch_receiver_fp32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st,
-                                 int rt = 0) {
+// the per-receiver kernel; rt: RHS tile (FP32; 0 = default choice)
+static void launch_receiver(sg_context *c, const double2 *x, double2 *y, int R, bool master, bool fp32, int rt,
+                            cudaStream_t st) {
+  CallMemory mem(st);
   CouplingLaunch L{};
   L.pos = c->pos.ptr;
   L.mofn = c->mofn.ptr;
-  L.coef = c->coef32.ptr;
-  L.pairs = c->pairs.ptr;
+  L.coef = fp32 ? (const void *)c->coef32.ptr : (const void *)c->coef64.ptr;
+  L.pairs = fp32 ? c->pairs.ptr : nullptr;
   L.n = c->n;
   L.bs = c->bs;
   L.n_int = c->n_int;
@@ -1100,33 +1098,34 @@ static void launch_receiver_fp32(sg_context *c, const double2 *x, double2 *y, in
   L.res = c->res;
   L.x = x;
   const size_t len = (size_t)c->n * c->bs * R;
-  c->bk_x32.reserve(len);
-  k_to_f32(x, c->bk_x32.ptr, len, st);
-  c->launches += 1;
-  L.x32 = c->bk_x32.ptr;
+  if (fp32) {  // one FP32 copy of the input instead of an FP64->FP32 conversion per pair
+    float2 *x32 = mem.get(c->bk_x32, len);
+    k_to_f32(x, x32, len, st);
+    c->launches += 1;
+    L.x32 = x32;
+    L.rt = rt;
+  }
   L.y = y;
   L.nrhs = R;
-  L.rt = rt;
   L.master = master ? 1 : 0;
   L.t = c->tmat.ptr;
   L.ptype = c->ptype.ptr;
   L.t_diag = c->t_diag;
   const int ns = choose_split(c->n, R);
-  if (ns > 1) {
-    c->w_partial.reserve((size_t)ns * c->n * c->bs * R);
-    L.partial = c->w_partial.ptr;
-  }
-  c->launches += launch_coupling(L, true, ns, st);
+  if (ns > 1) L.partial = mem.get(c->w_partial, ns * len);
+  c->launches += launch_coupling(L, fp32, ns, st);
 }
 
-// The interval-batched operators keep a workspace and order their calls by an event, which a captured
-// graph could not follow: under stream capture the other kernels run.
-static bool ib_usable(const sg_context *c, cudaStream_t st) {
-  if (!ib_supported(c)) return false;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+// Under stream capture the interval-batched operators need what an earlier call prepared; otherwise the other kernels run.
+static bool ib_usable(const sg_context *c, int R, cudaStream_t st) {
+  return ib_supported(c) && (!capturing(st) || ib_prepared(c, R));
+}
+static bool ib32_usable(const sg_context *c, int R, cudaStream_t st) {
+  return ib32_supported(c, R) && (!capturing(st) || ib32_prepared(c, R));
 }
 
+// One CUDA-event-timed run of each FP32 kernel on the live operands; the fastest is cached per RHS count. Runs once per
+// (context, nrhs) and synchronises the stream, so it must not be reached inside a stream capture.
 static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   // Candidates, each warmed once (first launches carry one-time set-up) and timed once with CUDA events on the live
   // operands; the ones that are fastest with many right-hand sides come first, and a candidate whose first run
@@ -1153,7 +1152,7 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
   // sides: 4.5e-7 against 2.7e-7; 13.6 against 7.2 ms); where an FP32-pipe kernel wins, that one rounds better
   // (100 spheres: 4.5e-8 against 5.6e-8) and stays.
   float ms_batched = -1.f;
-  if (ib32_supported(c, R) && ib_usable(c, st))
+  if (ib32_usable(c, R, st))
     ms_batched = time_it([&] { c->launches += launch_ibatch32(c, x, y, R, master, st); });
   // the tensor-core operators (3xTF32, accumulators drained every few emitters)
   float ms_tc = -1.f, ms_tcs = -1.f;
@@ -1188,7 +1187,7 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
   float best_rec = -1.f;
   int best_rt = tiles.front();
   for (int rt : tiles) {
-    const float ms = time_it([&] { launch_receiver_fp32(c, x, y, R, master, st, rt); });
+    const float ms = time_it([&] { launch_receiver(c, x, y, R, master, true, rt, st); });
     if (best_rec < 0.f || ms < best_rec) {
       best_rec = ms;
       best_rt = rt;
@@ -1221,6 +1220,7 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
   return v;
 }
 
+// y = M x or W x on padded vectors (public matvec entry points)
 void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool master, bool fp32, cudaStream_t st) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c->profiling) {
@@ -1249,9 +1249,9 @@ void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool maste
       batched = c->tuned.back().batched;
     }
   }
-  if (variant == 0 && !fp32 && ib_usable(c, st)) {
+  if (variant == 0 && !fp32 && ib_usable(c, R, st)) {
     c->launches += launch_ibatch(c, x, y, R, master, st);
-  } else if (batched && ib_usable(c, st)) {
+  } else if (batched && ib32_usable(c, R, st)) {
     c->launches += launch_ibatch32(c, x, y, R, master, st);
   } else if (variant == 5) {
     c->launches += launch_tcsym_matvec(c, x, y, R, master, st);
@@ -1262,38 +1262,7 @@ void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool maste
   } else if (variant == 1) {
     c->launches += launch_bucket_matvec(c, x, y, R, master, st);
   } else if (variant == 0) {
-    CouplingLaunch L{};
-    L.pos = c->pos.ptr;
-    L.mofn = c->mofn.ptr;
-    L.coef = fp32 ? (const void *)c->coef32.ptr : (const void *)c->coef64.ptr;
-    L.pairs = fp32 ? c->pairs.ptr : nullptr;
-    L.n = c->n;
-    L.bs = c->bs;
-    L.n_int = c->n_int;
-    L.ncoef = c->ncoef;
-    L.rho_min = c->rho_min;
-    L.res = c->res;
-    L.x = x;
-    if (fp32) {  // one FP32 copy of the input instead of an FP64->FP32 conversion per pair
-      const size_t len = (size_t)c->n * c->bs * R;
-      c->bk_x32.reserve(len);
-      k_to_f32(x, c->bk_x32.ptr, len, st);
-      c->launches += 1;
-      L.x32 = c->bk_x32.ptr;
-      L.rt = rt;
-    }
-    L.y = y;
-    L.nrhs = R;
-    L.master = master ? 1 : 0;
-    L.t = c->tmat.ptr;
-    L.ptype = c->ptype.ptr;
-    L.t_diag = c->t_diag;
-    const int ns = choose_split(c->n, R);
-    if (ns > 1) {
-      c->w_partial.reserve((size_t)ns * c->n * c->bs * R);
-      L.partial = c->w_partial.ptr;
-    }
-    c->launches += launch_coupling(L, fp32, ns, st);
+    launch_receiver(c, x, y, R, master, fp32, rt, st);
   }
   if (c->profiling) {
     SG_CUDA(cudaEventRecord(e1, st));
@@ -1308,6 +1277,7 @@ static void launch_df64(sg_context *c, const double2 *x, double2 *y, int R, bool
 static int df64_tile(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   for (const auto &t : c->tuned_df)
     if (t.first == R) return t.second;
+  if (capturing(st)) return 0;
   int best = 0;
   if (R % 8 == 0) {
     cudaEvent_t e[4];
@@ -1345,13 +1315,19 @@ void apply_padded_df64(sg_context *c, const double2 *x, double2 *y, int R, bool 
     mark(e1);
     if (c->profiling) c->events.push_back({e0, e1, 2});
   };
-  if (ib_usable(c, st)) {
+  if (ib_usable(c, R, st)) {
     mark(e0);
     c->launches += launch_ibatch(c, x, y, R, master, st);
     done();
     return;
   }
   const size_t ncoef_total = (size_t)c->n_int * c->ncoef * c->bs * c->bs;
+  if (!c->df_ready && capturing(st)) {  // its coefficients cannot be kept from there: the FP64 kernel
+    mark(e0);
+    launch_receiver(c, x, y, R, master, false, 0, st);
+    done();
+    return;
+  }
   if (!c->df_ready) {
     c->coefdf.reserve(ncoef_total);
     build_coefficients_df64(c->coef64.ptr, c->coefdf.ptr, ncoef_total, st);
@@ -1378,11 +1354,12 @@ static void launch_df64(sg_context *c, const double2 *x, double2 *y, int R, bool
   L.rho_min = c->rho_min;
   L.res = c->res;
   L.x = x;
+  CallMemory mem(st);
   const size_t len = (size_t)c->n * c->bs * R;
-  c->xdf.reserve(len);
-  k_to_df64(x, c->xdf.ptr, len, st);
+  double2 *xdf = mem.get(c->xdf, len);
+  k_to_df64(x, xdf, len, st);
   c->launches += 1;
-  L.xdf = c->xdf.ptr;
+  L.xdf = xdf;
   L.y = y;
   L.nrhs = R;
   L.master = master ? 1 : 0;
@@ -1390,10 +1367,7 @@ static void launch_df64(sg_context *c, const double2 *x, double2 *y, int R, bool
   L.ptype = c->ptype.ptr;
   L.t_diag = c->t_diag;
   const int ns = choose_split(c->n, R);
-  if (ns > 1) {
-    c->w_partial.reserve((size_t)ns * c->n * c->bs * R);
-    L.partial = c->w_partial.ptr;
-  }
+  if (ns > 1) L.partial = mem.get(c->w_partial, ns * len);
   c->launches += launch_coupling_df64(L, ns, st);
 }
 

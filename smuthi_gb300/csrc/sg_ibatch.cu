@@ -982,11 +982,21 @@ static void ib_digit_operands(sg_context *c, cudaStream_t st) {
 
 void ib_enter(sg_context *c, cudaStream_t st) {
   auto &P = c->ib;
+  if (capturing(st)) {  // a wait for the event would tie the graph to this one call; the host may wait in relaxed mode
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    SG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaEventSynchronize(P.done);
+    SG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    SG_CUDA(e);
+    return;
+  }
   if (!P.done) SG_CUDA(cudaEventCreateWithFlags(&P.done, cudaEventDisableTiming));
   else SG_CUDA(cudaStreamWaitEvent(st, P.done, 0));
 }
 
-void ib_leave(sg_context *c, cudaStream_t st) { SG_CUDA(cudaEventRecord(c->ib.done, st)); }
+void ib_leave(sg_context *c, cudaStream_t st) {
+  if (!capturing(st)) SG_CUDA(cudaEventRecord(c->ib.done, st));
+}
 
 // The tiles for rt right-hand sides: first tile of every interval. Where 64 columns make hardly more tiles than 128,
 // most are not half full and two sets of warps that overlap their tiles are faster: 100 spheres (1.00 times the tiles)
@@ -1016,6 +1026,26 @@ sg_context::IbTiles &ib_tiles(sg_context *c, int rt, int sets, cudaStream_t st) 
   return *P.tiles.back();
 }
 
+bool ib_has_tiles(const sg_context *c, int rt, int sets) {
+  for (const auto &t : c->ib.tiles)
+    if (t->rt == rt && t->asked == sets) return true;
+  return false;
+}
+
+// Right-hand sides at a time: their pairs share t and the phases and fill the tiles of a sparse interval, but every
+// further chunk goes through the slots again. 16 of them, one / four / sixteen at a time: 301 spheres (0.07 GB of V a
+// right-hand side) 2.90 / 1.76 / 1.45 ms, 1000 (0.5 GB) 23.7 / 20.9 / 20.6, 2000 (1.9 GB) 85.8 / 82.4 / 83.0, 4000
+// (7.7 GB) 334 / 334 / 374.
+int ib_group(const sg_context *c, int R) {
+  const size_t row = (size_t)c->n * c->n * c->bs * sizeof(double2);
+  return std::min(R, (int)std::min<size_t>(16, std::max<size_t>(1, 4 * kIbWorkspace / row)));
+}
+
+bool ib_prepared(const sg_context *c, int R) {
+  const int most = ib_group(c, R);
+  return c->ib.ready && c->ib.digits_ready && ib_has_tiles(c, most, 0) && (R % most == 0 || ib_has_tiles(c, R % most, 0));
+}
+
 template <int NC, int KP, int SETS>
 static void ib_launch(const IbArgs &a, cudaStream_t st) {
   static bool attr_done[64] = {};
@@ -1029,9 +1059,12 @@ static void ib_launch(const IbArgs &a, cudaStream_t st) {
 // y = M x or W x in FP64; returns the number of kernels launched
 int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   auto &P = c->ib;
+  CallMemory mem(st);
   ib_enter(c, st);
-  ib_plan(c, st);
-  ib_digit_operands(c, st);
+  if (!mem.graph) {
+    ib_plan(c, st);
+    ib_digit_operands(c, st);
+  }
   const int bs = c->bs;
   CouplingLaunch L{};
   L.n = c->n;
@@ -1045,11 +1078,8 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
   L.t_diag = c->t_diag;
   int mmax = 0, launched = 0;
   for (int m : c->h_mofn) mmax = std::max(mmax, std::abs(m));
-  // Right-hand sides at a time: their pairs share t and the phases and fill the tiles of a sparse interval, but every
-  // further chunk goes through the slots again. 16 of them, one / four / sixteen at a time: 301 spheres (0.07 GB of V a
-  // right-hand side) 2.90 / 1.76 / 1.45 ms, 1000 (0.5 GB) 23.7 / 20.9 / 20.6, 2000 (1.9 GB) 85.8 / 82.4 / 83.0, 4000
-  // (7.7 GB) 334 / 334 / 374.
-  const int most = (int)std::min<size_t>(16, std::max<size_t>(1, 4 * kIbWorkspace / ((size_t)c->n * c->n * bs * sizeof(double2))));
+  const int most = ib_group(c, R);
+  double2 *acc = nullptr;
   for (int r0 = 0, rt; r0 < R; r0 += rt) {
     rt = std::min(most, R - r0);
     auto &tl = ib_tiles(c, rt, 0, st);
@@ -1057,8 +1087,8 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     const size_t pair_bytes = (size_t)rt * bs * sizeof(double2);
     const int ntiles = tl.h_toff.back();
     const int chunk = (int)std::min<size_t>(ntiles, std::max<size_t>(1, kIbWorkspace / (pair_bytes * per)));
-    P.V.reserve((size_t)std::min<long long>((long long)chunk * per, (long long)c->n * c->n) * rt * bs);
-    if (chunk < ntiles) P.acc.reserve((size_t)c->n * bs * R);
+    double2 *V = mem.get(P.V, (size_t)std::min<long long>((long long)chunk * per, (long long)c->n * c->n) * rt * bs);
+    if (chunk < ntiles && !acc) acc = mem.get(P.acc, (size_t)c->n * bs * R);
     auto first_pair = [&](int t) -> long long {  // first pair of tile t
       const int b = (int)(std::upper_bound(tl.h_toff.begin(), tl.h_toff.end(), t) - tl.h_toff.begin()) - 1;
       if (b >= P.nb) return (long long)c->n * c->n;
@@ -1071,16 +1101,16 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     a.B = P.B.ptr;
     a.exps = P.exps.ptr;
     const size_t words = (size_t)c->n * rt * ib_kp(c);
-    P.xw.reserve(words);
-    P.xe.reserve(words);
+    int4 *xw = mem.get(P.xw, words);
+    int *xe = mem.get(P.xe, words);
     (ib_kp(c) == 32 ? ib_words_kernel<32> : ib_words_kernel<48>)<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(
-        x, c->n, bs, R, r0, rt, P.xw.ptr, P.xe.ptr);
+        x, c->n, bs, R, r0, rt, xw, xe);
     SG_CUDA(cudaGetLastError());
     ++launched;
-    a.x = P.xw.ptr;
-    a.xe = P.xe.ptr;
+    a.x = xw;
+    a.xe = xe;
     a.mofn = c->mofn.ptr;
-    a.V = P.V.ptr;
+    a.V = V;
     a.nb = P.nb;
     a.bs = bs;
     a.mmax = mmax;
@@ -1088,9 +1118,9 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     a.per = per;
     a.err = P.err.ptr;
     IbSum s{};
-    s.V = P.V.ptr;
+    s.V = V;
     s.slot = P.slot.ptr;
-    s.acc = P.acc.ptr;
+    s.acc = acc;
     s.err = P.err.ptr;
     s.rt = rt;
     s.r0 = r0;

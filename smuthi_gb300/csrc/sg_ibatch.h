@@ -36,7 +36,12 @@ __device__ __forceinline__ void ib_exponents(const double2 *C, int bs, int *eb, 
 void ib_plan(sg_context *c, cudaStream_t st);
 // tiles for rt right-hand sides; sets = 0: chosen for the FP64 operator
 sg_context::IbTiles &ib_tiles(sg_context *c, int rt, int sets, cudaStream_t st);
-// orders the calls that use the plan and its workspaces across streams
+// the tiles exist
+bool ib_has_tiles(const sg_context *c, int rt, int sets);
+// right-hand sides of the FP64 operator at a time
+int ib_group(const sg_context *c, int R);
+// Orders the calls that use the plan and its workspaces across streams. A captured call has workspaces of its own and only
+// needs the plan: what prepares it must have run.
 void ib_enter(sg_context *c, cudaStream_t st);
 void ib_leave(sg_context *c, cudaStream_t st);
 

@@ -567,11 +567,16 @@ bool ib32_supported(const sg_context *c, int R) {
   return std::min<size_t>(c->n_int, (size_t)c->n * c->n) * operand <= kIhMaxOperands;
 }
 
+bool ib32_prepared(const sg_context *c, int R) {
+  return c->ib.ready && c->ib.halves_ready && ib_has_tiles(c, 16, 1) && (R % 16 == 0 || ib_has_tiles(c, R % 16, 1));
+}
+
 // y = M x or W x in FP32; returns the number of kernels launched
 int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   auto &P = c->ib;
+  CallMemory mem(st);
   ib_enter(c, st);
-  ib_plan(c, st);
+  if (!mem.graph) ib_plan(c, st);
   const int bs = c->bs, kp = bs <= 32 ? 32 : 48;
   int launched = 0;
   if (!P.halves_ready) {
@@ -586,12 +591,12 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
     P.halves_ready = true;
   }
   const size_t len = (size_t)c->n * bs * R;
-  c->sym_yacc.reserve(len);
-  SG_CUDA(cudaMemsetAsync(c->sym_yacc.ptr, 0, len * sizeof(float2), st));
-  P.top.reserve(256);
-  SG_CUDA(cudaMemsetAsync(P.top.ptr, 0, R * sizeof(int), st));
+  float2 *yacc = mem.get(c->sym_yacc, len);
+  SG_CUDA(cudaMemsetAsync(yacc, 0, len * sizeof(float2), st));
+  int *top = mem.get(P.top, 256);
+  SG_CUDA(cudaMemsetAsync(top, 0, R * sizeof(int), st));
   const size_t rows = (size_t)c->n * bs;
-  ih_top_kernel<<<(unsigned)std::min<size_t>((rows * R + 2047) / 2048, (size_t)sm_count() * 4), 256, 0, st>>>(x, rows, R, P.top.ptr);
+  ih_top_kernel<<<(unsigned)std::min<size_t>((rows * R + 2047) / 2048, (size_t)sm_count() * 4), 256, 0, st>>>(x, rows, R, top);
   SG_CUDA(cudaGetLastError());
   ++launched;
   IhArgs a{};
@@ -600,26 +605,27 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
   a.B = P.H.ptr;
   a.exps = P.exps.ptr;
   a.mofn = c->mofn.ptr;
-  a.y = c->sym_yacc.ptr;
+  a.y = yacc;
   a.nb = P.nb;
   a.bs = bs;
   a.R = R;
   a.err = P.err.ptr;
   for (int m : c->h_mofn) a.mmax = std::max(a.mmax, std::abs(m));
+  const int chunks = ih_chunks(c->n);
+  double2 *total = chunks > 1 ? mem.get(P.acc, len) : nullptr;
+  float2 *xh = mem.get(P.xh, (size_t)c->n * kp * std::min(16, R));
   for (int r0 = 0; r0 < R; r0 += 16) {
     a.r0 = r0;
     a.rt = std::min(16, R - r0);
     auto &tl = ib_tiles(c, a.rt, 1, st);
     a.toff = tl.toff.ptr;
     a.per = tl.per;
-    const int ntiles = tl.h_toff.back(), chunks = ih_chunks(c->n);
-    if (chunks > 1) P.acc.reserve(len);
+    const int ntiles = tl.h_toff.back();
     const size_t elems = (size_t)c->n * kp * a.rt;
-    P.xh.reserve(elems);
-    ih_copy_kernel<<<(unsigned)((elems + 255) / 256), 256, 0, st>>>(x, c->n, bs, kp, R, r0, a.rt, P.top.ptr, P.xh.ptr);
+    ih_copy_kernel<<<(unsigned)((elems + 255) / 256), 256, 0, st>>>(x, c->n, bs, kp, R, r0, a.rt, top, xh);
     SG_CUDA(cudaGetLastError());
     ++launched;
-    a.x = P.xh.ptr;
+    a.x = xh;
     for (int q = 0; q < chunks; ++q) {
       a.t0 = (int)((long long)ntiles * q / chunks);
       a.t1 = (int)((long long)ntiles * (q + 1) / chunks);
@@ -636,14 +642,14 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
         ++launched;
       }
       if (chunks > 1) {
-        ih_fold_kernel<<<(unsigned)((rows * a.rt + 255) / 256), 256, 0, st>>>(a.y, P.acc.ptr, rows, R, r0, a.rt, q == 0,
+        ih_fold_kernel<<<(unsigned)((rows * a.rt + 255) / 256), 256, 0, st>>>(a.y, total, rows, R, r0, a.rt, q == 0,
                                                                               q == chunks - 1);
         SG_CUDA(cudaGetLastError());
         ++launched;
       }
     }
   }
-  launch_fp32_epilogue(c, x, y, R, master, st, P.top.ptr, P.err.ptr);
+  launch_fp32_epilogue(c, x, y, R, master, st, top, P.err.ptr, yacc);
   ib_leave(c, st);
   return launched + 1;
 }

@@ -61,6 +61,46 @@ struct DevBuf {
   }
 };
 
+inline bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  SG_CUDA(cudaStreamIsCapturing(st, &s));
+  return s != cudaStreamCaptureStatusNone;
+}
+
+// Scratch memory of one call: the context's buffers, or, under stream capture, memory that the graph allocates and frees
+// itself (nothing else can be allocated there, and a later call that grows a buffer of the context would leave the graph
+// with the old address).
+struct CallMemory {
+  struct Own {
+    const void *kept;
+    void *ptr;
+    size_t bytes;
+  };
+  cudaStream_t st;
+  bool graph;
+  std::vector<Own> own;
+  explicit CallMemory(cudaStream_t s) : st(s), graph(capturing(s)) {}
+  CallMemory(const CallMemory &) = delete;
+  CallMemory &operator=(const CallMemory &) = delete;
+  ~CallMemory() {
+    for (const Own &o : own) cudaFreeAsync(o.ptr, st);
+  }
+  // `count` elements in place of the context's buffer `kept`
+  template <typename T>
+  T *get(DevBuf<T> &kept, size_t count) {
+    if (!graph) {
+      kept.reserve(count);
+      return kept.ptr;
+    }
+    for (const Own &o : own)
+      if (o.kept == &kept && o.bytes >= count * sizeof(T)) return static_cast<T *>(o.ptr);
+    void *p = nullptr;
+    SG_CUDA(cudaMallocAsync(&p, count * sizeof(T), st));
+    own.push_back({&kept, p, count * sizeof(T)});
+    return static_cast<T *>(p);
+  }
+};
+
 // pinned host memory, the same way
 template <typename T>
 struct PinnedBuf {
@@ -116,11 +156,11 @@ int launch_tc_matvec(sg_context *c, const double2 *x, double2 *y, int R, bool ma
 bool tc_check_error(sg_context *c, cudaStream_t st);  // reads and clears the timeout flag (synchronises)
 bool tcsym_supported(const sg_context *c, int R);
 int launch_tcsym_matvec(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
-// FP32 W x in c->sym_yacc -> FP64 W x or x - T (W x) (diagonal or dense T); one launch
+// FP32 W x in yacc (null: c->sym_yacc) -> FP64 W x or x - T (W x) (diagonal or dense T); one launch
 // top: largest exponent fields of x per right-hand side, by which x was scaled (null: not); err: flag of a wait that ran
 // out (null: none), which makes the result NaN
 void launch_fp32_epilogue(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st,
-                          const int *top = nullptr, const int *err = nullptr);
+                          const int *top = nullptr, const int *err = nullptr, const float2 *yacc = nullptr);
 #ifdef __CUDACC__
 // power of two that brings values with exponent field up to `top` below 1 (as far as it is a normal number)
 __device__ __forceinline__ double fp32_scale(int top) {
@@ -137,6 +177,9 @@ void residual_norms(sg_context *c, const double2 *b, const double2 *x, int R, do
 // FP64 operator batched by lookup interval on the tensor cores (sg_ibatch.cu)
 bool ib_supported(const sg_context *c);
 bool ib32_supported(const sg_context *c, int R);
+// under stream capture they take only what an earlier call with as many right-hand sides has prepared
+bool ib_prepared(const sg_context *c, int R);
+bool ib32_prepared(const sg_context *c, int R);
 int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 bool ib_check_error(sg_context *c, cudaStream_t st);  // reads and clears the timeout flag (synchronises)

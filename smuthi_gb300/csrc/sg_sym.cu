@@ -649,9 +649,9 @@ int launch_sym_matvec(sg_context *c, const double2 *x, double2 *y, int R, bool m
 }
 
 void launch_fp32_epilogue(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st, const int *top,
-                          const int *err) {
+                          const int *err, const float2 *yacc) {
   const size_t len = (size_t)c->n * c->bs * R;
-  sym_epilogue_kernel<<<(unsigned)((len + 255) / 256), 256, 0, st>>>(c->sym_yacc.ptr, x, y, c->n, c->bs, R,
+  sym_epilogue_kernel<<<(unsigned)((len + 255) / 256), 256, 0, st>>>(yacc ? yacc : c->sym_yacc.ptr, x, y, c->n, c->bs, R,
                                                                      master ? 1 : 0, c->tmat.ptr, c->ptype.ptr,
                                                                      c->t_diag, top, err);
   SG_CUDA(cudaGetLastError());
