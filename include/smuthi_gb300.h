@@ -15,6 +15,7 @@
 #ifndef SMUTHI_GB300_H
 #define SMUTHI_GB300_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -125,8 +126,8 @@ int sg_master_matvec(sg_context *ctx, const double *x, double *y, int nrhs, int 
 
 /* Stream capture: make one uncaptured product of the same precision and nrhs first. The captured product then runs the
  * same kernels with scratch memory that belongs to the graph (SG_FP32 variants 1 to 5: in the context's, which later
- * products of other counts may move). Without it an FP64 product takes the per-receiver kernel, a double-float one of a
- * context that has made FP64-grade products of another nrhs too, and an FP32 one fails. */
+ * products of other counts may move). Without it an FP64 or double-float product takes the FP64 per-receiver kernel, and
+ * an FP32 one fails. */
 /* Device-pointer variants: x, y are device buffers in the reference layout;
  * `stream` is a cudaStream_t (NULL = the context's stream). Asynchronous. */
 int sg_coupling_matvec_dev(sg_context *ctx, const void *x, void *y, int nrhs, int precision, void *stream);
@@ -204,6 +205,13 @@ int sg_fp32_set_kernel(sg_context *ctx, int nrhs, int variant, int rhs_tile);
  * or more, blocksize <= 30 or 33 to 48) until the next set_particles, set_lookup or sg_fp32_set_kernel. No
  * counterpart in the reference. */
 int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms);
+
+/* Device memory of the interval-batched operators: at most `limit` bytes for plan, operands and workspaces (0: no
+ * limit), of which `workspace` (0: 2 GiB) for the contributions that are formed at a time, larger problems running in
+ * chunks. A state that does not fit, or whose allocations fail, uses the other kernels until the next set_particles,
+ * set_lookup or call of this function, which also gives back what they hold (and with it what captured products use).
+ * No counterpart in the reference. */
+int sg_batched_memory(sg_context *ctx, size_t limit, size_t workspace);
 
 /* Emitters accumulated into one tensor-memory accumulator of the tensor-core operator before it is
  * added into the FP32 total (default 8). Fewer emitters bound the tensor core's accumulation error

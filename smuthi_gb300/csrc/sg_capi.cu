@@ -156,7 +156,7 @@ int sg_set_particles(sg_context *ctx, int n_particles, const double *xy, int n_u
       SG_CUDA(cudaMemcpy(ctx->map.ptr, map.data(), n_unknowns * sizeof(int), cudaMemcpyHostToDevice));
     }
     ctx->pairs_ready = false;
-    ctx->ib.ready = false;
+    ctx->ib.ready = ctx->ib.refused = ctx->ib.captured = false;
     ctx->tuned_df.clear();
     ctx->kind = -1;  // the table must be re-uploaded for a new geometry
     ctx->vol = false;
@@ -211,7 +211,7 @@ int sg_set_lookup(sg_context *ctx, int kind, int len_rho, double rho_min, double
     ctx->rho_min = rho_min;
     ctx->res = resolution;
     ctx->pairs_ready = false;
-    ctx->ib.ready = false;
+    ctx->ib.ready = ctx->ib.refused = ctx->ib.captured = false;
     ctx->df_ready = false;
     ctx->tuned_df.clear();
     ctx->pgraphs.clear();  // their near-field blocks came from the old table
@@ -629,7 +629,9 @@ int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms)
       ensure_pairs(ctx, ctx->stream);  // builds the FP32 operator data now (it would clear the choice later)
       SG_REQUIRE(sg::ib32_supported(ctx, nrhs),
                  "the interval-batched FP32 operator needs nrhs >= 16, 32 particles or more and blocksize <= 30 or 33 to 48");
-      sg_context::Tuned t{nrhs, 0, 1, -1.f, -1.f, 0, -1.f, -1.f, -1.f, -1.f, true};
+      int rt = 16;  // of the per-receiver kernel, which runs where the batched one cannot
+      while (nrhs % rt) rt /= 2;
+      sg_context::Tuned t{nrhs, 0, rt, -1.f, -1.f, 0, -1.f, -1.f, -1.f, -1.f, true};
       auto &v = ctx->tuned;
       v.erase(std::remove_if(v.begin(), v.end(), [&](const sg_context::Tuned &o) { return o.nrhs == nrhs; }), v.end());
       v.push_back(t);
@@ -643,6 +645,19 @@ int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms)
       }
     if (taken) *taken = on;
     if (ms) *ms = time;
+    return SG_OK;
+  });
+}
+
+int sg_batched_memory(sg_context *ctx, size_t limit, size_t workspace) {
+  return guarded([&]() -> int {
+    SG_REQUIRE(ctx, "null context");
+    use_device(ctx);
+    auto &P = ctx->ib;
+    P.limit = limit;
+    P.workspace = workspace ? workspace : (size_t)2 << 30;
+    P.refused = false;
+    sg::ib_drop(ctx);
     return SG_OK;
   });
 }

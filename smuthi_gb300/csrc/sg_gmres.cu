@@ -1124,6 +1124,19 @@ static bool ib32_usable(const sg_context *c, int R, cudaStream_t st) {
   return ib32_supported(c, R) && (!capturing(st) || ib32_prepared(c, R));
 }
 
+// f() of a batched operator; false where its memory cannot be had, which leaves the state to the other kernels
+template <class F>
+static bool ib_run(sg_context *c, F &&f) {
+  try {
+    c->launches += f();
+    return true;
+  } catch (const NoMemory &) {
+    if (!c->ib.captured) ib_drop(c);
+    c->ib.refused = true;
+    return false;
+  }
+}
+
 // One CUDA-event-timed run of each FP32 kernel on the live operands; the fastest is cached per RHS count. Runs once per
 // (context, nrhs) and synchronises the stream, so it must not be reached inside a stream capture.
 static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
@@ -1152,8 +1165,10 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
   // sides: 4.5e-7 against 2.7e-7; 13.6 against 7.2 ms); where an FP32-pipe kernel wins, that one rounds better
   // (100 spheres: 4.5e-8 against 5.6e-8) and stays.
   float ms_batched = -1.f;
-  if (ib32_usable(c, R, st))
-    ms_batched = time_it([&] { c->launches += launch_ibatch32(c, x, y, R, master, st); });
+  if (ib32_usable(c, R, st)) {
+    ms_batched = time_it([&] { ib_run(c, [&] { return launch_ibatch32(c, x, y, R, master, st); }); });
+    if (c->ib.refused) ms_batched = -1.f;
+  }
   // the tensor-core operators (3xTF32, accumulators drained every few emitters)
   float ms_tc = -1.f, ms_tcs = -1.f;
   if (tcsym_supported(c, R))
@@ -1249,10 +1264,8 @@ void apply_padded(sg_context *c, const double2 *x, double2 *y, int R, bool maste
       batched = c->tuned.back().batched;
     }
   }
-  if (variant == 0 && !fp32 && ib_usable(c, R, st)) {
-    c->launches += launch_ibatch(c, x, y, R, master, st);
-  } else if (batched && ib32_usable(c, R, st)) {
-    c->launches += launch_ibatch32(c, x, y, R, master, st);
+  if (variant == 0 && !fp32 && ib_usable(c, R, st) && ib_run(c, [&] { return launch_ibatch(c, x, y, R, master, st); })) {
+  } else if (batched && ib32_usable(c, R, st) && ib_run(c, [&] { return launch_ibatch32(c, x, y, R, master, st); })) {
   } else if (variant == 5) {
     c->launches += launch_tcsym_matvec(c, x, y, R, master, st);
   } else if (variant == 4) {
@@ -1317,9 +1330,10 @@ void apply_padded_df64(sg_context *c, const double2 *x, double2 *y, int R, bool 
   };
   if (ib_usable(c, R, st)) {
     mark(e0);
-    c->launches += launch_ibatch(c, x, y, R, master, st);
-    done();
-    return;
+    if (ib_run(c, [&] { return launch_ibatch(c, x, y, R, master, st); })) {
+      done();
+      return;
+    }
   }
   const size_t ncoef_total = (size_t)c->n_int * c->ncoef * c->bs * c->bs;
   if (!c->df_ready && capturing(st)) {  // its coefficients cannot be kept from there: the FP64 kernel

@@ -881,7 +881,6 @@ __global__ void __launch_bounds__(256) ib_operand_kernel(const double2 *coef, co
 static constexpr int kIbMinParticles = 32;
 static constexpr long long kIbMaxPairs = 1ll << 27;      // 4 GB of pair records
 static constexpr size_t kIbMaxOperands = (size_t)32 << 30;  // bytes of the intervals' B operands
-static constexpr size_t kIbWorkspace = (size_t)2 << 30;  // bytes of V per chunk
 
 // padded blocksize
 static int ib_kp(const sg_context *c) { return c->bs <= IbNumbers<32>::MAXB ? 32 : 48; }
@@ -902,8 +901,28 @@ static void ib_dispatch(const sg_context *c, F &&f) {
   }
 }
 
+void ib_drop(sg_context *c) {
+  auto &P = c->ib;
+  P.ready = P.digits_ready = P.halves_ready = P.captured = false;
+  P.tiles.clear();
+  P.rec.release();
+  P.slot.release();
+  P.bk.release();
+  P.boff.release();
+  P.exps.release();
+  P.err.release();
+  P.B.release();
+  P.H.release();
+  P.xh.release();
+  P.top.release();
+  P.V.release();
+  P.acc.release();
+  P.xw.release();
+  P.xe.release();
+}
+
 bool ib_supported(const sg_context *c) {
-  if (c->vol || c->kind < 0 || c->bs > IbNumbers<48>::MAXB) return false;
+  if (c->vol || c->kind < 0 || c->ib.refused || c->bs > IbNumbers<48>::MAXB) return false;
   const long long pairs = (long long)c->n * c->n;
   if (pairs > kIbMaxPairs || c->n < kIbMinParticles) return false;
   size_t operand = 0;
@@ -938,8 +957,8 @@ void ib_plan(sg_context *c, cudaStream_t st) {
   SG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys.ptr, keys2.ptr, vals.ptr, vals2.ptr, np, 0, bits, st));
   tmp.reserve(bytes);
   SG_CUDA(cub::DeviceRadixSort::SortPairs(tmp.ptr, bytes, keys.ptr, keys2.ptr, vals.ptr, vals2.ptr, np, 0, bits, st));
-  P.rec.reserve(np);
-  P.slot.reserve(np);
+  P.take(P.rec, np);
+  P.take(P.slot, np);
   ib_records_kernel<<<grid, 256, 0, st>>>(c->pos.ptr, n, c->rho_min, c->res, n_int, vals2.ptr, P.rec.ptr, P.slot.ptr);
   SG_CUDA(cudaGetLastError());
   std::vector<int> cnt(n_int);
@@ -953,11 +972,11 @@ void ib_plan(sg_context *c, cudaStream_t st) {
       P.h_boff.push_back(P.h_boff.back() + cnt[k]);
     }
   P.nb = (int)bk.size();
-  P.bk.reserve(P.nb);
-  P.boff.reserve(P.nb + 1);
+  P.take(P.bk, P.nb);
+  P.take(P.boff, P.nb + 1);
   SG_CUDA(cudaMemcpyAsync(P.bk.ptr, bk.data(), P.nb * sizeof(int), cudaMemcpyHostToDevice, st));
   SG_CUDA(cudaMemcpyAsync(P.boff.ptr, P.h_boff.data(), (P.nb + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-  P.err.reserve(1);
+  P.take(P.err, 1);
   SG_CUDA(cudaMemsetAsync(P.err.ptr, 0, sizeof(int), st));
   SG_CUDA(cudaStreamSynchronize(st));  // the temporaries are released on return
   P.tiles.clear();
@@ -969,10 +988,10 @@ void ib_plan(sg_context *c, cudaStream_t st) {
 static void ib_digit_operands(sg_context *c, cudaStream_t st) {
   auto &P = c->ib;
   if (P.digits_ready) return;
-  P.exps.reserve((size_t)P.nb * 2 * ib_kp(c));
+  P.take(P.exps, (size_t)P.nb * 2 * ib_kp(c));
   ib_dispatch(c, [&](auto nc, auto kp) {
     constexpr int NC = decltype(nc)::value, KP = decltype(kp)::value;
-    P.B.reserve((size_t)P.nb * IbShape<NC, KP>::BBYTES);
+    P.take(P.B, (size_t)P.nb * IbShape<NC, KP>::BBYTES);
     ib_operand_kernel<NC, KP><<<P.nb, 256, 0, st>>>(c->coef64.ptr, P.bk.ptr, c->bs, P.B.ptr, P.exps.ptr);
   });
   SG_CUDA(cudaGetLastError());
@@ -988,6 +1007,7 @@ void ib_enter(sg_context *c, cudaStream_t st) {
     const cudaError_t e = cudaEventSynchronize(P.done);
     SG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     SG_CUDA(e);
+    P.captured = true;
     return;
   }
   if (!P.done) SG_CUDA(cudaEventCreateWithFlags(&P.done, cudaEventDisableTiming));
@@ -1019,7 +1039,7 @@ sg_context::IbTiles &ib_tiles(sg_context *c, int rt, int sets, cudaStream_t st) 
   t->h_toff.assign(1, 0);
   for (int b = 0; b < P.nb; ++b)
     t->h_toff.push_back(t->h_toff.back() + (P.h_boff[b + 1] - P.h_boff[b] + per - 1) / per);
-  t->toff.reserve(t->h_toff.size());
+  P.take(t->toff, t->h_toff.size());
   SG_CUDA(cudaMemcpyAsync(t->toff.ptr, t->h_toff.data(), t->h_toff.size() * sizeof(int), cudaMemcpyHostToDevice, st));
   SG_CUDA(cudaStreamSynchronize(st));
   P.tiles.push_back(std::move(t));
@@ -1038,7 +1058,7 @@ bool ib_has_tiles(const sg_context *c, int rt, int sets) {
 // (7.7 GB) 334 / 334 / 374.
 int ib_group(const sg_context *c, int R) {
   const size_t row = (size_t)c->n * c->n * c->bs * sizeof(double2);
-  return std::min(R, (int)std::min<size_t>(16, std::max<size_t>(1, 4 * kIbWorkspace / row)));
+  return std::min(R, (int)std::min<size_t>(16, std::max<size_t>(1, 4 * c->ib.workspace / row)));
 }
 
 bool ib_prepared(const sg_context *c, int R) {
@@ -1086,9 +1106,9 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     const int per = tl.per;
     const size_t pair_bytes = (size_t)rt * bs * sizeof(double2);
     const int ntiles = tl.h_toff.back();
-    const int chunk = (int)std::min<size_t>(ntiles, std::max<size_t>(1, kIbWorkspace / (pair_bytes * per)));
-    double2 *V = mem.get(P.V, (size_t)std::min<long long>((long long)chunk * per, (long long)c->n * c->n) * rt * bs);
-    if (chunk < ntiles && !acc) acc = mem.get(P.acc, (size_t)c->n * bs * R);
+    const int chunk = (int)std::min<size_t>(ntiles, std::max<size_t>(1, c->ib.workspace / (pair_bytes * per)));
+    double2 *V = ib_scratch(c, mem, P.V, (size_t)std::min<long long>((long long)chunk * per, (long long)c->n * c->n) * rt * bs);
+    if (chunk < ntiles && !acc) acc = ib_scratch(c, mem, P.acc, (size_t)c->n * bs * R);
     auto first_pair = [&](int t) -> long long {  // first pair of tile t
       const int b = (int)(std::upper_bound(tl.h_toff.begin(), tl.h_toff.end(), t) - tl.h_toff.begin()) - 1;
       if (b >= P.nb) return (long long)c->n * c->n;
@@ -1101,8 +1121,8 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     a.B = P.B.ptr;
     a.exps = P.exps.ptr;
     const size_t words = (size_t)c->n * rt * ib_kp(c);
-    int4 *xw = mem.get(P.xw, words);
-    int *xe = mem.get(P.xe, words);
+    int4 *xw = ib_scratch(c, mem, P.xw, words);
+    int *xe = ib_scratch(c, mem, P.xe, words);
     (ib_kp(c) == 32 ? ib_words_kernel<32> : ib_words_kernel<48>)<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(
         x, c->n, bs, R, r0, rt, xw, xe);
     SG_CUDA(cudaGetLastError());
@@ -1157,3 +1177,10 @@ bool ib_check_error(sg_context *c, cudaStream_t st) {
 }
 
 }  // namespace sg
+
+size_t sg_context::Ib::bytes() const {
+  size_t n = rec.n * sizeof(sg::IbRec) + (slot.n + bk.n + boff.n + exps.n + err.n + top.n + xe.n) * 4 + B.n + H.n +
+             xh.n * sizeof(float2) + (V.n + acc.n) * sizeof(double2) + xw.n * sizeof(int4);
+  for (const auto &t : tiles) n += t->toff.n * 4;
+  return n;
+}

@@ -36,6 +36,12 @@ __device__ __forceinline__ void ib_exponents(const double2 *C, int bs, int *eb, 
 void ib_plan(sg_context *c, cudaStream_t st);
 // tiles for rt right-hand sides; sets = 0: chosen for the FP64 operator
 sg_context::IbTiles &ib_tiles(sg_context *c, int rt, int sets, cudaStream_t st);
+// scratch memory of a call, within the limit
+template <typename T>
+T *ib_scratch(sg_context *c, CallMemory &mem, DevBuf<T> &kept, size_t count) {
+  if (!mem.graph) c->ib.take(kept, count);
+  return mem.get(kept, count);
+}
 // the tiles exist
 bool ib_has_tiles(const sg_context *c, int rt, int sets);
 // right-hand sides of the FP64 operator at a time

@@ -580,10 +580,10 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
   const int bs = c->bs, kp = bs <= 32 ? 32 : 48;
   int launched = 0;
   if (!P.halves_ready) {
-    P.exps.reserve((size_t)P.nb * 2 * kp);
+    P.take(P.exps, (size_t)P.nb * 2 * kp);
     ih_dispatch(c, [&](auto nc, auto kpc) {
       constexpr int NC = decltype(nc)::value, KP = decltype(kpc)::value;
-      P.H.reserve((size_t)P.nb * IhShape<NC, KP>::BBYTES);
+      P.take(P.H, (size_t)P.nb * IhShape<NC, KP>::BBYTES);
       ih_operand_kernel<NC, KP><<<P.nb, 256, 0, st>>>(c->coef64.ptr, P.bk.ptr, bs, P.H.ptr, P.exps.ptr);
     });
     SG_CUDA(cudaGetLastError());
@@ -593,7 +593,7 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
   const size_t len = (size_t)c->n * bs * R;
   float2 *yacc = mem.get(c->sym_yacc, len);
   SG_CUDA(cudaMemsetAsync(yacc, 0, len * sizeof(float2), st));
-  int *top = mem.get(P.top, 256);
+  int *top = ib_scratch(c, mem, P.top, 256);
   SG_CUDA(cudaMemsetAsync(top, 0, R * sizeof(int), st));
   const size_t rows = (size_t)c->n * bs;
   ih_top_kernel<<<(unsigned)std::min<size_t>((rows * R + 2047) / 2048, (size_t)sm_count() * 4), 256, 0, st>>>(x, rows, R, top);
@@ -612,8 +612,8 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
   a.err = P.err.ptr;
   for (int m : c->h_mofn) a.mmax = std::max(a.mmax, std::abs(m));
   const int chunks = ih_chunks(c->n);
-  double2 *total = chunks > 1 ? mem.get(P.acc, len) : nullptr;
-  float2 *xh = mem.get(P.xh, (size_t)c->n * kp * std::min(16, R));
+  double2 *total = chunks > 1 ? ib_scratch(c, mem, P.acc, len) : nullptr;
+  float2 *xh = ib_scratch(c, mem, P.xh, (size_t)c->n * kp * std::min(16, R));
   for (int r0 = 0; r0 < R; r0 += 16) {
     a.r0 = r0;
     a.rt = std::min(16, R - r0);

@@ -25,6 +25,11 @@ struct Error {
   std::string msg;
 };
 
+// a device allocation that failed, or that the caller's limit does not allow
+struct NoMemory : Error {
+  explicit NoMemory(size_t bytes) : Error{SG_ERR_CUDA, "out of device memory: " + std::to_string(bytes) + " bytes"} {}
+};
+
 #define SG_CUDA(call)                                                                          \
   do {                                                                                         \
     cudaError_t e_ = (call);                                                                   \
@@ -56,7 +61,13 @@ struct DevBuf {
     if (count <= n && ptr) return;
     release();
     if (count == 0) return;
-    SG_CUDA(cudaMalloc(&ptr, count * sizeof(T)));
+    const cudaError_t e = cudaMalloc(&ptr, count * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      ptr = nullptr;
+      throw NoMemory(count * sizeof(T));
+    }
+    SG_CUDA(e);
     n = count;
   }
 };
@@ -183,6 +194,7 @@ bool ib32_prepared(const sg_context *c, int R);
 int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 bool ib_check_error(sg_context *c, cudaStream_t st);  // reads and clears the timeout flag (synchronises)
+void ib_drop(sg_context *c);                          // gives back what the interval-batched operators hold
 struct IbRec {  // one ordered pair: fraction within its interval, direction, receiver i and emitter j
   double t, c, s;
   int i, j;
@@ -352,8 +364,8 @@ struct sg_context {
   sg::DevBuf<int> sym_err;  // set when a bounded wait of the pair-symmetric kernel ran out
   bool sym_err_init = false;
 
-  // interval-batched FP64 operator (sg_ibatch.cu): ordered pairs sorted by lookup interval, the
-  // intervals' digit operands, the pairs' contributions V of one chunk
+  // interval-batched operators (sg_ibatch.cu, sg_ibatch32.cu): ordered pairs sorted by lookup interval, the
+  // intervals' operands, the pairs' contributions V of one chunk
   struct IbTiles {
     int rt = 0, asked = 0, sets = 1, per = 0;  // right-hand sides; sets of warps, asked for (0: none) and taken; pairs per tile
     std::vector<int> h_toff;
@@ -373,6 +385,17 @@ struct sg_context {
     sg::DevBuf<int4> xw;  // words of x and their exponents
     sg::DevBuf<int> xe;
     std::vector<std::unique_ptr<IbTiles>> tiles;
+    size_t limit = 0;                       // bytes that all of the above may hold (0: no limit)
+    size_t workspace = (size_t)2 << 30;     // bytes of V per chunk
+    bool captured = false;                  // a graph uses the plan, which therefore stays
+    bool refused = false;                   // they did not fit: the other kernels until the next particles, lookup or limit
+    size_t bytes() const;
+    template <typename T>
+    void take(sg::DevBuf<T> &b, size_t count) {
+      const size_t held = b.n * sizeof(T), want = count * sizeof(T);
+      if (limit && want > held && bytes() - held + want > limit) throw sg::NoMemory(want);
+      b.reserve(count);
+    }
     cudaEvent_t done = nullptr;  // end of the last call: calls on other streams wait for it
     ~Ib() {
       if (done) cudaEventDestroy(done);

@@ -119,3 +119,72 @@ def test_fp32_sums_in_chunks(n, bs, R, gpu_context):
     ref = np.einsum("ijab,jbr->iar", w, x)
     for r in range(R):
         assert np.linalg.norm(y[rows, :, r] - ref[..., r]) <= 4.4e-6 * np.linalg.norm(ref[..., r])
+
+
+def _launches(ctx, x, precision):
+    before = ctx.launch_count()
+    y = ctx.coupling_matvec(x, precision)
+    return y, ctx.launch_count() - before
+
+
+@pytest.mark.parametrize("n,bs,R,kind", [(101, 30, 16, "linear"), (64, 30, 19, "cubic"), (50, 48, 3, "cubic"), (33, 7, 1, "linear")])
+def test_chunks_of_the_workspace(n, bs, R, kind, gpu_context):
+    """A workspace far below the contributions: many chunks of tiles, with edges inside intervals, groups of right-hand
+    sides and a remainder. Bound as in test_gpu_ibatch.py."""
+    from test_gpu_ibatch import _direct, _system
+    xy, m, rho, table = _system(gpu_context, n, bs, kind, 100 * n + bs)
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, bs, R)) + 1j * rng.standard_normal((n, bs, R))
+    ref = _direct(xy, m, rho, table, kind, x)
+    try:
+        for workspace in (1, 300_000, 1_000_000):
+            gpu_context.batched_memory(0, workspace)
+            y, launches = _launches(gpu_context, x.reshape(n * bs, R), _lib.SG_FP64)
+            assert launches >= 2 * n * n * bs * R * 16 // max(workspace, 128 * bs * 16)
+            y = y.reshape(n, bs, R)
+            for r in range(R):
+                assert np.linalg.norm(y[..., r] - ref[..., r]) <= 1e-13 * np.linalg.norm(ref[..., r])
+    finally:
+        gpu_context.batched_memory()
+
+
+@pytest.mark.parametrize("precision,R,tol", [(_lib.SG_FP64, 2, 1e-13), (_lib.SG_DF64, 2, 1e-12), (_lib.SG_FP32, 16, 2e-5)])
+def test_memory_that_cannot_be_had(precision, R, tol, gpu_context):
+    """Wherever an allocation of the batched operators fails, from the first to the last, the product comes from
+    another kernel; what fits takes them again. Bounds as elsewhere (double-float 1e-12, FP32 kernels 2e-5)."""
+    from test_gpu_ibatch import _direct, _system
+    n, bs = 110, 30
+    xy, m, rho, table = _system(gpu_context, n, bs, "linear", 5)
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, bs, R)) + 1j * rng.standard_normal((n, bs, R))
+    ref = _direct(xy, m, rho, table, "linear", x)
+    x, ref = x.reshape(n * bs, R), ref.reshape(n * bs, R)
+    try:
+        seen = set()
+        for limit in list(np.geomspace(1e3, 1e9, 60).astype(np.int64)) + [0]:
+            gpu_context.batched_memory(limit)
+            if precision == _lib.SG_FP32:
+                gpu_context.fp32_batched(R, take=True)
+            for _ in range(2):
+                y, launches = _launches(gpu_context, x, precision)
+                assert np.linalg.norm(y - ref) <= tol * np.linalg.norm(ref)
+            seen.add(launches if precision == _lib.SG_FP32 else y.tobytes())  # FP64-grade products repeat exactly
+        assert len(seen) == 2, "both routes were taken"
+    finally:
+        gpu_context.batched_memory()
+
+
+def test_autotuner_without_memory(gpu_context):
+    """The FP32 autotuner drops the batched operator where it does not fit, and keeps the others."""
+    from test_gpu_ibatch import _direct, _system
+    n, bs, R = 330, 30, 16
+    xy, m, rho, table = _system(gpu_context, n, bs, "linear", 6)
+    x = np.random.default_rng(n).standard_normal((n * bs, R)) + 0j
+    try:
+        gpu_context.batched_memory(1000)
+        y = gpu_context.coupling_matvec(x, _lib.SG_FP32)
+        assert gpu_context.fp32_batched(R) == (False, -1.0) and gpu_context.fp32_autotune(R)[0] >= 0
+        ref = _direct(xy, m, rho, table, "linear", x.reshape(n, bs, R)).reshape(n * bs, R)
+        assert np.linalg.norm(y - ref) <= 2e-5 * np.linalg.norm(ref)
+    finally:
+        gpu_context.batched_memory()
