@@ -1142,8 +1142,7 @@ static bool ib_run(sg_context *c, F &&f) {
 static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   // Candidates, each warmed once (first launches carry one-time set-up) and timed once with CUDA events on the live
   // operands; the ones that are fastest with many right-hand sides come first, and a candidate whose first run
-  // already takes over three times the fastest (and 5 ms for its set-up) is not run again. First product of a new state
-  // with all of them run twice and now: 2000 spheres, 16 right-hand sides 540 -> 407 ms; 1500, l_max 4, 64: 4.5 -> 2.3 s.
+  // already takes over three times the fastest (and 5 ms for its set-up) is not run again.
   cudaEvent_t e0, e1;
   SG_CUDA(cudaEventCreate(&e0));
   SG_CUDA(cudaEventCreate(&e1));
@@ -1161,14 +1160,6 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
     if (fastest < 0.f || ms < fastest) fastest = ms;
     return ms;
   };
-  // The interval-batched operator replaces the tensor-core ones, whose error is larger (2000 spheres, 16 right-hand
-  // sides: 4.5e-7 against 2.7e-7; 13.6 against 7.2 ms); where an FP32-pipe kernel wins, that one rounds better
-  // (100 spheres: 4.5e-8 against 5.6e-8) and stays.
-  float ms_batched = -1.f;
-  if (ib32_usable(c, R, st)) {
-    ms_batched = time_it([&] { ib_run(c, [&] { return launch_ibatch32(c, x, y, R, master, st); }); });
-    if (c->ib.refused) ms_batched = -1.f;
-  }
   // the tensor-core operators (3xTF32, accumulators drained every few emitters)
   float ms_tc = -1.f, ms_tcs = -1.f;
   if (tcsym_supported(c, R))
@@ -1210,8 +1201,6 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
   }
   float ms_bucket = -1.f;
   if (c->use_bucket) ms_bucket = time_it([&] { c->launches += launch_bucket_matvec(c, x, y, R, master, st); });
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   int v = 0;
   float best = best_rec;
   if (ms_bucket >= 0.f && ms_bucket < best) {
@@ -1230,8 +1219,23 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
     v = 5;
     best = ms_tcs;
   }
-  c->tuned.push_back({R, v, best_rt, best_rec, ms_bucket, sym_rt, ms_sym, ms_tc, ms_tcs, ms_batched,
-                      v >= 4 && ms_batched >= 0.f && ms_batched < best});
+  // The interval-batched operator replaces the tensor-core ones, whose error is larger (2000 spheres, 16 right-hand
+  // sides: 1.4e-6 against 4.4e-7; 13.6 against 7.3 ms); where an FP32-pipe kernel wins, that one rounds better
+  // (100 spheres: 4.5e-8 against 5.6e-8) and stays. So it is timed only after one of them has won, and never decides how
+  // often the others are run.
+  float ms_batched = -1.f;
+  bool batched = false;
+  if (v >= 4 && ib32_usable(c, R, st)) {
+    ms_batched = time_it([&] { ib_run(c, [&] { return launch_ibatch32(c, x, y, R, master, st); }); });
+    if (c->ib.refused) ms_batched = -1.f;
+    batched = ms_batched >= 0.f && ms_batched < best;
+    bool used = batched || c->ib.captured;
+    for (const auto &t : c->tuned) used = used || t.batched;
+    if (!used) ib_drop_halves(c);
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  c->tuned.push_back({R, v, best_rt, best_rec, ms_bucket, sym_rt, ms_sym, ms_tc, ms_tcs, ms_batched, batched});
   return v;
 }
 

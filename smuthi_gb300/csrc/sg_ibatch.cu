@@ -921,6 +921,14 @@ void ib_drop(sg_context *c) {
   P.xe.release();
 }
 
+void ib_drop_halves(sg_context *c) {
+  auto &P = c->ib;
+  if (!P.digits_ready) return ib_drop(c);
+  P.halves_ready = false;
+  P.H.release();
+  P.xh.release();
+}
+
 bool ib_supported(const sg_context *c) {
   if (c->vol || c->kind < 0 || c->ib.refused || c->bs > IbNumbers<48>::MAXB) return false;
   const long long pairs = (long long)c->n * c->n;

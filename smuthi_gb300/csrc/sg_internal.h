@@ -195,6 +195,7 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
 int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st);
 bool ib_check_error(sg_context *c, cudaStream_t st);  // reads and clears the timeout flag (synchronises)
 void ib_drop(sg_context *c);                          // gives back what the interval-batched operators hold
+void ib_drop_halves(sg_context *c);                   // what the FP32 one alone holds
 struct IbRec {  // one ordered pair: fraction within its interval, direction, receiver i and emitter j
   double t, c, s;
   int i, j;
