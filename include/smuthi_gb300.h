@@ -47,7 +47,7 @@ extern "C" {
  * sg_precond_select; a correction solve that fails to reduce its residual is redone without it */
 #define SG_PRECOND 4
 /* FP64-grade operator: with the radial lookup, 32 particles or more and blocksize <= 48 the
- * interval-batched operator that SG_FP64 uses; otherwise double-float arithmetic: every sum in two FP32
+ * kernel that SG_FP64 uses; otherwise double-float arithmetic: every sum in two FP32
  * words (about 48 significant bits) on the FP32 pipe, with the FP64 table split into two FP32 words (it
  * agrees with SG_FP64 to ~1e-13 relative). OR-ed into sg_gmres_solve's precision with SG_FP32, the
  * refinement's true residuals use it. No counterpart in the reference. */
@@ -205,6 +205,11 @@ int sg_fp32_set_kernel(sg_context *ctx, int nrhs, int variant, int rhs_tile);
  * or more, blocksize <= 30 or 33 to 48) until the next set_particles, set_lookup or sg_fp32_set_kernel. No
  * counterpart in the reference. */
 int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms);
+
+/* Kernel of the FP64-grade products with the radial lookup: 0 = the faster one by size and grid (default), 1 = the
+ * interval-batched one wherever it applies, 2 = the per-receiver ones (SG_FP64 in FP64, SG_DF64 in double-float). For
+ * tests and measurements of one kernel; no counterpart in the reference. */
+int sg_fp64_set_kernel(sg_context *ctx, int kernel);
 
 /* Device memory of the interval-batched operators: at most `limit` bytes for plan, operands and workspaces (0: no
  * limit), of which `workspace` (0: 2 GiB) for the contributions that are formed at a time, larger problems running in

@@ -28,7 +28,7 @@ EXPORTS = ("sg_last_error", "sg_version", "sg_create", "sg_destroy", "sg_set_par
            "sg_set_tmatrix", "sg_coupling_matvec", "sg_master_matvec", "sg_coupling_matvec_dev",
            "sg_master_matvec_dev", "sg_gmres_solve", "sg_gmres_solve_dev", "sg_true_residual", "sg_profile",
            "sg_kernel_timing", "sg_launch_count", "sg_measure_fma_peak", "sg_fp32_autotune", "sg_fp32_set_kernel",
-           "sg_fp32_batched", "sg_batched_memory",
+           "sg_fp32_batched", "sg_batched_memory", "sg_fp64_set_kernel",
            "sg_tc_set_window", "sg_coupling_matvec_linear_noalloc", "sg_precond_param_count", "sg_precond_add_graph",
            "sg_precond_select", "sg_precond_clear", "sg_precond_set_params", "sg_precond_get_params",
            "sg_precond_apply_dev", "sg_precond_train_step", "sg_precond_export_blocks", "sg_bessel_jac_table",
@@ -92,6 +92,7 @@ def _declare(L):
                              ctypes.POINTER(_D), ctypes.POINTER(_D), ctypes.POINTER(_D)],
         "sg_fp32_set_kernel": [_P, _I, _I, _I],
         "sg_fp32_batched": [_P, _I, _I, ctypes.POINTER(_I), ctypes.POINTER(_D)],
+        "sg_fp64_set_kernel": [_P, _I],
         "sg_batched_memory": [_P, ctypes.c_size_t, ctypes.c_size_t],
         "sg_tc_set_window": [_P, _I],
         "sg_plane_wave_swe": [_P, _I, _P, _I, _I, _P, _I, _P, _P, _P],
@@ -284,6 +285,10 @@ class Context:
         on, ms = ctypes.c_int(), ctypes.c_double()
         check(lib().sg_fp32_batched(self.h, int(nrhs), int(take), ctypes.byref(on), ctypes.byref(ms)))
         return bool(on.value), ms.value
+
+    def fp64_set_kernel(self, kernel=0):
+        """Kernel of FP64-grade products (0 the faster one, 1 interval-batched, 2 per-receiver: FP64 or double-float)."""
+        check(lib().sg_fp64_set_kernel(self.h, int(kernel)))
 
     def batched_memory(self, limit=0, workspace=0):
         """Bytes of device memory for the interval-batched operators (0: no limit) and for the contributions they form at

@@ -212,6 +212,7 @@ int sg_set_lookup(sg_context *ctx, int kind, int len_rho, double rho_min, double
     ctx->res = resolution;
     ctx->pairs_ready = false;
     ctx->ib.ready = ctx->ib.refused = ctx->ib.captured = false;
+    sg::ib_count_pairs(ctx, pos.data());
     ctx->df_ready = false;
     ctx->tuned_df.clear();
     ctx->pgraphs.clear();  // their near-field blocks came from the old table
@@ -649,6 +650,15 @@ int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms)
   });
 }
 
+int sg_fp64_set_kernel(sg_context *ctx, int kernel) {
+  return guarded([&]() -> int {
+    SG_REQUIRE(ctx, "null context");
+    SG_REQUIRE(kernel >= 0 && kernel <= 2, "kernel must be 0, 1 or 2");
+    ctx->fp64_kernel = kernel;
+    return SG_OK;
+  });
+}
+
 int sg_batched_memory(sg_context *ctx, size_t limit, size_t workspace) {
   return guarded([&]() -> int {
     SG_REQUIRE(ctx, "null context");
@@ -657,6 +667,7 @@ int sg_batched_memory(sg_context *ctx, size_t limit, size_t workspace) {
     P.limit = limit;
     P.workspace = workspace ? workspace : (size_t)2 << 30;
     P.refused = false;
+    P.pays.clear();
     sg::ib_drop(ctx);
     return SG_OK;
   });

@@ -1116,9 +1116,13 @@ static void launch_receiver(sg_context *c, const double2 *x, double2 *y, int R, 
   c->launches += launch_coupling(L, fp32, ns, st);
 }
 
+// FP64-grade products: the kernel that the caller has fixed, or the faster one
+static bool ib_wanted(sg_context *c, int R) {
+  return ib_supported(c) && (c->fp64_kernel == 1 || (c->fp64_kernel == 0 && ib_pays(c, R)));
+}
 // Under stream capture the interval-batched operators need what an earlier call prepared; otherwise the other kernels run.
-static bool ib_usable(const sg_context *c, int R, cudaStream_t st) {
-  return ib_supported(c) && (!capturing(st) || ib_prepared(c, R));
+static bool ib_usable(sg_context *c, int R, cudaStream_t st) {
+  return ib_wanted(c, R) && (!capturing(st) || ib_prepared(c, R));
 }
 static bool ib32_usable(const sg_context *c, int R, cudaStream_t st) {
   return ib32_supported(c, R) && (!capturing(st) || ib32_prepared(c, R));
@@ -1316,9 +1320,10 @@ static int df64_tile(sg_context *c, const double2 *x, double2 *y, int R, bool ma
   return best;
 }
 
-// The double-float operator is for what the interval-batched one does not take (sizes, stream capture): that one has
-// FP64 accuracy and is faster at every size, 16 right-hand sides with 2000 spheres 131 against 82 ms, with 100 0.41
-// against 0.22, one with 2000 24 against 5.2.
+// The double-float operator is for what the interval-batched one does not take. That one has FP64 accuracy (1e-15 of the
+// result against 4e-14) and is faster from about 200 spheres on: 16 right-hand sides with 2000 spheres 131 against 82 ms,
+// one 24 against 5.2. Smaller or sparser systems take the faster of it and the FP64 kernel, which keeps the accuracy;
+// the double-float kernel can be up to twice as fast there (100 spheres, 1 nm, cubic: 0.12 against 0.24 ms).
 void apply_padded_df64(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c->profiling) {
@@ -1340,7 +1345,8 @@ void apply_padded_df64(sg_context *c, const double2 *x, double2 *y, int R, bool 
     }
   }
   const size_t ncoef_total = (size_t)c->n_int * c->ncoef * c->bs * c->bs;
-  if (!c->df_ready && capturing(st)) {  // its coefficients cannot be kept from there: the FP64 kernel
+  const bool small = c->fp64_kernel == 0 && ib_supported(c) && !ib_pays(c, R);
+  if (small || (!c->df_ready && capturing(st))) {  // its coefficients cannot be kept from a capture
     mark(e0);
     launch_receiver(c, x, y, R, master, false, 0, st);
     done();

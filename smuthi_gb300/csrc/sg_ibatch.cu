@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(256) ib_operand_kernel(const double2 *coef, co
   }
 }
 
-static constexpr int kIbMinParticles = 32;
+static constexpr int kIbMinParticles = 32;  // down to here ib_pays has been measured
 static constexpr long long kIbMaxPairs = 1ll << 27;      // 4 GB of pair records
 static constexpr size_t kIbMaxOperands = (size_t)32 << 30;  // bytes of the intervals' B operands
 
@@ -940,6 +940,65 @@ bool ib_supported(const sg_context *c) {
   for (int m : c->h_mofn)
     if (m > mmax || m < -mmax) return false;
   return true;
+}
+
+// Beyond it the batched operator is the faster one however fine the lookup: 400 spheres on a 0.5 nm grid 0.72 ms against
+// 2.36, l_max = 1 0.70 against 0.90.
+static constexpr int kIbSmall = 640;
+
+void ib_count_pairs(sg_context *c, const double2 *pos) {
+  auto &P = c->ib;
+  P.h_counts.clear();
+  P.pays.clear();
+  const int n = c->n;
+  if (n < kIbMinParticles || n > kIbSmall) return;
+  std::vector<int> count(c->n_int, 0);
+  auto interval = [&](double rho) { return std::max(0, std::min(c->n_int - 1, (int)((rho - c->rho_min) / c->res))); };
+  count[interval(0.0)] += n;
+  for (int i = 0; i < n; ++i)
+    for (int j = i + 1; j < n; ++j) {
+      const double dx = pos[i].x - pos[j].x, dy = pos[i].y - pos[j].y;
+      count[interval(std::sqrt(dx * dx + dy * dy))] += 2;
+    }
+  for (int k : count)
+    if (k) P.h_counts.push_back(k);
+}
+
+// pairs per tile, and the sets of warps, for rt right-hand sides: tiles(per) counts them
+template <class F>
+static int ib_sets(int rt, F &&tiles) {
+  return 3 * tiles(kIbCols / 2 / rt) <= 4 * tiles(kIbCols / rt) ? 2 : 1;
+}
+
+// The batched operator's time goes by tiles, the per-receiver kernel's by pairs: few particles on a fine grid leave most
+// tiles with one pair. Both times in microseconds from 1364 products of 32 to 400 particles (l_max 1 to 4, grids of 0.5
+// to 5 nm, 1 to 16 right-hand sides), which they meet within a quarter. 32 spheres, 0.5 nm, linear: 51 us batched,
+// 25 per receiver; 100 spheres, 0.5 nm, cubic: 329 and 257, 1 nm: 237 and 257, 5 nm: 89 and 234.
+bool ib_pays(sg_context *c, int R) {
+  auto &P = c->ib;
+  if (c->n > kIbSmall) return true;
+  for (const auto &p : P.pays)
+    if (p.first == R) return p.second;
+  const int bs = c->bs, wide = (bs + 31) / 32, most = ib_group(c, R);
+  const int rows = kIbRows / c->ncoef, passes = (bs + rows - 1) / rows;
+  const double size = ib_kp(c) == 32 ? 1.0 : 1.65;
+  double batched = 0.0;
+  for (int r0 = 0, rt; r0 < R; r0 += rt) {
+    rt = std::min(most, R - r0);
+    auto tiles = [&](int per) {
+      long long t = 0;
+      for (int k : P.h_counts) t += (k + per - 1) / per;
+      return t;
+    };
+    const int sets = ib_sets(rt, tiles);
+    const double tile = size * (sets == 2 ? 3.0 + 6.5 * passes : 4.0 + 6.5 * passes + 0.2 * bs);
+    batched += 16.0 + 7.0 * passes * size + tile * tiles(kIbCols / sets / rt) / sm_count();
+  }
+  const double pairs = 1e-3 * c->n * c->n * 152 / sm_count();
+  const double receiver = wide * (0.35 * c->n + pairs * (2.3 + 0.129 * bs * (c->ncoef - 1) + 0.286 * bs * R));
+  const bool pays = receiver >= 0.95 * batched;
+  P.pays.push_back({R, pays});
+  return pays;
 }
 
 void ib_plan(sg_context *c, cudaStream_t st) {
@@ -1042,7 +1101,7 @@ sg_context::IbTiles &ib_tiles(sg_context *c, int rt, int sets, cudaStream_t st) 
   };
   t->rt = rt;
   t->asked = sets;
-  t->sets = sets ? sets : 3 * count(kIbCols / 2 / rt) <= 4 * count(kIbCols / rt) ? 2 : 1;
+  t->sets = sets ? sets : ib_sets(rt, count);
   const int per = t->per = kIbCols / t->sets / rt;
   t->h_toff.assign(1, 0);
   for (int b = 0; b < P.nb; ++b)

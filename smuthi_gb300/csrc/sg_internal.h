@@ -187,6 +187,8 @@ void solve_padded(sg_context *c, const double2 *b, double2 *x, int R, double rto
 void residual_norms(sg_context *c, const double2 *b, const double2 *x, int R, double *rel, cudaStream_t st);
 // FP64 operator batched by lookup interval on the tensor cores (sg_ibatch.cu)
 bool ib_supported(const sg_context *c);
+bool ib_pays(sg_context *c, int R);                             // faster than the per-receiver FP64 kernel
+void ib_count_pairs(sg_context *c, const double2 *pos);         // pairs per interval of a small system, for ib_pays
 bool ib32_supported(const sg_context *c, int R);
 // under stream capture they take only what an earlier call with as many right-hand sides has prepared
 bool ib_prepared(const sg_context *c, int R);
@@ -352,6 +354,7 @@ struct sg_context {
     bool batched = false;     // it replaces the variant
   };
   std::vector<Tuned> tuned;
+  int fp64_kernel = 0;  // FP64-grade products: 0 by size, 1 interval-batched, 2 per-receiver
   std::vector<std::pair<int, int>> tuned_df;  // double-float kernel: (nrhs, RHS tile)
   int bk_T = 0, bk_tiles = 0, bk_S = 0;
   sg::DevBuf<int> bk_members, bk_offs;
@@ -388,6 +391,8 @@ struct sg_context {
     std::vector<std::unique_ptr<IbTiles>> tiles;
     size_t limit = 0;                       // bytes that all of the above may hold (0: no limit)
     size_t workspace = (size_t)2 << 30;     // bytes of V per chunk
+    std::vector<int> h_counts;              // pairs of every non-empty interval (small systems)
+    std::vector<std::pair<int, bool>> pays; // ib_pays by right-hand sides
     bool captured = false;                  // a graph uses the plan, which therefore stays
     bool refused = false;                   // they did not fit: the other kernels until the next particles, lookup or limit
     size_t bytes() const;

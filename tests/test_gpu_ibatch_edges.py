@@ -9,6 +9,13 @@ from smuthi_gb300 import _lib
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def batched(gpu_context):
+    gpu_context.fp64_set_kernel(1)
+    yield
+    gpu_context.fp64_set_kernel()
+
+
 def _line(n, step, res, bs, seed, scale=1.0):
     """Particles on a line, `step` apart, and a smooth random table on a grid from zero."""
     rng = np.random.default_rng(seed)
