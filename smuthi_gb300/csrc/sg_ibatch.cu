@@ -907,10 +907,8 @@ void ib_drop(sg_context *c) {
   P.tiles.clear();
   P.rec.release();
   P.slot.release();
-  P.bk.release();
-  P.boff.release();
-  P.exps.release();
-  P.err.release();
+  P.ints.release();
+  P.tmp.release();
   P.B.release();
   P.H.release();
   P.xh.release();
@@ -1001,51 +999,58 @@ bool ib_pays(sg_context *c, int R) {
   return pays;
 }
 
+// Few allocations and one synchronisation: a first product is most of what a small system's program may ask for. The
+// sort's buffers stay for the next plan unless they are large. 100 spheres, linear: first product 0.43 ms with an
+// allocation of its own for every array and four synchronisations, 0.35 now, 0.20 on new particles of the same context
+// (0.24 before; the per-receiver kernel 0.19 and 0.18); 1000 spheres 2.12 and 1.70 (13.5).
+static constexpr size_t kIbKeep = (size_t)64 << 20;
+
 void ib_plan(sg_context *c, cudaStream_t st) {
   auto &P = c->ib;
   if (P.ready) return;
-  const int n = c->n, n_int = c->n_int;
+  const int n = c->n, n_int = c->n_int, kp = ib_kp(c);
   const size_t np = (size_t)n * n;
-  DevBuf<unsigned> keys, keys2, vals, vals2;
-  DevBuf<int> counts;
-  DevBuf<unsigned char> tmp;
-  keys.reserve(np);
-  keys2.reserve(np);
-  vals.reserve(np);
-  vals2.reserve(np);
-  counts.reserve(n_int);
-  SG_CUDA(cudaMemsetAsync(counts.ptr, 0, n_int * sizeof(int), st));
-  const unsigned grid = (unsigned)((np + 255) / 256);
-  ib_keys_kernel<<<grid, 256, 0, st>>>(c->pos.ptr, n, c->rho_min, c->res, n_int, keys.ptr, vals.ptr, counts.ptr);
-  SG_CUDA(cudaGetLastError());
   int bits = 1;
   while ((1 << bits) < n_int) ++bits;
   size_t bytes = 0;
-  SG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys.ptr, keys2.ptr, vals.ptr, vals2.ptr, np, 0, bits, st));
-  tmp.reserve(bytes);
-  SG_CUDA(cub::DeviceRadixSort::SortPairs(tmp.ptr, bytes, keys.ptr, keys2.ptr, vals.ptr, vals2.ptr, np, 0, bits, st));
+  unsigned *none = nullptr;
+  SG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, none, none, none, none, np, 0, bits, st));
+  const size_t part = (np * sizeof(unsigned) + 255) / 256 * 256, rest = (n_int * sizeof(int) + 255) / 256 * 256;
+  P.take(P.tmp, 4 * part + rest + bytes);
+  unsigned *keys = reinterpret_cast<unsigned *>(P.tmp.ptr), *keys2 = keys + part / 4, *vals = keys2 + part / 4,
+           *vals2 = vals + part / 4;
+  int *counts = reinterpret_cast<int *>(vals2 + part / 4);
+  SG_CUDA(cudaMemsetAsync(counts, 0, n_int * sizeof(int), st));
+  const unsigned grid = (unsigned)((np + 255) / 256);
+  ib_keys_kernel<<<grid, 256, 0, st>>>(c->pos.ptr, n, c->rho_min, c->res, n_int, keys, vals, counts);
+  SG_CUDA(cudaGetLastError());
+  SG_CUDA(cub::DeviceRadixSort::SortPairs(reinterpret_cast<unsigned char *>(counts) + rest, bytes, keys, keys2, vals, vals2, np,
+                                          0, bits, st));
   P.take(P.rec, np);
   P.take(P.slot, np);
-  ib_records_kernel<<<grid, 256, 0, st>>>(c->pos.ptr, n, c->rho_min, c->res, n_int, vals2.ptr, P.rec.ptr, P.slot.ptr);
+  ib_records_kernel<<<grid, 256, 0, st>>>(c->pos.ptr, n, c->rho_min, c->res, n_int, vals2, P.rec.ptr, P.slot.ptr);
   SG_CUDA(cudaGetLastError());
   std::vector<int> cnt(n_int);
-  SG_CUDA(cudaMemcpyAsync(cnt.data(), counts.ptr, n_int * sizeof(int), cudaMemcpyDeviceToHost, st));
+  SG_CUDA(cudaMemcpyAsync(cnt.data(), counts, n_int * sizeof(int), cudaMemcpyDeviceToHost, st));
   SG_CUDA(cudaStreamSynchronize(st));
-  std::vector<int> bk;
+  // intervals, first pairs, error flag (zero) and, filled with the operands, exponents
+  P.h_ints.clear();
   P.h_boff.assign(1, 0);
   for (int k = 0; k < n_int; ++k)
     if (cnt[k] > 0) {
-      bk.push_back(k);
+      P.h_ints.push_back(k);
       P.h_boff.push_back(P.h_boff.back() + cnt[k]);
     }
-  P.nb = (int)bk.size();
-  P.take(P.bk, P.nb);
-  P.take(P.boff, P.nb + 1);
-  SG_CUDA(cudaMemcpyAsync(P.bk.ptr, bk.data(), P.nb * sizeof(int), cudaMemcpyHostToDevice, st));
-  SG_CUDA(cudaMemcpyAsync(P.boff.ptr, P.h_boff.data(), (P.nb + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-  P.take(P.err, 1);
-  SG_CUDA(cudaMemsetAsync(P.err.ptr, 0, sizeof(int), st));
-  SG_CUDA(cudaStreamSynchronize(st));  // the temporaries are released on return
+  P.nb = (int)P.h_ints.size();
+  P.h_ints.insert(P.h_ints.end(), P.h_boff.begin(), P.h_boff.end());
+  P.h_ints.push_back(0);
+  P.take(P.ints, P.h_ints.size() + (size_t)P.nb * 2 * kp);
+  P.bk = P.ints.ptr;
+  P.boff = P.bk + P.nb;
+  P.err = P.boff + P.nb + 1;
+  P.exps = P.err + 1;
+  SG_CUDA(cudaMemcpyAsync(P.ints.ptr, P.h_ints.data(), P.h_ints.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+  if (P.tmp.n > kIbKeep) P.tmp.release();
   P.tiles.clear();
   c->launches += 2;
   P.ready = true;
@@ -1055,11 +1060,10 @@ void ib_plan(sg_context *c, cudaStream_t st) {
 static void ib_digit_operands(sg_context *c, cudaStream_t st) {
   auto &P = c->ib;
   if (P.digits_ready) return;
-  P.take(P.exps, (size_t)P.nb * 2 * ib_kp(c));
   ib_dispatch(c, [&](auto nc, auto kp) {
     constexpr int NC = decltype(nc)::value, KP = decltype(kp)::value;
     P.take(P.B, (size_t)P.nb * IbShape<NC, KP>::BBYTES);
-    ib_operand_kernel<NC, KP><<<P.nb, 256, 0, st>>>(c->coef64.ptr, P.bk.ptr, c->bs, P.B.ptr, P.exps.ptr);
+    ib_operand_kernel<NC, KP><<<P.nb, 256, 0, st>>>(c->coef64.ptr, P.bk, c->bs, P.B.ptr, P.exps);
   });
   SG_CUDA(cudaGetLastError());
   c->launches += 1;
@@ -1108,7 +1112,6 @@ sg_context::IbTiles &ib_tiles(sg_context *c, int rt, int sets, cudaStream_t st) 
     t->h_toff.push_back(t->h_toff.back() + (P.h_boff[b + 1] - P.h_boff[b] + per - 1) / per);
   P.take(t->toff, t->h_toff.size());
   SG_CUDA(cudaMemcpyAsync(t->toff.ptr, t->h_toff.data(), t->h_toff.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-  SG_CUDA(cudaStreamSynchronize(st));
   P.tiles.push_back(std::move(t));
   return *P.tiles.back();
 }
@@ -1183,10 +1186,10 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     };
     IbArgs a{};
     a.rec = P.rec.ptr;
-    a.boff = P.boff.ptr;
+    a.boff = P.boff;
     a.toff = tl.toff.ptr;
     a.B = P.B.ptr;
-    a.exps = P.exps.ptr;
+    a.exps = P.exps;
     const size_t words = (size_t)c->n * rt * ib_kp(c);
     int4 *xw = ib_scratch(c, mem, P.xw, words);
     int *xe = ib_scratch(c, mem, P.xe, words);
@@ -1203,12 +1206,12 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
     a.mmax = mmax;
     a.rt = rt;
     a.per = per;
-    a.err = P.err.ptr;
+    a.err = P.err;
     IbSum s{};
     s.V = V;
     s.slot = P.slot.ptr;
     s.acc = acc;
-    s.err = P.err.ptr;
+    s.err = P.err;
     s.rt = rt;
     s.r0 = r0;
     s.width = (bs * rt + 31) / 32 * 32;
@@ -1237,16 +1240,16 @@ int launch_ibatch(sg_context *c, const double2 *x, double2 *y, int R, bool maste
 bool ib_check_error(sg_context *c, cudaStream_t st) {
   if (!c->ib.ready) return false;
   int e = 0;
-  SG_CUDA(cudaMemcpyAsync(&e, c->ib.err.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  SG_CUDA(cudaMemcpyAsync(&e, c->ib.err, sizeof(int), cudaMemcpyDeviceToHost, st));
   SG_CUDA(cudaStreamSynchronize(st));
-  if (e) SG_CUDA(cudaMemsetAsync(c->ib.err.ptr, 0, sizeof(int), st));
+  if (e) SG_CUDA(cudaMemsetAsync(c->ib.err, 0, sizeof(int), st));
   return e != 0;
 }
 
 }  // namespace sg
 
 size_t sg_context::Ib::bytes() const {
-  size_t n = rec.n * sizeof(sg::IbRec) + (slot.n + bk.n + boff.n + exps.n + err.n + top.n + xe.n) * 4 + B.n + H.n +
+  size_t n = rec.n * sizeof(sg::IbRec) + (slot.n + ints.n + top.n + xe.n) * 4 + tmp.n + B.n + H.n +
              xh.n * sizeof(float2) + (V.n + acc.n) * sizeof(double2) + xw.n * sizeof(int4);
   for (const auto &t : tiles) n += t->toff.n * 4;
   return n;

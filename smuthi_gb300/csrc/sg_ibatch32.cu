@@ -580,11 +580,10 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
   const int bs = c->bs, kp = bs <= 32 ? 32 : 48;
   int launched = 0;
   if (!P.halves_ready) {
-    P.take(P.exps, (size_t)P.nb * 2 * kp);
     ih_dispatch(c, [&](auto nc, auto kpc) {
       constexpr int NC = decltype(nc)::value, KP = decltype(kpc)::value;
       P.take(P.H, (size_t)P.nb * IhShape<NC, KP>::BBYTES);
-      ih_operand_kernel<NC, KP><<<P.nb, 256, 0, st>>>(c->coef64.ptr, P.bk.ptr, bs, P.H.ptr, P.exps.ptr);
+      ih_operand_kernel<NC, KP><<<P.nb, 256, 0, st>>>(c->coef64.ptr, P.bk, bs, P.H.ptr, P.exps);
     });
     SG_CUDA(cudaGetLastError());
     ++launched;
@@ -601,15 +600,15 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
   ++launched;
   IhArgs a{};
   a.rec = P.rec.ptr;
-  a.boff = P.boff.ptr;
+  a.boff = P.boff;
   a.B = P.H.ptr;
-  a.exps = P.exps.ptr;
+  a.exps = P.exps;
   a.mofn = c->mofn.ptr;
   a.y = yacc;
   a.nb = P.nb;
   a.bs = bs;
   a.R = R;
-  a.err = P.err.ptr;
+  a.err = P.err;
   for (int m : c->h_mofn) a.mmax = std::max(a.mmax, std::abs(m));
   const int chunks = ih_chunks(c->n);
   double2 *total = chunks > 1 ? ib_scratch(c, mem, P.acc, len) : nullptr;
@@ -649,7 +648,7 @@ int launch_ibatch32(sg_context *c, const double2 *x, double2 *y, int R, bool mas
       }
     }
   }
-  launch_fp32_epilogue(c, x, y, R, master, st, top, P.err.ptr, yacc);
+  launch_fp32_epilogue(c, x, y, R, master, st, top, P.err, yacc);
   ib_leave(c, st);
   return launched + 1;
 }

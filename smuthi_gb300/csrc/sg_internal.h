@@ -378,10 +378,12 @@ struct sg_context {
   struct Ib {
     bool ready = false, digits_ready = false, halves_ready = false;
     int nb = 0;
-    std::vector<int> h_boff;
+    std::vector<int> h_boff, h_ints;
     sg::DevBuf<sg::IbRec> rec;
     sg::DevBuf<unsigned> slot;
-    sg::DevBuf<int> bk, boff, exps, err;
+    sg::DevBuf<int> ints;            // the next four
+    int *bk = nullptr, *boff = nullptr, *exps = nullptr, *err = nullptr;
+    sg::DevBuf<unsigned char> tmp;   // the sort's
     sg::DevBuf<unsigned char> B, H;  // operands: digits (FP64), FP16 halves (FP32)
     sg::DevBuf<float2> xh;           // FP32 copy of x for the FP32 form
     sg::DevBuf<int> top;             // its scales
