@@ -234,9 +234,10 @@ struct Solver {
     *launches += 2;
   }
 
-  // device scalars to the host (pinned, kept with the context)
+  // Device scalars to the host. The pinned buffer stays with the context and is made for the longest column at once:
+  // pinning costs as much as a small solve.
   const double2 *fetch(const double2 *d, size_t n) {
-    c->h_scalars.reserve(n);
+    c->h_scalars.reserve(std::max(n, (size_t)kHcol * R));
     SG_CUDA(cudaMemcpyAsync(c->h_scalars.ptr, d, n * sizeof(double2), cudaMemcpyDeviceToHost, st));
     SG_CUDA(cudaStreamSynchronize(st));
     return c->h_scalars.ptr;
