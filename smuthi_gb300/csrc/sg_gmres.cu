@@ -1147,7 +1147,8 @@ static bool ib_run(sg_context *c, F &&f) {
 static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, bool master, cudaStream_t st) {
   // Candidates, each warmed once (first launches carry one-time set-up) and timed once with CUDA events on the live
   // operands; the ones that are fastest with many right-hand sides come first, and a candidate whose first run
-  // already takes over three times the fastest (and 5 ms for its set-up) is not run again.
+  // already takes half as long again as the fastest, and 5 ms for its set-up, is not run again (first product of 2000
+  // spheres with 16 right-hand sides 395 ms; 514 up to three times the fastest).
   cudaEvent_t e0, e1;
   SG_CUDA(cudaEventCreate(&e0));
   SG_CUDA(cudaEventCreate(&e1));
@@ -1160,7 +1161,7 @@ static int autotune_fp32(sg_context *c, const double2 *x, double2 *y, int R, boo
       SG_CUDA(cudaEventRecord(e1, st));
       SG_CUDA(cudaEventSynchronize(e1));
       SG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-      if (run == 0 && fastest >= 0.f && ms > 3.f * fastest + 5.f) return ms;
+      if (run == 0 && fastest >= 0.f && ms > 1.5f * fastest + 5.f) return ms;
     }
     if (fastest < 0.f || ms < fastest) fastest = ms;
     return ms;
