@@ -756,10 +756,9 @@ int sg_farfield_sum_heights(sg_context *ctx, int n_particles, const void *xy, in
     SG_REQUIRE(ctx && xy && coef && m_of_n && kpar && S && alpha && out, "null argument");
     use_device(ctx);
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    sg::farfield_sum((const double2 *)xy, n_particles, blocksize, nrhs, (const double2 *)coef, m_max, m_of_n, nk,
-                     (const double *)kpar, (const double2 *)S, na, (const double *)alpha, (const double2 *)zphase,
-                     (double2 *)out, st);
-    ctx->launches += 1;
+    ctx->launches += sg::farfield_sum((const double2 *)xy, n_particles, blocksize, nrhs, (const double2 *)coef, m_max, m_of_n,
+                                      nk, (const double *)kpar, (const double2 *)S, na, (const double *)alpha,
+                                      (const double2 *)zphase, (double2 *)out, st);
     return SG_OK;
   });
 }

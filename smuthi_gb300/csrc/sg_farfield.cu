@@ -24,7 +24,7 @@
 // columns wide; more right-hand sides share each phase between four. (A tile of eight columns, with phase
 // times exp(i m alpha) formed per particle, spent 296 operations on one right-hand side's two columns: 1000
 // particles, l_max 3, 181 x 721 directions 69.8 ms; now 19.5.) Larger m_max takes the general kernel, whose
-// registers do not grow with m_max.
+// registers do not grow with m_max, and so do a few particles with many right-hand sides (ff_sum_per_m).
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -47,6 +47,7 @@ struct FfArgs {
   const int *moff;       // [nm + 1] CSR over m = -mmax..mmax of the n with that m
   const int *mlist;      // [B]
   const double2 *zph;    // [K][N] per-particle height factor, or null
+  const double2 *sc;     // sine table
   double2 *out;          // [R][2][K][A]
   int N, B, R, K, A, mmax;
 };
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(kFfThreads) ff_sum_m_kernel(const FfArgs f) {
   const double kap = f.kpar[k];
   double ca = 1.0, sa = 0.0;
   if (a < f.A) sincos(f.alpha[a], &sa, &ca);
-  sc_fill(T);
+  sc_load(f.sc, T);
   double2 F[NM][CT];
 #pragma unroll
   for (int m = 0; m < NM; ++m)
@@ -132,13 +133,18 @@ __global__ void __launch_bounds__(kFfThreads) ff_sum_m_kernel(const FfArgs f) {
 #pragma unroll
   for (int c = 0; c < CT; ++c) acc[c] = make_double2(0.0, 0.0);
 #pragma unroll
-  for (int m = 0; m < NM; ++m) {
-    double s, c;
-    sincos((double)(m - MM) * f.alpha[a], &s, &c);
+  for (int m = MM; m >= 0; --m) {  // m and -m share their sine and cosine
+    double s = 0.0, c = 1.0;
+    if (m > 0) sincos((double)m * f.alpha[a], &s, &c);
 #pragma unroll
-    for (int cc = 0; cc < CT; ++cc) {
-      acc[cc].x = fma(c, F[m][cc].x, fma(-s, F[m][cc].y, acc[cc].x));
-      acc[cc].y = fma(c, F[m][cc].y, fma(s, F[m][cc].x, acc[cc].y));
+    for (int h = 0; h < (m > 0 ? 2 : 1); ++h) {
+      const double sh = h ? s : -s;
+#pragma unroll
+      for (int cc = 0; cc < CT; ++cc) {
+        const double2 v = F[h ? MM + m : MM - m][cc];
+        acc[cc].x = fma(c, v.x, fma(-sh, v.y, acc[cc].x));
+        acc[cc].y = fma(c, v.y, fma(sh, v.x, acc[cc].y));
+      }
     }
   }
   ff_store<CT>(f, k, a, c0, acc);
@@ -210,7 +216,18 @@ static void ff_launch(const FfArgs &f, cudaStream_t st) {
   }
 }
 
-void farfield_sum(const double2 *xy, int n, int bs, int nrhs, const double2 *coef, int mmax, const int *mofn_host,
+// The kernel with one sum per m spends more once per direction and column tile (its tiles are half as wide), the general
+// one more per particle; FP64 operations of both. 16 right-hand sides, l_max 3, 181 x 721 directions: 1 particle 0.88 ms
+// against 0.66 with the general kernel, 5 1.80 against 1.69, 20 5.3 against 5.5; one right-hand side 0.25 against 0.30.
+static bool ff_sum_per_m(int n, int nrhs, int mmax) {
+  if (mmax > 4) return false;
+  const double nm = 2 * mmax + 1, ct = nrhs == 1 ? 2 : 4;
+  const int wide = (2 * nrhs + kFfCT - 1) / kFfCT, narrow = (2 * nrhs + (int)ct - 1) / (int)ct;
+  return narrow * (n * (19 + 4 * ct * nm) + 44 * mmax + 300) <= wide * (n * (44 + 38 * nm) + 44 * nm + 172);
+}
+
+// returns the number of kernels launched
+int farfield_sum(const double2 *xy, int n, int bs, int nrhs, const double2 *coef, int mmax, const int *mofn_host,
                   int nk, const double *kpar, const double2 *S, int na, const double *alpha, const double2 *zphase,
                   double2 *out, cudaStream_t st) {
   SG_REQUIRE(n >= 1 && bs >= 1 && nrhs >= 1 && nk >= 1 && na >= 1, "empty far-field problem");
@@ -224,13 +241,15 @@ void farfield_sum(const double2 *xy, int n, int bs, int nrhs, const double2 *coe
     }
     moff[mi + 1] = (int)mlist.size();
   }
-  DevBuf<int> d_moff, d_mlist;
-  d_moff.reserve(nm + 1);
-  d_mlist.reserve(bs);
-  SG_CUDA(cudaMemcpyAsync(d_moff.ptr, moff.data(), (nm + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-  SG_CUDA(cudaMemcpyAsync(d_mlist.ptr, mlist.data(), bs * sizeof(int), cudaMemcpyHostToDevice, st));
-  FfArgs f{xy, coef, S, kpar, alpha, d_moff.ptr, d_mlist.ptr, zphase, out, n, bs, nrhs, nk, na, mmax};
-  switch (mmax) {
+  moff.insert(moff.end(), mlist.begin(), mlist.end());
+  DevBuf<double2> scratch;  // sine table, then moff and mlist
+  scratch.reserve(kScTable + (moff.size() * sizeof(int) + sizeof(double2) - 1) / sizeof(double2));
+  int *d_moff = reinterpret_cast<int *>(scratch.ptr + kScTable);
+  SG_CUDA(cudaMemcpyAsync(d_moff, moff.data(), moff.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+  const bool per_m = ff_sum_per_m(n, nrhs, mmax);
+  if (per_m) sc_table(scratch.ptr, st);
+  FfArgs f{xy, coef, S, kpar, alpha, d_moff, d_moff + nm + 1, zphase, scratch.ptr, out, n, bs, nrhs, nk, na, mmax};
+  switch (per_m ? mmax : kFfMaxM) {
     case 0: ff_launch<0>(f, st); break;
     case 1: ff_launch<1>(f, st); break;
     case 2: ff_launch<2>(f, st); break;
@@ -244,7 +263,8 @@ void farfield_sum(const double2 *xy, int n, int bs, int nrhs, const double2 *coe
     }
   }
   SG_CUDA(cudaGetLastError());
-  SG_CUDA(cudaStreamSynchronize(st));  // the staging buffers above are released on return
+  SG_CUDA(cudaStreamSynchronize(st));  // the scratch buffer above is released on return
+  return per_m ? 2 : 1;
 }
 
 }  // namespace sg

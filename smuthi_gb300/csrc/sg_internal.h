@@ -278,7 +278,7 @@ void lookup_contract(const double2 *a, int nr, int nk, const double2 *g, int nco
                      double2 *out, long long out_stride, cudaStream_t st);
 
 // particle sum of the scattered plane-wave expansion (sg_farfield.cu); synchronous
-void farfield_sum(const double2 *xy, int n, int bs, int nrhs, const double2 *coef, int mmax, const int *mofn_host,
+int farfield_sum(const double2 *xy, int n, int bs, int nrhs, const double2 *coef, int mmax, const int *mofn_host,
                   int nk, const double *kpar, const double2 *S, int na, const double *alpha, const double2 *zphase,
                   double2 *out, cudaStream_t st);
 

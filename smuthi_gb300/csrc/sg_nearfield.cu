@@ -37,6 +37,7 @@ struct PweArgs {
   const double2 *Q;         // [3][nk][na]
   const double2 *P;         // [nk]
   const double *alpha;      // [na]
+  const double2 *sc;        // sine table
   double2 *partial;         // [ksplit][3][np]
   int np, nk, na, ksplit;
 };
@@ -90,7 +91,7 @@ __global__ void __launch_bounds__(32 * kNfWarps) pwe_field_kernel(const PweArgs 
   extern __shared__ double2 nf_smem[];  // sine table, then (cos alpha, sin alpha) [na]
   __shared__ double2 red[kNfWarps][3][32];
   double2 *T = nf_smem, *csa = nf_smem + kScTable;
-  sc_fill(T);
+  sc_load(A.sc, T);
   for (int a = threadIdx.x; a < A.na; a += blockDim.x) sincos(A.alpha[a], &csa[a].y, &csa[a].x);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -171,18 +172,17 @@ int pwe_field(int field, int np, const double *x, const double *y, const double 
   SG_REQUIRE(field == 0 || (omega > 0 && std::isfinite(omega)), "omega must be positive");
   SG_REQUIRE(k.x != 0.0 || k.y != 0.0, "wavenumber must be nonzero");
   const size_t plane = (size_t)nk * na;
-  DevBuf<double2> Q, P, partial;
-  Q.reserve(3 * plane);
-  P.reserve(nk);
-  pwe_prep_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, st>>>(field, g, kp, kz, alpha, nk, na, k, omega, Q.ptr,
-                                                                   P.ptr);
-  SG_CUDA(cudaGetLastError());
   const int bx = (np + 31) / 32;
   int ksplit = (4 * sm_count() + bx - 1) / bx;  // about four blocks of 256 threads per SM
   const int maxs = nk / kNfWarps > 0 ? nk / kNfWarps : 1;  // keep >= one kappa node per warp
   ksplit = ksplit < 1 ? 1 : (ksplit > maxs ? maxs : ksplit);
-  partial.reserve((size_t)ksplit * 3 * np);
-  PweArgs A{x, y, z, kp, kz, Q.ptr, P.ptr, alpha, partial.ptr, np, nk, na, ksplit};
+  DevBuf<double2> scratch;
+  scratch.reserve(kScTable + 3 * plane + nk + (size_t)ksplit * 3 * np);
+  double2 *Q = scratch.ptr + kScTable, *P = Q + 3 * plane, *partial = P + nk;
+  sc_table(scratch.ptr, st);
+  pwe_prep_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, st>>>(field, g, kp, kz, alpha, nk, na, k, omega, Q, P);
+  SG_CUDA(cudaGetLastError());
+  PweArgs A{x, y, z, kp, kz, Q, P, alpha, scratch.ptr, partial, np, nk, na, ksplit};
   const size_t smem = (kScTable + (size_t)na) * sizeof(double2);
   static bool attr_set[64] = {};
   if (first_on_device(attr_set))
@@ -190,10 +190,10 @@ int pwe_field(int field, int np, const double *x, const double *y, const double 
                                  (int)((kScTable + 8192) * sizeof(double2))));
   pwe_field_kernel<<<dim3(bx, ksplit), 32 * kNfWarps, smem, st>>>(A);
   SG_CUDA(cudaGetLastError());
-  pwe_reduce_kernel<<<(unsigned)((3 * (size_t)np + 255) / 256), 256, 0, st>>>(partial.ptr, np, ksplit, out);
+  pwe_reduce_kernel<<<(unsigned)((3 * (size_t)np + 255) / 256), 256, 0, st>>>(partial, np, ksplit, out);
   SG_CUDA(cudaGetLastError());
-  SG_CUDA(cudaStreamSynchronize(st));  // the scratch buffers are released on return
-  return 3;
+  SG_CUDA(cudaStreamSynchronize(st));  // the scratch buffer is released on return
+  return 4;
 }
 
 // ------------------------------------------------------------------ plane waves -> regular SWE at points

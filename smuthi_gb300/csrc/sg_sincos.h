@@ -21,13 +21,19 @@ static constexpr double kScH2 = 2.391888279584674e-19;          // the rest of i
 static constexpr double kScMagic = 6755399441055744.0;          // 1.5 2^52: n in the low mantissa bits
 static constexpr unsigned kScMaxHigh = 0x41D00000u;             // high word of 2^30: beyond it sincos() itself
 
-// (sin, cos) of 2 pi j / 1024 into shared memory; the caller synchronises
-__device__ __forceinline__ void sc_fill(double2 *table) {
-  for (int j = threadIdx.x; j < kScTable; j += blockDim.x) {
-    double s, c;
-    sincospi((double)j / (kScTable / 2), &s, &c);
-    table[j] = make_double2(s, c);
-  }
+// (sin, cos) of 2 pi j / 1024, once per call: every block of a kernel forming it for itself took as long as three
+// particles or nodes, more than the whole sum of a small system
+static __global__ void __launch_bounds__(128) sc_table_kernel(double2 *table) {
+  const int j = blockIdx.x * 128 + threadIdx.x;
+  double s, c;
+  sincospi((double)j / (kScTable / 2), &s, &c);
+  table[j] = make_double2(s, c);
+}
+static inline void sc_table(double2 *table, cudaStream_t st) { sc_table_kernel<<<kScTable / 128, 128, 0, st>>>(table); }
+
+// the table into shared memory; the caller synchronises
+__device__ __forceinline__ void sc_load(const double2 *from, double2 *table) {
+  for (int j = threadIdx.x; j < kScTable; j += blockDim.x) table[j] = __ldg(from + j);
 }
 
 __device__ __forceinline__ void sc_sincos(double x, const double2 *table, double *s, double *c) {
