@@ -92,6 +92,17 @@ def algorithmic_flops(n, bs, kind, nrhs):
     return float(n) * n * bs * bs * (c_int + 8 * nrhs)
 
 
+def digit_products(bs):
+    """Digit products per element of the interval-batched FP64 operator: weights 0 .. 6, from blocksize 31 on 0 .. 7."""
+    return 28 if bs <= 30 else 34
+
+
+def batched_flops(n, bs, kind, nrhs, products):
+    """Tensor-core arithmetic of an interval-batched product: every coefficient matrix of a pair's interval times every
+    right-hand side, `products` times."""
+    return float(n) * n * 8.0 * bs * bs * (2 if kind == "linear" else 4) * nrhs * products
+
+
 def algorithmic_bytes(n, bs, kind, n_int, nrhs, fp32):
     coef = (2 if kind == "linear" else 4) * n_int * bs * bs * (8 if fp32 else 16)
     pairs = n * n * 16 if fp32 else n * 16
@@ -252,9 +263,19 @@ def run_ours(args, rank, world, local_rank):
     peak64 = ctx.fma_peak(_lib.SG_FP64)
     fp32_dominant = ms32 >= max(ms64, msdf)
     kind = spec["kind"]
+    peaks = {}
+    try:
+        peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
+    except Exception:
+        pass
+    hbm_peak = peaks.get("hbm_gbs", 6800.0)
+    tensor_peak = peaks.get("bf16_tflops", 1900.0)
+    fl = algorithmic_flops(n, bs, kind, R)
+    # FP64-grade products of more than 640 particles (fewer: by size) with blocksize <= 48 are interval-batched
+    batched64 = 640 < n and n * n <= 2 ** 27 and bs <= 48
+    work = None  # arithmetic of the kernel itself where it is not the interpolation that `fl` counts
     if fp32_dominant:
-        avg_ms = ms32 / max(n32, 1)
-        fl = algorithmic_flops(n, bs, kind, R)
+        avg_ms, n_timed = ms32 / max(n32, 1), n32
         v32, t32 = ctx.fp32_autotune(R)[:2]
         name = {0: "coupling_kernel<float> (per receiver, RHS tile %d)" % t32,
                 1: "bucket_kernel (interval-bucketed)",
@@ -262,28 +283,28 @@ def run_ours(args, rank, world, local_rank):
                 3: "sym_kernel (pair-symmetric, two warps per receiver, RHS tile %d)" % t32,
                 4: "tc_coupling_kernel (tcgen05 3xTF32, %d RHS)" % t32,
                 5: "tcsym_kernel (pair-symmetric tcgen05 3xTF32, %d RHS)" % t32}.get(v32, "FP32 operator")
+        peak, bound = peak32, "fp32"
         if ctx.fp32_batched(R)[0]:
             name = "ih_kernel (interval-batched, tcgen05 FP16 parts, %d RHS)" % R
-        peak, bound = peak32, "fp32"
+            work, peak, bound = batched_flops(n, bs, kind, R, 3), tensor_peak, "tensor"
         byts = algorithmic_bytes(n, bs, kind, n_int, R, True)
     elif msdf >= ms64:
-        # double-float kernel on the FP32 pipe: FP64-grade flops against the FP32 pipe's peak
-        avg_ms = msdf / max(ndf, 1)
-        fl = algorithmic_flops(n, bs, kind, R)
-        peak, bound, name = peak32, "fp32", "SG_DF64 operator: ib_kernel (interval-batched) where it applies"
+        avg_ms, n_timed = msdf / max(ndf, 1), ndf
+        if batched64:
+            work, peak, bound = batched_flops(n, bs, kind, R, digit_products(bs)), tensor_peak, "tensor"
+            name = "ib_kernel (interval-batched, tcgen05 FP16 digits)"
+        else:  # FP64-grade flops against the FP32 pipe's peak
+            peak, bound, name = peak32, "fp32", "SG_DF64 operator (by size: ib_kernel, coupling_kernel<double>, <df64>)"
         byts = algorithmic_bytes(n, bs, kind, n_int, R, False)
     else:
-        avg_ms = ms64 / max(n64, 1)
-        fl = algorithmic_flops(n, bs, kind, R)
-        peak, bound, name = peak64, "fp64", "coupling_kernel<double>"
+        avg_ms, n_timed = ms64 / max(n64, 1), n64
+        if batched64:
+            work, peak, bound = batched_flops(n, bs, kind, R, digit_products(bs)), tensor_peak, "tensor"
+            name = "ib_kernel (interval-batched, tcgen05 FP16 digits)"
+        else:
+            peak, bound, name = peak64, "fp64", "SG_FP64 operator (by size: ib_kernel, coupling_kernel<double>)"
         byts = algorithmic_bytes(n, bs, kind, n_int, R, False)
-    achieved = fl / (avg_ms * 1e-3) / 1e12
-    peaks = {}
-    try:
-        peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
-    except Exception:
-        pass
-    hbm_peak = peaks.get("hbm_gbs", 6800.0)
+    achieved = (work or fl) / (avg_ms * 1e-3) / 1e12
     traffic = None
     try:
         tr = json.load(open(os.path.join(ROOT, "profiles", "ncu_traffic.json")))
@@ -295,17 +316,22 @@ def run_ours(args, rank, world, local_rank):
     plain_avg64 = pms64 / max(pn64, 1)
     roof = {"bound": bound, "kernel": name, "achieved": round(achieved, 3), "peak": round(peak, 3),
             "unit": "TFLOP/s", "frac": round(achieved / peak, 4), "traffic": traffic,
-            "peak_source": "FMA-chain probe kernel of this library, measured in this run (the pipe has no "
-                           "entry in MEASURED_PEAKS.json)",
-            "flops_per_launch": fl, "avg_launch_ms": round(avg_ms, 4),
-            "launches": n32 if fp32_dominant else (ndf if name.endswith("<df64>") else n64),
+            "peak_source": ("MEASURED_PEAKS.json, bf16" if bound == "tensor" else
+                            "FMA-chain probe kernel of this library, measured in this run (the pipe has no "
+                            "entry in MEASURED_PEAKS.json)"),
+            "flops_per_launch": work or fl, "interpolation_flops": fl, "avg_launch_ms": round(avg_ms, 4),
+            "launches": n_timed,
             "hbm": {"achieved_gbs": round(byts / (avg_ms * 1e-3) / 1e9, 1), "peak_gbs": hbm_peak,
                     "frac": round(byts / (avg_ms * 1e-3) / 1e9 / hbm_peak, 4), "algorithmic_bytes": byts,
                     "peak_source": "MEASURED_PEAKS.json" if peaks else "fallback"}}
-    fp64_plain_roof = {"kernel": "coupling_kernel<double> (plain drop-in, R=1)", "avg_launch_ms": round(plain_avg64, 3),
-                       "achieved": round(algorithmic_flops(n, bs, kind, 1) / (plain_avg64 * 1e-3) / 1e12, 3),
-                       "peak": round(peak64, 3), "unit": "TFLOP/s",
-                       "frac": round(algorithmic_flops(n, bs, kind, 1) / (plain_avg64 * 1e-3) / 1e12 / peak64, 4)}
+    pfl, ppeak = algorithmic_flops(n, bs, kind, 1), peak64
+    if batched64:
+        pfl, ppeak = batched_flops(n, bs, kind, 1, digit_products(bs)), tensor_peak
+    pach = pfl / (plain_avg64 * 1e-3) / 1e12
+    fp64_plain_roof = {"kernel": ("ib_kernel (interval-batched)" if batched64 else "SG_FP64 operator") + ", plain drop-in, R=1",
+                       "bound": "tensor" if batched64 else "fp64", "avg_launch_ms": round(plain_avg64, 3),
+                       "achieved": round(pach, 3), "peak": round(ppeak, 3), "unit": "TFLOP/s",
+                       "frac": round(pach / ppeak, 4)}
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
@@ -432,7 +458,9 @@ def run_target(args, local_rank):
                            "precond_fallbacks": info.precond_fallbacks, "residual_arithmetic": "df64",
                            "fp32_kernel": dict(zip(("variant", "rhs_tile", "ms_per_receiver", "ms_bucketed",
                                                     "ms_symmetric", "ms_tensor_core", "ms_tensor_core_symmetric"),
-                                                   ctx.fp32_autotune(R)))},
+                                                   ctx.fp32_autotune(R)),
+                                               **dict(zip(("interval_batched", "ms_interval_batched"),
+                                                          ctx.fp32_batched(R))))},
            "plain_fp64": {"s_per_rhs": round(plain_s, 3), "iterations": pinfo.iterations,
                           "fp64_matvecs": pinfo.fp64_matvecs, "rel_residual_fp64": float(prelres[0]),
                           "restart": 20, "x0": "b"},
