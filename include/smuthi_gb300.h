@@ -127,7 +127,7 @@ int sg_master_matvec(sg_context *ctx, const double *x, double *y, int nrhs, int 
 /* Stream capture: make one uncaptured product of the same precision and nrhs first. The captured product then runs the
  * same kernels with scratch memory that belongs to the graph (SG_FP32 variants 1 to 5: in the context's, which later
  * products of other counts may move). Without it an FP64 or double-float product takes the FP64 per-receiver kernel, and
- * an FP32 one fails. */
+ * an FP32 one fails. set_particles, set_lookup and sg_batched_memory end the life of what was captured. */
 /* Device-pointer variants: x, y are device buffers in the reference layout;
  * `stream` is a cudaStream_t (NULL = the context's stream). Asynchronous. */
 int sg_coupling_matvec_dev(sg_context *ctx, const void *x, void *y, int nrhs, int precision, void *stream);
@@ -202,8 +202,9 @@ int sg_fp32_set_kernel(sg_context *ctx, int nrhs, int variant, int rhs_tile);
 /* The interval-batched FP32 operator (pairs grouped by lookup interval, tensor cores) takes the place of
  * variants 4 and 5 for an RHS count >= 16 when the autotuner finds it faster: *taken = 1 then, and *ms its
  * time (-1 when not timed; either pointer may be NULL). take != 0 fixes it for that RHS count (32 particles
- * or more, blocksize <= 30 or 33 to 48) until the next set_particles, set_lookup or sg_fp32_set_kernel. No
- * counterpart in the reference. */
+ * or more, blocksize <= 30 or 33 to 48) until the next set_particles, set_lookup or sg_fp32_set_kernel. Its
+ * sums, like those of variants 1 to 3 and 5, are formed by atomics: the last bits of a product differ from run to run
+ * (variants 0 and 4, fixed with sg_fp32_set_kernel, repeat exactly). No counterpart in the reference. */
 int sg_fp32_batched(sg_context *ctx, int nrhs, int take, int *taken, double *ms);
 
 /* Kernel of the FP64-grade products with the radial lookup: 0 = the faster one by size and grid (default), 1 = the

@@ -24,7 +24,9 @@
 // their largest magnitude and one sign, and would then be rounded at 2^-51 of the scales, under a sum
 // that is itself 60 times as large. Blocksizes 31 to 48 take 8-bit digits of 55-bit numbers and the
 // weights d = 0..7, at most 7 * 96 * 2^14 < 2^24. The digits are combined in 64-bit integers, in which
-// the powers of t and the rotations follow; the result is independent of how the pairs are grouped.
+// the powers of t and the rotations follow; the result is independent of how the pairs are grouped. Accuracy is by the
+// scales, row of C times column of x, and not by element: an element 2^-9 and more below them (2^-2 with 8-bit digits)
+// keeps fewer than 53 bits.
 //
 // One CTA per SM walks a contiguous range of tiles; a tile is up to 128 complex columns (pairs x
 // right-hand sides) of one interval:
@@ -39,8 +41,8 @@
 // A second kernel sums V over the emitters of every receiver in index order (deterministic) and forms
 // W x or x - T W x. V is a bounded workspace: larger problems run in chunks of tiles.
 //
-// What bounds it: instruction issue (42% of the slots, half of them two-cycle integer instructions) and the
-// tensor core (34%) in turn: a tile of 2000 spheres takes 44 thousand cycles, of which 16 are MMAs, 6 forming A,
+// What bounds it: instruction issue (42% of the slots with 1000 spheres, half of them two-cycle integer instructions) and
+// the tensor core (34%) in turn: a tile of 2000 spheres takes 44 thousand cycles, of which 16 are MMAs, 6 forming A,
 // 13 the last combination; operand memory does not allow a second tile in flight. 2000 spheres, cubic lookup, one
 // right-hand side: 80.5 ms with the per-receiver kernel, 9.3 with Re and Im of u as separate rows of A in shared
 // memory (twice the accumulators to read and combine), 5.2 now; 1201 spheres with l_max = 4: 82.4, 8.0, 5.05; 100

@@ -17,11 +17,13 @@
 //
 // Every wait is bounded; a wait that runs out sets the error flag, and all roles leave.
 //
-// What bounds it: instruction issue of forming and combining (2000 spheres, 16 right-hand sides: 7.19 ms; 6.8 without
-// the atomics, 8.6 against 9.4 without two thirds of the MMAs in a first form whose scales were two factors per
-// element; fetching the next tile's x ahead costs more registers than it hides, 7.56). Against the pair-symmetric 3xTF32
-// kernel: 2000 spheres, cubic, 16: 13.6 -> 7.19 ms, error 4.5e-7 -> 2.7e-7; film of 4001, linear, 16: 45.9 -> 23.9 ms,
-// 2.7e-7 -> 2.0e-7; against the one-directional one: 1500 spheres, l_max 4, 64: 33.6 -> 32.0 ms, 8.3e-7 -> 2.3e-7.
+// What bounds it: each set's own chain. 1000 spheres, 16 right-hand sides: 60% of the issue slots, 36% of the tensor core;
+// the schedulers' five warps wait for x_j and for the set's products (2000 spheres: 6.8 of 7.2 ms without the atomics, 8.6
+// against 9.4 without two thirds of the MMAs in a first form whose scales were two factors per element; fetching the next
+// tile's x ahead costs more registers than it hides, 7.56). Four powers of t times three products make 14.5 ms of MMAs of
+// 1500 spheres with l_max 4 and 64 right-hand sides. Against the pair-symmetric 3xTF32 kernel: 2000 spheres, cubic, 16:
+// 13.6 -> 7.28 ms, error of x - T W x 4.5e-7 -> 1.2e-7; film of 4001, linear, 16: 45.9 -> 24.1 ms, 2.7e-7 -> 7.3e-8;
+// against the one-directional one, which repeats exactly: 1500 spheres, l_max 4, 64: 33.6 -> 31.0 ms, 8.3e-7 -> 1.4e-7.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -6,7 +6,8 @@
 //   sin r = r - r^3/6 + r^5/120,  cos r - 1 = -r^2/2 + r^4/24
 // leave Taylor remainders below 6e-22 and 2e-18. r is formed with two fused multiply-adds against h in two
 // parts: n h_1 is subtracted without rounding error (the difference is a multiple of h_1's last place below
-// h), so r is good to its own last place. The result is within 0.7 units in the last place of max(|sin|, |cos|).
+// h), so r is good to its own last place. The result is within 0.7 units in the last place of max(|sin|, |cos|) of what
+// the table's values give, which carry the error of sincospi (CUDA states at most two such units for it).
 // 16 FP64 operations and one 16-byte table read; sincos() takes about 44 of them.
 #pragma once
 
